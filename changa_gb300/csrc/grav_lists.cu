@@ -40,6 +40,7 @@
 #include "chg_internal.h"
 #include "f32x2.cuh"
 #include "list_eval.cuh"
+#include "list_far.cuh"
 
 namespace chg {
 namespace {
@@ -606,13 +607,17 @@ struct Variant {
   int tp;  // 0 source-parallel, 1 target-parallel (list_kernel_tp), 2 paired (list_kernel_tp2),
            // 3 paired with TMA-staged cell records (list_kernel_tma; FP32-mixed cell lists,
            //   list_kernel_tp2 for the others), 4 register-blocked paired (list_kernel_rb,
-           //   group = the most targets per lane)
+           //   group = the most targets per lane), 5 far-first, a CTA of `group` threads per
+           //   bucket (list_kernel_block), 6 far-first, a warp per bucket (list_kernel_far),
+           // 7 one of these two by the number of buckets
 };
 constexpr Variant kVariants[] = {{2, 16, 0}, {3, 16, 0}, {4, 16, 0}, {3, 32, 0}, {2, 32, 0},
                                  {2, 0, 1},  {3, 0, 1},  {4, 0, 1},  {2, 0, 2},  {3, 0, 2},
                                  {4, 0, 2},  {2, 0, 3},  {1, 0, 3},  {2, 3, 4},  {2, 2, 4},
-                                 {3, 2, 4},  {1, 3, 4}};
+                                 {3, 2, 4},  {1, 3, 4},  {3, 0, 6},  {6, 128, 5},
+                                 {0, 0, 7}};
 constexpr int kNumVariants = sizeof(kVariants) / sizeof(kVariants[0]);
+constexpr int kFarVariant = 17, kBlockVariant = 18, kAutoVariant = 19;
 
 /* Source-parallel list kernel of the FP32 forms.  Per warp and bucket: the
  * targets (kTB at a time) sit in shared memory; for each chunk of kTC
@@ -2342,7 +2347,7 @@ __global__ void cells_as_parts_kernel(const double* __restrict__ m, int stride, 
 }
 
 /* The FP64 form runs list_kernel (its cost is the FP64 pipe); the FP32
- * forms run one of the variants below: paired target-parallel by default
+ * forms run one of the variants below: the far-first kernels by default
  * (the fastest on the measured workloads), the others on request or by the
  * autotuner. */
 template <typename K>
@@ -2355,6 +2360,25 @@ int blocks_per_sm(K kernel, std::atomic<int>* cache) {
     cache->store(nb, std::memory_order_relaxed);
   }
   return nb;
+}
+
+template <typename K>
+cudaError_t launch_block(K kernel, int threads, std::atomic<int>* cache, int kid, const ListArgs& a,
+                        cudaStream_t s) {
+  if (a.n_buckets <= 0) return cudaSuccess;
+  int nb = cache->load(std::memory_order_relaxed);
+  if (!nb) {
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kernel, threads, 0) != cudaSuccess ||
+        nb < 1)
+      nb = 1;
+    cache->store(nb, std::memory_order_relaxed);
+  }
+  const long long cap = (long long)sm_count() * nb;
+  const int grid = (int)(a.n_buckets < cap ? a.n_buckets : cap);
+  TimingScope ts(kid, s);
+  kernel<<<grid, threads, 0, s>>>(a);
+  count_launch();
+  return cudaGetLastError();
 }
 
 template <typename K>
@@ -2373,7 +2397,8 @@ cudaError_t launch_kernel(K kernel, std::atomic<int>* occ_cache, int kid, const 
 /* current variant per list kernel id (FP32 forms); several host threads
  * may launch while another sets a variant, so each launch loads its id's
  * variant once, atomically */
-std::atomic<int> g_variant[6] = {{8}, {10}, {0}, {0}, {8}, {10}};
+std::atomic<int> g_variant[6] = {{kAutoVariant}, {kAutoVariant}, {0},
+                                 {0},            {kAutoVariant}, {kAutoVariant}};
 /* poll limit of the TMA variants' mbarrier waits (a test hook lowers it) */
 constexpr int kDefaultWaitPolls = 1 << 22;
 std::atomic<int> g_tma_wait_polls{kDefaultWaitPolls};
@@ -2443,7 +2468,21 @@ cudaError_t launch_variant(const ListArgs& a, cudaStream_t s) {
     }
     return launch_kernel(list_kernel_tp2<FORM, CELL, var.minb>, &occ, list_kernel_id(FORM, CELL),
                          a, s);
-  } else if constexpr (var.tp == 4)
+  } else if constexpr (var.tp == 7) {
+    /* a CTA per bucket while the buckets are fewer than the warps that
+     * list_kernel_far keeps resident (24 per SM).  On both sides of that
+     * line, cells / particles in us, CTA against warp: 2230 buckets 30 / 37
+     * against 32 / 37, 4300 buckets 83 / 169 against 85 / 173, 6030 buckets
+     * 91 / 91 against 90 / 77. */
+    return (long long)a.n_buckets <= 24ll * sm_count() ? launch_variant<FORM, CELL, kBlockVariant>(a, s)
+                                                       : launch_variant<FORM, CELL, kFarVariant>(a, s);
+  } else if constexpr (var.tp == 5)
+    return launch_block(list_kernel_block<FORM, CELL, var.group, var.minb>, var.group, &occ,
+                        list_kernel_id(FORM, CELL), a, s);
+  else if constexpr (var.tp == 6)
+    return launch_kernel(list_kernel_far<FORM, CELL, var.minb>, &occ, list_kernel_id(FORM, CELL), a,
+                         s);
+  else if constexpr (var.tp == 4)
     return launch_kernel(list_kernel_rb<FORM, CELL, var.minb, var.group>, &occ,
                          list_kernel_id(FORM, CELL), a, s);
   else if constexpr (var.tp == 2)

@@ -86,12 +86,14 @@ int changa_gb300_kernel_time(int kernel, double *total_ms, long long *launches);
 /* Shape variants of the FP32-form list kernels (kernel ids 0, 1, 4, 5):
  * 0-4 source-parallel (resident blocks per SM x list chunks per reduction),
  * 5-7 target-parallel (2/3/4 blocks per SM), 8-10 target-parallel with
- * paired .f32x2 arithmetic (2/3/4 blocks per SM; defaults 8 for cell lists,
- * 10 for particle lists), 11-12 paired with the FP32-mixed cell records
+ * paired .f32x2 arithmetic (2/3/4 blocks per SM), 11-12 paired with the FP32-mixed cell records
  * staged by TMA tile::gather4 copies (2/1 blocks per SM; the other lists
  * run the paired kernel), 13-16 paired with 1-3 targets per lane chosen
  * per bucket (blocks per SM / most targets per lane: 2/3, 2/2, 3/2, 1/3),
- * which keeps the lanes of buckets of 17-31 targets busy.  The autotuner
+ * which keeps the lanes of buckets of 17-31 targets busy, 17-18 paired with
+ * each block's unsoftened sources first (17 a warp per bucket, 18 a CTA per
+ * bucket), 19 (the default) one of these two by the number of buckets.  The
+ * autotuner
  * (changa_gb300/autotune.py) times them on a workload and selects one per
  * kernel. */
 int changa_gb300_list_variant_count(void);
