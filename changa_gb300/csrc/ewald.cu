@@ -34,6 +34,7 @@
 
 #include "chg_internal.h"
 #include "f32x2.cuh"
+#include "fp64_math.cuh"
 
 namespace chg {
 namespace {
@@ -278,16 +279,22 @@ struct EwaldFpArgs {
   double L, fEwCut2, alpha, alpha2, k1, ka;
   int nReps, nEwReps, nEwhLoop;
   double ewt[CHANGA_MAX_EWH][5];
+  /* the table as whole h, one of each pair h, -h with its coefficients
+   * doubled; n_whole is 0 for a table of other vectors */
+  int n_whole;
+  float cut2;  // fEwCut2 rounded up
+  signed char h[CHANGA_MAX_EWH][4];
+  double hc[CHANGA_MAX_EWH][2];  // cosine and sine coefficients
 };
+constexpr int kWholeMax = 4;  // largest component of a whole h
 
 /* FP64 real-space term (Ewald.cpp:137-240): quadrupole, or with HEX the
  * hexadecapole expansion of the complete root moments (g4, g5 added). */
-template <bool HEX>
+template <bool HEX, class Gauss>
 __device__ __forceinline__ void ewald_term_f64(const EwaldFpArgs& P, double x, double y, double z,
-                                               bool hole, double fInner2, double& fPot,
-                                               double& ax, double& ay, double& az) {
+                                               double r2, bool hole, double fInner2, Gauss gauss,
+                                               double& fPot, double& ax, double& ay, double& az) {
   const double* mom = P.mom;
-  double r2 = x * x + y * y + z * z;
   double g0, g1, g2, g3, g4 = 0.0, g5 = 0.0;
   if (r2 < fInner2) {
     double alphan = P.ka;
@@ -306,12 +313,16 @@ __device__ __forceinline__ void ewald_term_f64(const EwaldFpArgs& P, double x, d
       g5 = alphan * ((1.0 / 13.0) * r2 - (1.0 / 11.0));
     }
   } else {
-    const double dir = rsqrt(r2);
+    /* erfc from its scaled form, which shares the exponential with the
+     * Gaussian terms; erf itself where it is small (there the terms below
+     * lose digits of it) */
+    const double dir = rsqrt_normal(r2);
     const double dir2 = dir * dir;
-    double a = exp(-r2 * P.alpha2);
-    a *= P.ka * dir2;
+    const double e = gauss(r2);  // exp(-alpha^2 r^2)
+    const double a = e * (P.ka * dir2);
     const double ar = P.alpha * (r2 * dir);
-    g0 = hole ? -erf(ar) : erfc(ar);
+    if (hole && ar < 0.5) g0 = -erf(ar);
+    else g0 = hole ? fma(e, erfcx(ar), -1.0) : e * erfcx(ar);
     g0 *= dir;
     g1 = g0 * dir2 + a;
     double alphan = 2 * P.alpha2;
@@ -342,47 +353,185 @@ __device__ __forceinline__ void ewald_term_f64(const EwaldFpArgs& P, double x, d
 }
 
 
+/* One thread per particle.  FP64 instructions bound it (one per SM in 16
+ * cycles), so the replicas are first culled in FP32 against the box of the
+ * warp's 32 particles (about 90 of 343 are left, and only they are tested in
+ * FP64), and the Fourier terms of whole h come from powers of
+ * exp(2 pi i d_k / L), three sines and cosines per particle instead of one
+ * per h and four FP64 operations per product; the Gaussian of a replica is a
+ * product over the axes.  120011 particles, cut 2.6, h-cut 2.8: 3392 us with
+ * a test per replica, an exponential and an erfc per term and a sincos per h,
+ * 2370 so (FP64 pipe 86% busy; erfcx is most of what is left). */
 template <bool HEX>
 __global__ void __launch_bounds__(128) ewald_f64_kernel(const double* __restrict__ parts,
                                                         long long n_parts,
                                                         const int* __restrict__ idx,
                                                         long long n_idx, double* __restrict__ vars,
                                                         const __grid_constant__ EwaldFpArgs P) {
+  constexpr int kBatch = 128;  // replicas culled at a time
+  __shared__ double rx[4][kBatch], ry[4][kBatch], rz[4][kBatch];  // replica offsets
+  __shared__ int rcode[4][kBatch];                                // offsets per axis, and the hole
+  /* first exp(-alpha^2 (d + i L)^2) per axis for |i| <= 3, then
+   * exp(2 pi i k d / L) for k = 1 .. kWholeMax */
+  __shared__ double pw[3][kWholeMax][2][128];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (k >= n_idx) return;
-  const long long j = idx ? (long long)idx[k] : k;
-  if (j < 0 || j >= n_parts) return;
-  const double* p = parts + 5 * j;
-  const double dxd = p[2] - P.mom[3], dyd = p[3] - P.mom[4], dzd = p[4] - P.mom[5];
-  const int nE = P.nEwReps, nR = P.nReps;
-  double fPot = P.mom[2] * P.k1, ax = 0, ay = 0, az = 0;
-  const double fInner2 = 1.2e-3 * P.L * P.L;
-  for (int ix = -nE; ix <= nE; ++ix) {
-    const bool hx = (ix >= -nR && ix <= nR);
-    const double x = dxd + ix * P.L;
-    for (int iy = -nE; iy <= nE; ++iy) {
-      const bool hxy = hx && (iy >= -nR && iy <= nR);
-      const double y = dyd + iy * P.L;
-      for (int iz = -nE; iz <= nE; ++iz) {
-        const bool hole = hxy && (iz >= -nR && iz <= nR);
-        const double z = dzd + iz * P.L;
-        const double r2 = x * x + y * y + z * z;
-        if (r2 > P.fEwCut2 && !hole) continue;
-        ewald_term_f64<HEX>(P, x, y, z, hole, fInner2, fPot, ax, ay, az);
-      }
+  long long j = -1;
+  if (k < n_idx) {
+    j = idx ? (long long)idx[k] : k;
+    if (j < 0 || j >= n_parts) j = -1;
+  }
+  const bool live = j >= 0;
+  if (!__any_sync(0xffffffffu, live)) return;
+  double dd[3] = {0.0, 0.0, 0.0};
+  if (live)
+    for (int c = 0; c < 3; ++c) dd[c] = parts[5 * j + 2 + c] - P.mom[3 + c];
+  const double dxd = dd[0], dyd = dd[1], dzd = dd[2];
+  float lo[3], hi[3];
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    lo[c] = live ? (float)dd[c] : 3e38f;
+    hi[c] = live ? (float)dd[c] : -3e38f;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      lo[c] = fminf(lo[c], __shfl_xor_sync(0xffffffffu, lo[c], o));
+      hi[c] = fmaxf(hi[c], __shfl_xor_sync(0xffffffffu, hi[c], o));
     }
   }
-  for (int i = 0; i < P.nEwhLoop; ++i) {
-    const double* e = P.ewt[i];
-    const double hdotx = e[0] * dxd + e[1] * dyd + e[2] * dzd;
-    double s, c;
-    sincos(hdotx, &s, &c);
-    fPot += e[3] * c + e[4] * s;
-    const double t = e[3] * s - e[4] * c;
-    ax += e[0] * t;
-    ay += e[1] * t;
-    az += e[2] * t;
+  const int nE = P.nEwReps, nR = P.nReps;
+  const long long side = 2 * nE + 1, nrep = side * side * side;
+  const float L = (float)P.L;
+  double fPot = P.mom[2] * P.k1, ax = 0, ay = 0, az = 0;
+  const double fInner2 = 1.2e-3 * P.L * P.L;
+  const bool split = nE <= 3;  // the Gaussian as a product over the axes
+  if (split)
+    for (int c = 0; c < 3; ++c)
+      for (int i = -nE; i <= nE; ++i) {
+        const double u = dd[c] + i * P.L;
+        (&pw[c][0][0][0])[(i + 3) * 128 + threadIdx.x] = exp(-P.alpha2 * (u * u));
+      }
+  for (long long r0 = 0; r0 < nrep; r0 += kBatch) {
+    int count = 0;
+    for (int b = 0; b < kBatch; b += 32) {
+      const long long r = r0 + b + lane;
+      bool keep = false;
+      int i[3] = {0, 0, 0};
+      bool hole = false;
+      if (r < nrep) {
+        i[0] = (int)(r / (side * side)) - nE;
+        i[1] = (int)(r / side % side) - nE;
+        i[2] = (int)(r % side) - nE;
+        hole = abs(i[0]) <= nR && abs(i[1]) <= nR && abs(i[2]) <= nR;
+        float d2 = 0.f;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          const float a = lo[c] + i[c] * L, z = hi[c] + i[c] * L;
+          const float m = a > 0.f ? a : (z < 0.f ? -z : 0.f);
+          d2 = fmaf(m, m, d2);
+        }
+        keep = hole || !(d2 > P.cut2 * 1.0001f);  // room for the rounding of FP32 offsets
+      }
+      const unsigned m = __ballot_sync(0xffffffffu, keep);
+      if (keep) {
+        const int at = count + __popc(m & ((1u << lane) - 1u));
+        rx[warp][at] = i[0] * P.L;
+        ry[warp][at] = i[1] * P.L;
+        rz[warp][at] = i[2] * P.L;
+        rcode[warp][at] = split ? (i[0] + 3) | (i[1] + 3) << 3 | (i[2] + 3) << 6 | hole << 9 : hole << 9;
+      }
+      count += __popc(m);
+    }
+    __syncwarp();
+    for (int q = 0; q < count; ++q) {
+      const int code = rcode[warp][q];
+      const bool hole = code >> 9;
+      const double x = dxd + rx[warp][q], y = dyd + ry[warp][q], z = dzd + rz[warp][q];
+      const double r2 = x * x + y * y + z * z;
+      if (!live || (r2 > P.fEwCut2 && !hole)) continue;
+      ewald_term_f64<HEX>(P, x, y, z, r2, hole, fInner2,
+                          [&](double s) {
+                            if (!split) return exp(-s * P.alpha2);
+                            const double* g = &pw[0][0][0][0] + threadIdx.x;
+                            return g[128 * (code & 7)] * g[128 * (8 + (code >> 3 & 7))] *
+                                   g[128 * (16 + (code >> 6 & 7))];
+                          },
+                          fPot, ax, ay, az);
+    }
+    __syncwarp();  // the list is rewritten by the next batch
   }
+  if (P.n_whole > 0) {
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      double s1, c1;
+      sincospi(2.0 * (dd[c] / P.L), &s1, &c1);
+      double re = c1, im = s1;
+      pw[c][0][0][threadIdx.x] = re;
+      pw[c][0][1][threadIdx.x] = im;
+#pragma unroll
+      for (int q = 1; q < kWholeMax; ++q) {
+        const double t = fma(re, c1, -(im * s1));
+        im = fma(re, s1, im * c1);
+        re = t;
+        pw[c][q][0][threadIdx.x] = re;
+        pw[c][q][1][threadIdx.x] = im;
+      }
+    }
+    /* exp(2 pi i h d / L) along axis c */
+    auto axis = [&](int c, int h, double& re, double& im) {
+      if (h == 0) {
+        re = 1.0;
+        im = 0.0;
+      } else {
+        re = pw[c][abs(h) - 1][0][threadIdx.x];
+        const double s = pw[c][abs(h) - 1][1][threadIdx.x];
+        im = h < 0 ? -s : s;
+      }
+    };
+    double kx = 0, ky = 0, kz = 0, xr = 1.0, xi = 0.0;
+    int hx = 127, hy = 127;
+    for (int i = 0; i < P.n_whole; ++i) {
+      const int nx = P.h[i][0], ny = P.h[i][1], nz = P.h[i][2];
+      if (nx != hx || ny != hy) {  // uniform over the launch
+        double yr, yi, zr, zi;
+        axis(0, nx, yr, yi);
+        axis(1, ny, zr, zi);
+        xr = fma(yr, zr, -(yi * zi));
+        xi = fma(yr, zi, yi * zr);
+        hx = nx;
+        hy = ny;
+      }
+      double zr, zi;
+      axis(2, nz, zr, zi);
+      const double c = fma(xr, zr, -(xi * zi)), s = fma(xr, zi, xi * zr);
+      const double hc = P.hc[i][0], hs = P.hc[i][1];
+      double t = hc * s;
+      fPot = fma(hc, c, fPot);
+      if (hs != 0.0) {
+        fPot = fma(hs, s, fPot);
+        t = fma(-hs, c, t);
+      }
+      kx = fma((double)nx, t, kx);
+      ky = fma((double)ny, t, ky);
+      kz = fma((double)nz, t, kz);
+    }
+    const double tl = 2.0 * 3.14159265358979323846 / P.L;
+    ax = fma(tl, kx, ax);
+    ay = fma(tl, ky, ay);
+    az = fma(tl, kz, az);
+  } else {
+    for (int i = 0; i < P.nEwhLoop; ++i) {
+      const double* e = P.ewt[i];
+      const double hdotx = e[0] * dxd + e[1] * dyd + e[2] * dzd;
+      double s, c;
+      sincos(hdotx, &s, &c);
+      fPot += e[3] * c + e[4] * s;
+      const double t = e[3] * s - e[4] * c;
+      ax += e[0] * t;
+      ay += e[1] * t;
+      az += e[2] * t;
+    }
+  }
+  if (!live) return;
   double* v = vars + 5 * j;
   v[0] += ax;
   v[1] += ay;
@@ -746,6 +895,57 @@ cudaError_t launch_ewald_f32(const CompactPartData* parts, VariablePartData* var
   return cudaGetLastError();
 }
 
+namespace {
+
+struct HPair {
+  int h[3];
+  double c, s;
+};
+
+/* The table as whole h.  The terms of h and -h are equal: the cosine
+ * coefficient is even in h, the sine coefficient and the phase odd.  The
+ * table (EwaldInit's loop over the cube of h) holds both; one of each pair
+ * is kept with its coefficients doubled (exact in floating point), which
+ * halves the k-space loop.  Entries without an exact mirror are kept as
+ * they are.  Returns whether every row is 2 pi h / L to rounding. */
+bool pair_h(const ChangaEwaldParams& p, double L, std::vector<HPair>& out) {
+  const double f = L / (2.0 * M_PI);
+  const int n = p.nEwhLoop;
+  bool whole = true;
+  std::vector<int> hi(3 * (size_t)n);
+  std::vector<char> used((size_t)n, 0);
+  for (int i = 0; i < n; ++i)
+    for (int k = 0; k < 3; ++k) {
+      const double h = p.ewt[5 * i + k] * f;
+      hi[3 * i + k] = (int)rint(h);
+      whole = whole && fabs(h - rint(h)) <= 1e-14 * (1.0 + fabs(h));
+    }
+  for (int i = 0; i < n; ++i) {
+    if (used[i]) continue;
+    const double* e = p.ewt + 5 * i;
+    double scale = 1.0;
+    for (int j = i + 1; j < n; ++j) {
+      const double* g = p.ewt + 5 * j;
+      if (!used[j] && hi[3 * j] == -hi[3 * i] && hi[3 * j + 1] == -hi[3 * i + 1] &&
+          hi[3 * j + 2] == -hi[3 * i + 2] && g[3] == e[3] && g[4] == -e[4]) {
+        used[j] = 1;
+        scale = 2.0;
+        break;
+      }
+    }
+    out.push_back(HPair{{hi[3 * i], hi[3 * i + 1], hi[3 * i + 2]}, scale * e[3], scale * e[4]});
+  }
+  return whole;
+}
+
+}  // namespace
+
+/* Threads per block (one per particle): single warps while blocks of four
+ * would leave SMs without one.  Each warp's results are the same either way
+ * (a warp culls for its own 32 particles).  3000 particles, FP64: 495 us
+ * with blocks of 128. */
+static int ewald_threads(long long n) { return n <= 128ll * sm_count() ? 32 : 128; }
+
 cudaError_t launch_ewald_fp(int form, const double* parts, long long n_parts, const int* idx,
                             long long n_idx, const ChangaEwaldParams& p, double* vars,
                             cudaStream_t s, bool hex) {
@@ -771,11 +971,24 @@ cudaError_t launch_ewald_fp(int form, const double* parts, long long n_parts, co
     P.nEwhLoop = p.nEwhLoop;
     for (int i = 0; i < p.nEwhLoop; ++i)
       for (int k = 0; k < 5; ++k) P.ewt[i][k] = p.ewt[5 * i + k];
+    P.cut2 = (float)P.fEwCut2;
+    /* the powers serve tables whose rows are 2 pi h / L to rounding */
+    std::vector<HPair> pairs;
+    P.n_whole = pair_h(p, L, pairs) ? (int)pairs.size() : 0;
+    for (int i = 0; i < P.n_whole; ++i) {
+      for (int k = 0; k < 3; ++k) {
+        if (abs(pairs[i].h[k]) > kWholeMax) P.n_whole = 0;
+        P.h[i][k] = (signed char)pairs[i].h[k];
+      }
+      P.hc[i][0] = pairs[i].c;
+      P.hc[i][1] = pairs[i].s;
+    }
     if (hex) fill_hex_root(p.momc, P.hex);
-    int blocks = (int)((n_idx + 127) / 128);
+    const int threads = ewald_threads(n_idx);
+    const int blocks = (int)((n_idx + threads - 1) / threads);
     TimingScope ts(kKidEwaldF64, s);
-    if (hex) ewald_f64_kernel<true><<<blocks, 128, 0, s>>>(parts, n_parts, idx, n_idx, vars, P);
-    else ewald_f64_kernel<false><<<blocks, 128, 0, s>>>(parts, n_parts, idx, n_idx, vars, P);
+    if (hex) ewald_f64_kernel<true><<<blocks, threads, 0, s>>>(parts, n_parts, idx, n_idx, vars, P);
+    else ewald_f64_kernel<false><<<blocks, threads, 0, s>>>(parts, n_parts, idx, n_idx, vars, P);
     count_launch();
     return cudaGetLastError();
   }
@@ -798,42 +1011,20 @@ cudaError_t launch_ewald_fp(int form, const double* parts, long long n_parts, co
   P.twopi_over_L = (float)(2.0 * M_PI / L);
   P.nReps = p.nReps;
   P.nEwReps = nE;
-  /* The terms of h and -h are equal: the cosine coefficient is even in h,
-   * the sine coefficient and the phase odd.  The table (EwaldInit's loop
-   * over the cube of h) holds both; one of each pair is kept with its
-   * coefficients doubled (exact in floating point), which halves the
-   * k-space loop.  Entries without an exact mirror are kept as they are. */
   {
-    const double f = L / (2.0 * M_PI);
-    const int n = p.nEwhLoop;
-    std::vector<int> hi(3 * (size_t)n);
-    std::vector<char> used((size_t)n, 0);
-    for (int i = 0; i < n; ++i)
-      for (int k = 0; k < 3; ++k) hi[3 * i + k] = (int)rint(p.ewt[5 * i + k] * f);
+    std::vector<HPair> pairs;
+    pair_h(p, L, pairs);
     int m = 0;
-    for (int i = 0; i < n; ++i) {
-      if (used[i]) continue;
-      const double* e = p.ewt + 5 * i;
-      double scale = 1.0;
-      for (int j = i + 1; j < n; ++j) {
-        const double* g = p.ewt + 5 * j;
-        if (!used[j] && hi[3 * j] == -hi[3 * i] && hi[3 * j + 1] == -hi[3 * i + 1] &&
-            hi[3 * j + 2] == -hi[3 * i + 2] && g[3] == e[3] && g[4] == -e[4]) {
-          used[j] = 1;
-          scale = 2.0;
-          break;
-        }
-      }
-      P.h[m] = make_float4((float)hi[3 * i], (float)hi[3 * i + 1], (float)hi[3 * i + 2],
-                           (float)(scale * e[3]));
-      P.hs[m] = (float)(scale * e[4]);
+    for (const HPair& e : pairs) {
+      P.h[m] = make_float4((float)e.h[0], (float)e.h[1], (float)e.h[2], (float)e.c);
+      P.hs[m] = (float)e.s;
       ++m;
     }
     P.nEwhLoop = m;
   }
   if (hex) fill_hex_root(p.momc, P.hex);
-  int threads = kMixWarps * 32;
-  int blocks = (int)((n_idx + threads - 1) / threads);
+  const int threads = ewald_threads(n_idx);
+  const int blocks = (int)((n_idx + threads - 1) / threads);
   TimingScope ts(kKidEwaldMix, s);
   if (hex) ewald_mix_kernel<true><<<blocks, threads, 0, s>>>(parts, n_parts, idx, n_idx, vars, P);
   else ewald_mix_kernel<false><<<blocks, threads, 0, s>>>(parts, n_parts, idx, n_idx, vars, P);

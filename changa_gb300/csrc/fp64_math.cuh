@@ -1,0 +1,24 @@
+/* FP64 helpers of the plain FP64 form. */
+#pragma once
+
+namespace chg {
+namespace {
+
+/* 1/sqrt(x) for positive normal x, from the hardware's approximation (some
+ * 20 bits): with e = 1 - x y^2, 1/sqrt(x) = y (1 - e)^(-1/2), whose series
+ * y (1 + e/2 + 3 e^2 / 8) is cut at e^3 / 3, below FP64 rounding.  Five FP64
+ * operations; 0 at infinity as rsqrt gives, NaN for a zero or subnormal. */
+__device__ __forceinline__ double rsqrt_normal(double x) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double e = fma(-(x * y), y, 1.0);
+  return fma(fma(e, 0.375, 0.5), e * y, y);
+}
+
+/* The larger of two doubles that are not negative, on the integer pipe. */
+__device__ __forceinline__ double max_nonneg(double a, double b) {
+  return __longlong_as_double(max(__double_as_longlong(a), __double_as_longlong(b)));
+}
+
+}  // namespace
+}  // namespace chg

@@ -41,6 +41,7 @@
 #include "f32x2.cuh"
 #include "list_eval.cuh"
 #include "list_far.cuh"
+#include "list_f64.cuh"
 
 namespace chg {
 namespace {
@@ -55,70 +56,6 @@ template <typename T>
 struct Acc {
   T ax, ay, az, pot, idt2;
 };
-
-/* One cell on one target (gravity.h:436-472 / HostCUDA.cu:1091-1164).
- * rec: {sx, sy, sz, M, soft, tr, xx, xy, xz, yy, yz, zz}; r = target - s. */
-template <typename T>
-__device__ __forceinline__ void pc_interact(const T* rec, T tx, T ty, T tz, T tsoft, T tmass,
-                                            Acc<T>& acc) {
-  const T rx = tx - rec[0], ry = ty - rec[1], rz = tz - rec[2];
-  const T M = rec[3];
-  const T rsq = rx * rx + ry * ry + rz * rz;
-  if (rsq != T(0)) {
-    const T dir = rsqrt_t(rsq);
-    const T twoh = rec[4] + tsoft;
-    T a, b, c, d;
-    if (rsq < twoh * twoh) {
-      splineq_near(dir, rsq, twoh, a, b, c, d);
-    } else {
-      const T dir2 = dir * dir;
-      a = dir;
-      b = dir2 * dir;
-      c = T(3) * b * dir2;
-      d = T(5) * c * dir2;
-    }
-    const T xx = rec[6], xy = rec[7], xz = rec[8], yy = rec[9], yz = rec[10], zz = rec[11];
-    const T qirx = xx * rx + xy * ry + xz * rz;
-    const T qiry = xy * rx + yy * ry + yz * rz;
-    const T qirz = xz * rx + yz * ry + zz * rz;
-    const T qir = T(0.5) * (qirx * rx + qiry * ry + qirz * rz);
-    const T tr = rec[5];
-    const T qir3 = b * M + d * qir - c * tr;
-    acc.pot -= M * a + c * qir - b * tr;
-    acc.ax -= qir3 * rx - c * qirx;
-    acc.ay -= qir3 * ry - c * qiry;
-    acc.az -= qir3 * rz - c * qirz;
-    acc.idt2 = max_t(acc.idt2, (tmass + M) * b);
-  }
-}
-
-/* One source particle on one target (gravity.h:276-301 /
- * HostCUDA.cu:1654-1711).  rec: {sx, sy, sz, m, soft}; r = s - target. */
-template <typename T>
-__device__ __forceinline__ void pp_interact(const T* rec, T tx, T ty, T tz, T tsoft, T tmass,
-                                            Acc<T>& acc) {
-  const T rx = rec[0] - tx, ry = rec[1] - ty, rz = rec[2] - tz;
-  const T m = rec[3];
-  const T rsq = rx * rx + ry * ry + rz * rz;
-  if (rsq != T(0)) {
-    const T twoh = rec[4] + tsoft;
-    const T dir = rsqrt_t(rsq);
-    const T r1 = rsq * dir;
-    T a, b;
-    if (r1 < twoh) {
-      spline_near(r1, dir, twoh, a, b);
-    } else {
-      a = dir;
-      b = dir * dir * dir;
-    }
-    const T bm = b * m;
-    acc.pot -= m * a;
-    acc.ax += rx * bm;
-    acc.ay += ry * bm;
-    acc.az += rz * bm;
-    acc.idt2 = max_t(acc.idt2, (tmass + m) * b);
-  }
-}
 
 /* One hexadecapole cell on one target: momEvalFmomrcm (moments.c:
  * 1469-1525, CUDAMoments.cu:14-109) for the scaled reduced moments of the
@@ -199,8 +136,9 @@ struct FormT<kMix> {
   using A = double;
 };
 
-/* Builds the staged record of list entry e in dst. */
-template <int FORM, bool CELL, bool HEX = false>
+/* Builds the staged record of hexadecapole cell entry e in dst: {x y z M
+ * radius, then the 21 moments}. */
+template <int FORM>
 __device__ __forceinline__ void stage_entry(const ListArgs& a, int e, float3 chi, float3 clo,
                                             typename FormT<FORM>::T* dst) {
   const int2 ent = __ldg(a.list + e);
@@ -208,105 +146,42 @@ __device__ __forceinline__ void stage_entry(const ListArgs& a, int e, float3 chi
   if ((unsigned long long)idx >= (unsigned long long)a.n_src) idx = 0;  // memory safety
   const int code = (ent.y >> 22) & 0x1ff;
   const int ox = (code & 7) - 3, oy = ((code >> 3) & 7) - 3, oz = ((code >> 6) & 7) - 3;
-  if constexpr (FORM == kF32) {
-    const float fp = a.fperiod_f;
-    if constexpr (CELL) {
-      const float4* m = reinterpret_cast<const float4*>(
-          static_cast<const CudaMultipoleMoments*>(a.src) + idx);
-      const float4 m0 = __ldg(m), m1 = __ldg(m + 1), m2 = __ldg(m + 2);
-      // m0 {radius, soft, M, cm.x}  m1 {cm.y, cm.z, xx, xy}  m2 {xz, yy, yz, zz}
-      float4* d4 = reinterpret_cast<float4*>(dst);
-      d4[0] = make_float4((float)ox * fp + m0.w, (float)oy * fp + m1.x, (float)oz * fp + m1.y, m0.z);
-      d4[1] = make_float4(m0.y, 0.5f * (m1.z + m2.y + m2.w), m1.z, m1.w);
-      d4[2] = m2;
-    } else {
-      const CompactPartData* p = static_cast<const CompactPartData*>(a.src) + idx;
-      const float m = __ldg(&p->mass), s = __ldg(&p->soft);
-      const float px = __ldg(&p->position.x), py = __ldg(&p->position.y), pz = __ldg(&p->position.z);
-      float4* d4 = reinterpret_cast<float4*>(dst);
-      d4[0] = make_float4((float)ox * fp + px, (float)oy * fp + py, (float)oz * fp + pz, m);
-      d4[1] = make_float4(s, 0.f, 0.f, 0.f);
-    }
-  } else if constexpr (FORM == kF64) {
+  if constexpr (FORM == kF64) {
     const double fp = a.fperiod_d;
-    if constexpr (CELL && HEX) {
-      /* hexadecapole moments: 27 doubles per node */
-      const double* m = static_cast<const double*>(a.src) + 27 * idx;
-      dst[0] = (double)ox * fp + __ldg(m + 3);
-      dst[1] = (double)oy * fp + __ldg(m + 4);
-      dst[2] = (double)oz * fp + __ldg(m + 5);
-      dst[3] = __ldg(m + 2);
-      dst[4] = __ldg(m + 0);
+    const double* m = static_cast<const double*>(a.src) + 27 * idx;
+    dst[0] = (double)ox * fp + __ldg(m + 3);
+    dst[1] = (double)oy * fp + __ldg(m + 4);
+    dst[2] = (double)oz * fp + __ldg(m + 5);
+    dst[3] = __ldg(m + 2);
+    dst[4] = __ldg(m + 0);
 #pragma unroll
-      for (int k = 0; k < 21; ++k) dst[5 + k] = __ldg(m + 6 + k);
-    } else if constexpr (CELL) {
-      const double* m = static_cast<const double*>(a.src) + 12 * idx;
-      dst[0] = (double)ox * fp + __ldg(m + 3);
-      dst[1] = (double)oy * fp + __ldg(m + 4);
-      dst[2] = (double)oz * fp + __ldg(m + 5);
-      dst[3] = __ldg(m + 2);
-      dst[4] = __ldg(m + 1);
-      const double xx = __ldg(m + 6), xy = __ldg(m + 7), xz = __ldg(m + 8);
-      const double yy = __ldg(m + 9), yz = __ldg(m + 10), zz = __ldg(m + 11);
-      dst[5] = 0.5 * (xx + yy + zz);
-      dst[6] = xx;
-      dst[7] = xy;
-      dst[8] = xz;
-      dst[9] = yy;
-      dst[10] = yz;
-      dst[11] = zz;
-    } else {
-      const double* p = static_cast<const double*>(a.src) + 5 * idx;
-      dst[0] = (double)ox * fp + __ldg(p + 2);
-      dst[1] = (double)oy * fp + __ldg(p + 3);
-      dst[2] = (double)oz * fp + __ldg(p + 4);
-      dst[3] = __ldg(p + 0);
-      dst[4] = __ldg(p + 1);
-    }
+    for (int k = 0; k < 21; ++k) dst[5 + k] = __ldg(m + 6 + k);
   } else {  // kMix
+    /* packed cell, 8 float4: {hi.xyz, M} {lo.xyz, soft} {radius, xx, xy, xz}
+     * {yy, yz, xxx, xyy} {xxy, yyy, xxz, yyz} {xyz, xxxx, xyyy, xxxy}
+     * {yyyy, xxxz, yyyz, xxyy} {xxyz, xyyz, 0, 0}: words 2..7 carry the
+     * radius and the 21 moments in order */
     const float fp = a.fperiod_f;
     float4* d4 = reinterpret_cast<float4*>(dst);
-    if constexpr (CELL && HEX) {
-      /* packed hexadecapole cell, 8 float4: {hi.xyz, M} {lo.xyz, soft}
-       * {radius, xx, xy, xz} {yy, yz, xxx, xyy} {xxy, yyy, xxz, yyz}
-       * {xyz, xxxx, xyyy, xxxy} {yyyy, xxxz, yyyz, xxyy} {xxyz, xyyz, 0, 0} */
-      const float4* m = static_cast<const float4*>(a.src) + kCellHexPackF4 * idx;
-      const float4 h = __ldg(m), l = __ldg(m + 1);
-      const float sx = ((h.x - chi.x) + (float)ox * fp) + (l.x - clo.x);
-      const float sy = ((h.y - chi.y) + (float)oy * fp) + (l.y - clo.y);
-      const float sz = ((h.z - chi.z) + (float)oz * fp) + (l.z - clo.z);
-      d4[0] = make_float4(sx, sy, sz, h.w);
-      /* rec[4] = radius, rec[5..25] = the 21 moments: the packed words 2..7
-       * carry exactly that sequence */
+    const float4* m = static_cast<const float4*>(a.src) + kCellHexPackF4 * idx;
+    const float4 h = __ldg(m), l = __ldg(m + 1);
+    const float sx = ((h.x - chi.x) + (float)ox * fp) + (l.x - clo.x);
+    const float sy = ((h.y - chi.y) + (float)oy * fp) + (l.y - clo.y);
+    const float sz = ((h.z - chi.z) + (float)oz * fp) + (l.z - clo.z);
+    d4[0] = make_float4(sx, sy, sz, h.w);
 #pragma unroll
-      for (int w = 0; w < 6; ++w) d4[1 + w] = __ldg(m + 2 + w);
-    } else if constexpr (CELL) {
-      const float4* m = static_cast<const float4*>(a.src) + kCellPackF4 * idx;
-      const float4 h = __ldg(m), l = __ldg(m + 1), q0 = __ldg(m + 2), q1 = __ldg(m + 3);
-      const float sx = ((h.x - chi.x) + (float)ox * fp) + (l.x - clo.x);
-      const float sy = ((h.y - chi.y) + (float)oy * fp) + (l.y - clo.y);
-      const float sz = ((h.z - chi.z) + (float)oz * fp) + (l.z - clo.z);
-      d4[0] = make_float4(sx, sy, sz, h.w);
-      d4[1] = make_float4(l.w, q1.z, q0.x, q0.y);
-      d4[2] = make_float4(q0.z, q0.w, q1.x, q1.y);
-    } else {
-      const float4* p = static_cast<const float4*>(a.src) + kPartPackF4 * idx;
-      const float4 h = __ldg(p), l = __ldg(p + 1);
-      const float sx = ((h.x - chi.x) + (float)ox * fp) + (l.x - clo.x);
-      const float sy = ((h.y - chi.y) + (float)oy * fp) + (l.y - clo.y);
-      const float sz = ((h.z - chi.z) + (float)oz * fp) + (l.z - clo.z);
-      d4[0] = make_float4(sx, sy, sz, h.w);
-      d4[1] = make_float4(l.w, 0.f, 0.f, 0.f);
-    }
+    for (int w = 0; w < 6; ++w) d4[1 + w] = __ldg(m + 2 + w);
   }
 }
 
-template <int FORM, bool CELL, bool HEX = false>
-__global__ void __launch_bounds__(kThreads, 2) list_kernel(const ListArgs a) {
+/* Hexadecapole cell lists: the FP64 form, and the FP32-mixed form with
+ * synchronous staging (variant 0). */
+template <int FORM>
+__global__ void __launch_bounds__(kThreads, 2) list_kernel_hex(const ListArgs a) {
   using T = typename FormT<FORM>::T;
   using A = typename FormT<FORM>::A;
-  constexpr int RW = CELL ? (HEX ? 28 : 12) : 8;  // record width in T, multiple of 4
-  constexpr int SB = HEX ? 16 : 32;                // entries staged per block
+  constexpr int RW = 28;  // record width in T, multiple of 4
+  constexpr int SB = 16;  // entries staged per block
   __shared__ __align__(16) T stage[kWarps][SB * RW];
   __shared__ A red[kWarps][5][32];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -339,18 +214,10 @@ __global__ void __launch_bounds__(kThreads, 2) list_kernel(const ListArgs a) {
       const bool active = g < G;
       const long long ti = tbase + t0 + t;
 
-      T tx, ty, tz, tsoft, tmass;
-      if constexpr (FORM == kF32) {
-        const CompactPartData* p = static_cast<const CompactPartData*>(a.tgt) + ti;
-        tmass = __ldg(&p->mass);
-        tsoft = __ldg(&p->soft);
-        tx = __ldg(&p->position.x);
-        ty = __ldg(&p->position.y);
-        tz = __ldg(&p->position.z);
-      } else if constexpr (FORM == kF64) {
+      T tx, ty, tz, tmass;
+      if constexpr (FORM == kF64) {
         const double* p = static_cast<const double*>(a.tgt) + 5 * ti;
         tmass = __ldg(p);
-        tsoft = __ldg(p + 1);
         tx = __ldg(p + 2);
         ty = __ldg(p + 3);
         tz = __ldg(p + 4);
@@ -361,24 +228,21 @@ __global__ void __launch_bounds__(kThreads, 2) list_kernel(const ListArgs a) {
         ty = (h.y - chi.y) + (l.y - clo.y);
         tz = (h.z - chi.z) + (l.z - clo.z);
         tmass = h.w;
-        tsoft = l.w;
       }
 
-      /* running totals: plain for kF32/kF64, Kahan pairs for kMix */
+      /* running totals: plain for kF64, Kahan pairs for kMix */
       T sx = 0, sy = 0, sz = 0, sp = 0, idt2 = 0;
       float cx = 0.f, cy = 0.f, cz = 0.f, cp = 0.f;
 
       for (int e0 = e_begin; e0 < e_end; e0 += SB) {
         const int ne = min(SB, e_end - e0);
-        if (lane < ne) stage_entry<FORM, CELL, HEX>(a, e0 + lane, chi, clo, st + lane * RW);
+        if (lane < ne) stage_entry<FORM>(a, e0 + lane, chi, clo, st + lane * RW);
         __syncwarp();
         if (active) {
           Acc<T> acc{T(0), T(0), T(0), T(0), idt2};
 #pragma unroll 4
           for (int k = g; k < ne; k += G) {
-            if constexpr (CELL && HEX) hex_interact<T>(st + k * RW, tx, ty, tz, tmass, acc);
-            else if constexpr (CELL) pc_interact<T>(st + k * RW, tx, ty, tz, tsoft, tmass, acc);
-            else pp_interact<T>(st + k * RW, tx, ty, tz, tsoft, tmass, acc);
+            hex_interact<T>(st + k * RW, tx, ty, tz, tmass, acc);
           }
           idt2 = acc.idt2;
           if constexpr (FORM == kMix) {
@@ -422,21 +286,12 @@ __global__ void __launch_bounds__(kThreads, 2) list_kernel(const ListArgs a) {
           ri = max_t(ri, red[warp][4][l]);
         }
         const long long to = tbase + t0 + lane;
-        if constexpr (FORM == kF32) {
-          VariablePartData* v = static_cast<VariablePartData*>(a.vars) + to;
-          v->a.x += rx;
-          v->a.y += ry;
-          v->a.z += rz;
-          v->potential += rp;
-          v->dtGrav = fmaxf(ri, v->dtGrav);
-        } else {
-          double* v = static_cast<double*>(a.vars) + 5 * to;
-          v[0] += rx;
-          v[1] += ry;
-          v[2] += rz;
-          v[3] += rp;
-          v[4] = fmax(ri, v[4]);
-        }
+        double* v = static_cast<double*>(a.vars) + 5 * to;
+        v[0] += rx;
+        v[1] += ry;
+        v[2] += rz;
+        v[3] += rp;
+        v[4] = fmax(ri, v[4]);
       }
       __syncwarp();
     }
@@ -2517,7 +2372,7 @@ template <int FORM, bool CELL>
 cudaError_t launch_t(const ListArgs& a, cudaStream_t s) {
   if constexpr (FORM == kF64) {
     static std::atomic<int> occ{0};
-    return launch_kernel(list_kernel<FORM, CELL>, &occ, list_kernel_id(FORM, CELL), a, s);
+    return launch_block(list_kernel_f64<CELL>, kF64Threads, &occ, list_kernel_id(FORM, CELL), a, s);
   } else if constexpr (kHexDropIn && FORM == kF32 && CELL) {
     static std::atomic<int> occ{0};
     return launch_kernel(list_kernel_hex2<kF32, 2>, &occ, list_kernel_id(kF32, true), a, s);
@@ -2587,14 +2442,14 @@ cudaError_t launch_pack_cells(const double* moments, long long n, float4* out, c
 }
 
 /* hexadecapole FP32-mixed cell kernel: 0 synchronous staging
- * (list_kernel<kMix, true, true>), 1/2 paired (list_kernel_hex2, 1/2
+ * (list_kernel_hex<kMix>), 1/2 paired (list_kernel_hex2, 1/2
  * resident blocks per SM) */
 std::atomic<int> g_hex_variant{2};
 
 cudaError_t launch_list_hex(int form, const ListArgs& a, cudaStream_t s) {
   if (form == kF64) {
     static std::atomic<int> occ{0};
-    return launch_kernel(list_kernel<kF64, true, true>, &occ, list_kernel_id(kF64, true), a, s);
+    return launch_kernel(list_kernel_hex<kF64>, &occ, list_kernel_id(kF64, true), a, s);
   }
   if (form == kMix) {
     const int kid = list_kernel_id(kMix, true);
@@ -2608,7 +2463,7 @@ cudaError_t launch_list_hex(int form, const ListArgs& a, cudaStream_t s) {
       return launch_kernel(list_kernel_hex2<kMix, 2>, &occ, kid, a, s);
     }
     static std::atomic<int> occ{0};
-    return launch_kernel(list_kernel<kMix, true, true>, &occ, kid, a, s);
+    return launch_kernel(list_kernel_hex<kMix>, &occ, kid, a, s);
   }
   return cudaErrorInvalidValue;
 }

@@ -113,3 +113,95 @@ def test_far_first_kernels_at_tile_edges(cuda_ok, variant, masses, period):
         assert relp.max() < 1e-4 and np.median(relp[pot > 0]) < 1e-6, relp.max()
         np.testing.assert_allclose(v[:, 4], ref[:, 4], rtol=4e-4)
         assert not v[acc == 0, :3].any() or np.abs(v[acc == 0, :3]).max() < 1e-20
+
+
+@pytest.mark.parametrize("masses", ["one", "several"])
+@pytest.mark.parametrize("period", [0.0, 1.0])
+def test_fp64_kernel_at_tile_edges(cuda_ok, masses, period):
+    """The plain FP64 form over the same sizes and lengths, buckets of more
+    targets than a CTA has threads, and coincident sources and targets."""
+    import torch
+    rng = np.random.default_rng(20261207)
+    sizes = np.array([s for s in SIZES + [255, 256, 257, 300] for _ in LENGTHS], np.int32)
+    n = int(sizes.sum()) + 100
+    parts = np.empty((n, 5))
+    parts[:, 0] = 1.0 / n if masses == "one" else rng.choice([1.0, 3.0, 7.5], n) / n
+    parts[:, 1] = rng.choice([0.0, 1e-3, 0.02, 0.1], n)
+    parts[:, 2:] = rng.uniform(-0.5, 0.5, (n, 3))
+    at = 0
+    for size in sizes:
+        parts[at:at + size, 2:] = rng.uniform(-0.5, 0.5, 3) + rng.uniform(-0.02, 0.02, (size, 3))
+        at += size
+    nm = 512
+    mom = np.zeros((nm, 12))
+    mom[:, 0], mom[:, 1] = 0.05, rng.choice([0.0, 1e-3, 0.1], nm)
+    mom[:, 2] = rng.uniform(0.5, 2.0, nm) / nm
+    mom[:, 3:6] = rng.uniform(-0.5, 0.5, (nm, 3))
+    mom[:64, 3:6] = parts[rng.integers(0, at, 64), 2:]  # cells centred on a target
+    mom[:, 6:] = rng.uniform(-1e-4, 1e-4, (nm, 6)) * mom[:, 2:3]
+    lib = N.cuda_lib()
+    dp, dm = torch.from_numpy(parts).cuda(), torch.from_numpy(mom).cuda()
+    for cell in (False, True):
+        n_src, host = (nm, mom) if cell else (n, parts)
+        req = request(rng, n_src, period)
+        more = sizes[len(req.sizes):]
+        lens = np.tile(LENGTHS, len(more) // len(LENGTHS))
+        lst = np.zeros((int(lens.sum()), 2), np.int32)
+        lst[:, 0] = rng.integers(0, n_src, len(lst))
+        lst[:, 1] = (3 | 3 << 3 | 3 << 6) << 22
+        req = ListRequest(np.concatenate([req.list, lst]),
+                          np.concatenate([req.markers, req.markers[-1] + np.cumsum(lens)])
+                          .astype(np.int32),
+                          np.concatenate([[0], np.cumsum(sizes)[:-1]]).astype(np.int32), sizes,
+                          np.arange(len(sizes), dtype=np.int32))
+        ref = (oracle.cell_forces if cell else oracle.part_forces)(host, parts, req, fperiod=period)
+        v = torch.zeros((n, 5), dtype=torch.float64, device="cuda")
+        r, keep = device(req)
+        call = lib.changa_cell_forces_fp64 if cell else lib.changa_part_forces_fp64
+        N.check(call((dm if cell else dp).data_ptr(), n_src, dp.data_ptr(), n, C.byref(r), period,
+                     v.data_ptr(), torch.cuda.current_stream().cuda_stream))
+        v = v.cpu().numpy()
+        col = (2, slice(3, 6)) if cell else (0, slice(2, 5))
+        acc, pot = bound(req, host[:, col[0]], host[:, col[1]], parts[:, 2:], 1e-5, period)
+        # separations are exact differences of coordinates below 2 to 2^-53,
+        # at distances of 1e-5 and more (closer pairs are softened or rare)
+        assert np.isfinite(v).all()
+        ok = np.isfinite(ref).all(1)  # the oracle divides by r = 0 for a cell on its target
+        assert ok.sum() >= n - 64
+        assert (np.abs(v - ref)[ok, :3].max(1) / np.maximum(acc[ok], 1e-30)).max() < 1e-9
+        assert (np.abs(v - ref)[ok, 3] / np.maximum(pot[ok], 1e-30)).max() < 1e-9
+        np.testing.assert_allclose(v[ok, 4], ref[ok, 4], rtol=1e-9)
+
+
+@pytest.mark.parametrize("cut,n_rep", [(2.6, 1), (2.6, 2), (4.6, 1)])
+@pytest.mark.parametrize("whole", [True, False])
+def test_ewald_fp64_replicas_and_tables(cuda_ok, cut, n_rep, whole):
+    """The FP64 Ewald term with more replicas than one culled batch, a ragged
+    particle count, and a table whose vectors are not whole (which takes the
+    sine and cosine of each)."""
+    import torch
+    from changa_gb300 import gravity
+    rng = np.random.default_rng(5)
+    n = 1001
+    parts = np.empty((n, 5))
+    parts[:, 0], parts[:, 1] = 1.0 / n, 1e-3
+    parts[:, 2:] = rng.uniform(0, 1, (n, 3)) ** 2
+    m = parts[:, 0]
+    cm = (m[:, None] * parts[:, 2:]).sum(0) / m.sum()
+    d = parts[:, 2:] - cm
+    q = np.einsum("n,ni,nj->ij", m, d, d)
+    root = np.array([0.8, 1e-3, m.sum(), *cm, q[0, 0], q[0, 1], q[0, 2], q[1, 1], q[1, 2], q[2, 2]])
+    ref = oracle.ewald_forces(parts, root, 1.0, n_rep, cut, 2.8)
+    p = gravity.EwaldConfig(1.0, n_rep, cut, 2.8).params(root)
+    if not whole:
+        p._keep[:, :3] *= 1 + 1e-12
+    dp = torch.from_numpy(parts).cuda()
+    v = torch.zeros((n, 5), dtype=torch.float64, device="cuda")
+    N.check(N.cuda_lib().changa_ewald_forces(N.CHANGA_FORM_FP64, dp.data_ptr(), n, None, n,
+                                             C.byref(p), v.data_ptr(),
+                                             torch.cuda.current_stream().cuda_stream))
+    v = v.cpu().numpy()
+    # the tables differ by 1e-12; near the root the recursion of the g_n loses
+    # up to (alpha r)^-6 = (4 * 1.2e-3)^-3 of 2^-53 of the O(1) terms
+    assert np.abs(v[:, :4] - ref[:, :4]).max() < 1e-8
+    assert np.median(np.abs(v[:, :4] - ref[:, :4])) < 1e-11
