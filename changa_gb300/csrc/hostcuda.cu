@@ -151,8 +151,20 @@ static void signal(cudaStream_t s, void* cb) {
 
 static size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
-constexpr size_t kDefaultHostChunkBytes = size_t(256) << 20;
-static std::atomic<size_t> g_host_chunk_bytes{kDefaultHostChunkBytes};
+/* Bytes per upload chunk of a list of `bytes`: the caller's setting
+ * (changa_gb300_set_host_chunk_bytes), else an eighth of the list, between 32
+ * and 256 MiB, so that the upload of a list of a few hundred MB overlaps its
+ * kernels too.  Each chunk's kernel drains for about a bucket's time, so
+ * chunks below 32 MiB lose more than they overlap.  us per call with chunks
+ * of 256 / 64 / 32 / 16 / 8 MiB: runs entry, 2^20 particles (208 MB of
+ * cells) 4190 / 3540 / 3595 / 3784 / 4144; drop-in, 500009 particles (110 MB
+ * and 240 MB of lists) 3470 / 3613 / 2557 / 2952 / 3391. */
+constexpr size_t kMinHostChunkBytes = size_t(32) << 20, kMaxHostChunkBytes = size_t(256) << 20;
+static std::atomic<size_t> g_host_chunk_bytes{0};
+static size_t host_chunk_bytes(size_t bytes) {
+  if (const size_t set = g_host_chunk_bytes.load()) return set;
+  return std::min(kMaxHostChunkBytes, std::max(kMinHostChunkBytes, bytes / 8));
+}
 
 /* The library-owned streams of the host-array entries on each device
  * (created once): which 0 carries the uploads, which 1 the read-backs, so
@@ -301,7 +313,8 @@ static int run_request_chunked(CudaRequest* r, bool cell, const void* sources, l
     a.n_tgt = n_tgt;
     a.vars = r->d_localVars;
     a.list = d.list;
-    a.n_entries = e1 > e0 ? e1 : e0;  // entries past this chunk have not landed yet
+    /* entries past this chunk have not landed yet; none lie past the list */
+    a.n_entries = std::min<long long>(e1 > e0 ? e1 : e0, r->numInteractions);
     a.markers = d.markers + b0;
     a.starts = d.starts + b0;
     a.sizes = d.sizes + b0;
@@ -340,8 +353,14 @@ static int run_request(CudaRequest* r, bool cell, const void* sources, long long
                                      r->bucketStarts, r->bucketSizes, nb, n_src, n_tgt);
     if (rc) return record_error(rc, "request validation", __FILE__, __LINE__);
   }
-  /* a list of more than two chunks streams in chunk by chunk */
-  const long long per = (long long)(g_host_chunk_bytes.load() / sizeof(ILCell));
+  /* a list of more than two chunks streams in chunk by chunk; under capture
+   * every copy stays on the request's stream (the library's copy stream is
+   * not part of the capture) unless the list is past the largest chunks */
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  CHG_CUDA(cudaStreamIsCapturing(r->stream, &capture));
+  size_t chunk = host_chunk_bytes((size_t)std::max(0, r->numInteractions) * sizeof(ILCell));
+  if (capture != cudaStreamCaptureStatusNone) chunk = std::max(chunk, kMaxHostChunkBytes);
+  const long long per = (long long)(chunk / sizeof(ILCell));
   if (r->numInteractions > 2 * per) {
     cudaStream_t c = library_stream();
     if (c) return run_request_chunked(r, cell, sources, n_src, n_tgt, nb, per, c);
@@ -1145,7 +1164,7 @@ int changa_gravity_step_hexa(int form, const double* moments, long long n_moment
 }
 
 void changa_gb300_set_host_chunk_bytes(size_t bytes) {
-  g_host_chunk_bytes.store(bytes == 0 ? kDefaultHostChunkBytes : bytes < 4096 ? 4096 : bytes);
+  g_host_chunk_bytes.store(bytes == 0 ? 0 : bytes < 4096 ? 4096 : bytes);
 }
 
 /* Page-locked (or registered) host memory: a read-back into it returns at
@@ -1177,7 +1196,7 @@ static std::pair<long long, long long> target_range(const ChangaListRequest* r, 
 /* Host-array evaluation, pipelined: the particles go first, in slices that
  * the compute stream packs and gives their Ewald term as they land; then
  * the moments and the small arrays, then each interaction list in chunks of
- * about kChunkBytes, all on a copy stream.  The compute stream packs the
+ * about host_chunk_bytes(), all on a copy stream.  The compute stream packs the
  * moments and launches the list kernel on each chunk's bucket range as
  * soon as its entries have landed, so the list stream from host memory
  * overlaps the force arithmetic.  The last list's
@@ -1218,7 +1237,6 @@ static int step_host_impl(int form, const double* moments, long long n_moments,
   const int f = form == CHANGA_FORM_FP64 ? kF64 : kMix;
   cudaStream_t c = library_stream();
   if (!c) return record_error(cudaErrorUnknown, "gravity_step_host: copy stream", __FILE__, __LINE__);
-  const size_t kChunkBytes = g_host_chunk_bytes.load();
 
   cudaStream_t rb = library_stream(1);
   if (!rb) return record_error(cudaErrorUnknown, "gravity_step_host: copy stream", __FILE__, __LINE__);
@@ -1237,9 +1255,13 @@ static int step_host_impl(int form, const double* moments, long long n_moments,
       rview = pview;
       rview.markers = pruns->run_markers;
       rview.n_entries = pruns->n_runs;
-      list_chunks(&rview, (long long)(kChunkBytes / sizeof(ILPart)), k == last, chunks[k]);
+      list_chunks(&rview,
+                  (long long)(host_chunk_bytes((size_t)pruns->n_runs * sizeof(ILPart)) / sizeof(ILPart)),
+                  k == last, chunks[k]);
     } else {
-      list_chunks(r, (long long)(kChunkBytes / sizeof(ILCell)), k == last, chunks[k]);
+      list_chunks(r,
+                  (long long)(host_chunk_bytes((size_t)r->n_entries * sizeof(ILCell)) / sizeof(ILCell)),
+                  k == last, chunks[k]);
     }
   }
 
@@ -1290,7 +1312,7 @@ static int step_host_impl(int form, const double* moments, long long n_moments,
   std::vector<std::pair<long long, long long>> slices;
   {
     const long long per =
-        std::max<long long>(32, (long long)(kChunkBytes / 4 / (5 * sizeof(double))) & ~31LL);
+        std::max<long long>(32, (long long)(host_chunk_bytes(pb) / 4 / (5 * sizeof(double))) & ~31LL);
     for (long long a = 0; a < n_parts; a += per) slices.push_back({a, std::min(n_parts, a + per)});
   }
 

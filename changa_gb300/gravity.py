@@ -16,6 +16,7 @@ Three ways in, all through ``libchanga_gb300.so``:
 from __future__ import annotations
 
 import ctypes as C
+import functools
 import math
 
 import numpy as np
@@ -29,6 +30,7 @@ def _p(a):
     return a.ctypes.data_as(C.c_void_p)
 
 
+@functools.cache
 def _cudart():
     """The CUDA runtime (for cudaFree / cudaStreamSynchronize of buffers the
     drop-in entry points allocate, as ChaNGa's DataManager does)."""

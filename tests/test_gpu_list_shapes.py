@@ -205,3 +205,44 @@ def test_ewald_fp64_replicas_and_tables(cuda_ok, cut, n_rep, whole):
     # up to (alpha r)^-6 = (4 * 1.2e-3)^-3 of 2^-53 of the O(1) terms
     assert np.abs(v[:, :4] - ref[:, :4]).max() < 1e-8
     assert np.median(np.abs(v[:, :4] - ref[:, :4])) < 1e-11
+
+
+@pytest.mark.parametrize("extra", [-1, 0, 1, 40000])
+def test_dropin_list_around_two_default_chunks(cuda_ok, extra):
+    """A drop-in list of just under, at and over two default upload chunks
+    (32 MiB for lists this long), against the same list in one upload.  The
+    sources lie in one octant of every target at separations above 0.4, so
+    nothing cancels: a block of 32 terms is summed in FP32 (32 x 2^-24 = 2e-6
+    of the sum) before it joins the compensated total, and twice that for two
+    orders of summation is below 1e-5."""
+    from types import SimpleNamespace
+    from changa_gb300 import gravity
+    rng = np.random.default_rng(5)
+    n_entries, nb, nt, n = (8 << 20) + extra, 4001, 8, 40000
+    n_tgt = nb * nt
+    pos = rng.uniform(0.5, 1.0, (n, 3))
+    pos[:n_tgt] = rng.uniform(0.0, 0.05, (n_tgt, 3))
+    parts = np.concatenate([np.full((n, 1), 1.0 / n), np.full((n, 1), 1e-3), pos], 1).astype(np.float32)
+    lst = np.empty((n_entries, 2), np.int32)
+    lst[:, 0] = rng.integers(n_tgt, n, n_entries)
+    lst[:, 1] = 0x49 * 3 << 22  # the replica at the origin
+    markers = np.linspace(0, n_entries, nb + 1).astype(np.int32)
+    starts = np.arange(nb, dtype=np.int32) * nt
+    sizes = np.full(nb, nt, np.int32)
+    empty = ListRequest(np.empty((0, 2), np.int32), np.zeros(1, np.int32), np.empty(0, np.int32),
+                        np.empty(0, np.int32), np.empty(0, np.int32))
+    inp = gravity.DropInInputs(SimpleNamespace(
+        n=n, order=2, period=0.0, plist=ListRequest(lst, markers, starts, sizes, np.arange(nb)),
+        cells=empty, abi_moments=lambda: np.zeros((4, 12), np.float32), abi_parts=lambda: parts))
+    lib = N.cuda_lib()
+    try:
+        got = gravity.dropin_step(inp).copy()
+        lib.changa_gb300_set_host_chunk_bytes(1 << 30)
+        try:
+            whole = gravity.dropin_step(inp).copy()
+        finally:
+            lib.changa_gb300_set_host_chunk_bytes(0)  # the default
+    finally:
+        inp.free()
+    assert (whole[:n_tgt, :3] > 0).all() and not whole[n_tgt:].any()
+    np.testing.assert_allclose(got, whole, rtol=1e-5)
