@@ -28,18 +28,18 @@
  *
  * Decisions equal the host walk's FP64 decisions.  GB300 issues FP64 at a
  * small fraction of its FP32 rate, so each opening test is first made in
- * FP32 from rounded copies of the node data, with a bound on how far the
- * FP32 distance can lie from the FP64 one: the clipped box distance and the
- * farthest-corner distance are 1-Lipschitz in the coordinates, so an input
- * error of delta moves a squared distance g^2 by at most 2 g delta +
- * delta^2.  Only tests whose FP32 value lies within that margin of the
- * threshold are repeated in FP64, with the host's expressions (this file is
- * compiled without FMA contraction, as the host code is).
+ * FP32 with a bound on how far the FP32 distance can lie from the FP64 one
+ * (open_criterion_screened).  Only tests whose FP32 value lies within that
+ * margin of the threshold are repeated in FP64, with the host's expressions
+ * (this file is compiled without FMA contraction, as the host code is).
  */
+#include <algorithm>
 #include <atomic>
 #include <cstring>
 #include <type_traits>
 #include <vector>
+
+#include <cuda_bf16.h>
 
 #include "chg_internal.h"
 #include "list_eval.cuh"
@@ -51,7 +51,7 @@ constexpr int kWalkWarps = 4;      // warps (buckets) per block
 constexpr int kWarpStack = 512;    // stack entries per warp (the deepest seen: 211)
 constexpr int kWarpStackLarge = 1024;  // the re-run after a warp exhausted kWarpStack
 constexpr int kChunk = 256;        // entries per pool chunk of the append pass
-constexpr int kMaxChunks = 128;    // chunks per bucket and list in the append pass
+constexpr int kHere = 3 | (3 << 3) | (3 << 6);  // replica code of no offset
 enum { kCount = 0, kFill = 1, kAppend = 2 };
 
 struct WalkArgs {
@@ -87,11 +87,13 @@ struct WalkArgs {
   long long pool_chunks[3];
   int* overflow;
   int bucket_stride;
-  /* per node, one 32-byte record for the traversal (see WalkNode) */
+  /* per node, what the traversal reads (see WalkNode) */
   const struct WalkNode* nodes;
-  const float4* boxf;   // 2 n_nodes: {lesser.xyz, 0}, {greater.xyz, 0}
-  const float2* hexf;   // n_nodes: {softening, monopole opening radius^2} (hexadecapole rules)
+  const struct WalkBox* boxes;
+  const float4* boxf;   // order 4: 2 n_nodes, {lesser.xyz, 0}, {greater.xyz, 0}
+  const float2* hexf;   // order 4: n_nodes, {softening, monopole opening radius^2}
   float period32;
+  float e_rep;          // what a replica offset adds to the screen's margin
   /* two-phase walk.  Groups: nodes whose subtree holds few buckets (each
    * bucket in exactly one group, the group node on its chain).  Phase 1
    * walks a group node's chain once for all its buckets: its units are the
@@ -103,31 +105,75 @@ struct WalkArgs {
   const int* group_node;     // n_groups
   int n_groups;
   const int* bucket_group;   // n_buckets: group of each bucket
-  int* n_front;              // phase 1 count pass: frontier entries per group
-  const long long* off_front;  // phase 1 fill pass: frontier offsets; phase 2: CSR over groups
-  int2* front;               // phase 1 fill pass output, phase 2 input: {node, replica code}
-  const long long* pre_off[2];  // phase 2: CSR over groups of the prefix cells / particles
-  const int2* pre[2];
+  int* n_front;              // phase 1: frontier entries per group
+  const long long* off_front;  // phase 1 fill pass: frontier offsets
+  int2* front;               // phase 1 output: {node, replica code}
+  /* Phase 1 in one traversal (append mode): group g's prefix cells, prefix
+   * particles and frontier go to slots of slot[k] entries at g slot[k]; a
+   * group that needs more sets *slot_over and is walked again by count and
+   * fill.  Phase 2 reads list k of group g at goff[k][g] (goff[k] null: at
+   * g slot[k]), gcnt[k][g] entries. */
+  int slot[3];
+  int* slot_over;
+  const long long* goff[3];
+  const int* gcnt[3];
+  const int2* glist[3];
 };
 
-/* What the traversal reads of a source node, in one 32-byte record (two
- * 16-byte loads from one sector): FP32 centre and opening radius^2 for the
- * screened test, then {child0, child1, first, count}. */
+/* What the traversal reads of a source node, in one 32-byte record: its
+ * centre as a sum of two parts per axis, the high in FP32 and the low in
+ * BF16, and its opening radius^2 for the screened test (infinite for the at
+ * most 6 particles that are always opened); and a, b: a bucket's ~first and
+ * count, else its one or two children (b -1 when there is one). */
 struct __align__(32) WalkNode {
-  float4 geo;
-  int4 link;
+  float4 geo;   // centre, high parts; opening radius^2
+  int a, b;
+  unsigned low_xy, low_z;  // low parts: x in the low half, y in the high; z in the high
 };
 
+/* The same of a local node: its box's centre (two parts per axis), half
+ * extents, and the margin E of tests against it (BF16, rounded up). */
+struct __align__(32) WalkBox {
+  float4 mid;   // centre, high parts; low parts of x and y as in WalkNode
+  float4 half;  // half extents; low part of z in the high half, E in the low half
+};
+
+__device__ __forceinline__ float bf_lo(unsigned v) { return __uint_as_float(v << 16); }
+__device__ __forceinline__ float bf_hi(unsigned v) { return __uint_as_float(v & 0xffff0000u); }
+/* v rounded to BF16 (up: to the next one not below a positive v), as its 16 bits. */
+__device__ __forceinline__ unsigned to_bf(float v) {
+  return (unsigned)__bfloat16_as_ushort(__float2bfloat16_rn(v));
+}
+__device__ __forceinline__ unsigned to_bf_up(float v) {
+  return (unsigned)__bfloat16_as_ushort(__float2bfloat16_ru(v));
+}
 
 constexpr float kU = 5.9604645e-08f;  // 2^-24, the FP32 unit roundoff
 
-/* Each node's traversal record (FP32 centre and opening radius squared,
- * the latter formed in FP64 exactly as open_criterion forms it, and its
- * links) and its FP32 box. */
+/* The screened test's margins.  With u = 2^-24, a value x split into an FP32
+ * and a BF16 part is within 2^-33 |x| of their sum (an infinity or a part below
+ * the normal range aside, which the 1e-37 in E and the FP64 test cover).  The
+ * difference of two split centres D = (c_hi - m_hi) + (c_lo - m_lo) is then
+ * within 2.1 u |delta| + 2^-32 (|c| + |m|) of delta = c - m, and |c| <= |m| +
+ * |delta|.  A box distance g = |delta| - h (h rounded to FP32) or a far
+ * distance |delta| + h is within 4 u g + eps with eps = 4 u h + 2^-30 (|m| + h),
+ * which also covers the FP64 path's own rounding; a replica offset o adds
+ * 4 u |o| to eps.  Since 2 g eps <= w g^2 + eps^2 / w, with w = 2^-13 a sum v of
+ * three squares is within 1.3e-4 v + E of its FP64 value, E = 3 (2^13 + 2)
+ * eps^2, and the 7e-6 by which 1.3e-4 exceeds 2^-13 covers the rounding of the
+ * sums, of the FP32 threshold and of the comparison.  E is kept twice that, so
+ * that the offset's part may be added to it: (a + b)^2 <= 2 a^2 + 2 b^2. */
+constexpr float kScreen = 1.3e-4f;
+constexpr double kScreenE = 2.0 * 3.0 * 8200.0;
+
+/* Each node's traversal records; the opening radius squared is formed in FP64
+ * exactly as open_criterion forms it.  Under the hexadecapole rules also the
+ * FP32 box, softening and monopole radius. */
 __global__ void walk_prep_kernel(const double* __restrict__ geom, const double* __restrict__ bbox,
                                  const int* __restrict__ info, long long n_nodes, double theta,
                                  double theta_mono, WalkNode* __restrict__ nodes,
-                                 float4* __restrict__ boxf, float2* __restrict__ hexf) {
+                                 WalkBox* __restrict__ boxes, float4* __restrict__ boxf,
+                                 float2* __restrict__ hexf) {
   for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < n_nodes;
        g += (long long)gridDim.x * blockDim.x) {
     const double* gg = geom + 6 * g;
@@ -135,25 +181,52 @@ __global__ void walk_prep_kernel(const double* __restrict__ geom, const double* 
     double radius = kOpenGeom * gg[3] / theta;
     if (radius < gg[3]) radius = gg[3];
     const int* f = info + 4 * g;
-    nodes[g].geo = make_float4((float)gg[0], (float)gg[1], (float)gg[2], (float)(radius * radius));
-    nodes[g].link = make_int4(f[0], f[1], f[2], f[3]);
+    const float r2 = f[3] <= 6 ? __int_as_float(0x7f800000) : (float)(radius * radius);
+    const float cx = (float)gg[0], cy = (float)gg[1], cz = (float)gg[2];
+    WalkNode nd;
+    nd.geo = make_float4(cx, cy, cz, r2);
+    nd.low_xy = to_bf((float)(gg[0] - cx)) | to_bf((float)(gg[1] - cy)) << 16;
+    nd.low_z = to_bf((float)(gg[2] - cz)) << 16;
+    if (f[0] < 0 && f[1] < 0) {
+      nd.a = ~f[2];
+      nd.b = f[3];
+    } else {
+      nd.a = f[0] >= 0 ? f[0] : f[1];
+      nd.b = f[0] >= 0 ? f[1] : -1;
+    }
+    nodes[g] = nd;
     const double* b = bbox + 6 * g;
-    boxf[2 * g] = make_float4((float)b[0], (float)b[1], (float)b[2], 0.0f);
-    boxf[2 * g + 1] = make_float4((float)b[3], (float)b[4], (float)b[5], 0.0f);
-    /* the monopole radius as open_criterion forms it, squared in FP64 */
-    const double rm = kOpenGeom * gg[3] / theta_mono;
-    hexf[g] = make_float2((float)gg[4], (float)(rm * rm));
+    double m[3], h[3], mx = 0.0, hx = 0.0;
+    for (int k = 0; k < 3; ++k) {
+      m[k] = 0.5 * (b[k] + b[3 + k]);
+      h[k] = 0.5 * (b[3 + k] - b[k]);
+      mx = fmax(mx, fabs(m[k]));
+      hx = fmax(hx, fabs(h[k]));
+    }
+    const double u = kU, eps = 4.0 * u * hx + 64.0 * u / 65536.0 * (mx + hx);
+    const float px = (float)m[0], py = (float)m[1], pz = (float)m[2];
+    const unsigned lxy = to_bf((float)(m[0] - px)) | to_bf((float)(m[1] - py)) << 16;
+    const unsigned lze = to_bf((float)(m[2] - pz)) << 16 | to_bf_up((float)(kScreenE * eps * eps + 1e-37));
+    WalkBox bx;
+    bx.mid = make_float4(px, py, pz, __uint_as_float(lxy));
+    bx.half = make_float4((float)h[0], (float)h[1], (float)h[2], __uint_as_float(lze));
+    boxes[g] = bx;
+    if (boxf) {
+      boxf[2 * g] = make_float4((float)b[0], (float)b[1], (float)b[2], 0.0f);
+      boxf[2 * g + 1] = make_float4((float)b[3], (float)b[4], (float)b[5], 0.0f);
+      /* the monopole radius as open_criterion forms it, squared in FP64 */
+      const double rm = kOpenGeom * gg[3] / theta_mono;
+      hexf[g] = make_float2((float)gg[4], (float)(rm * rm));
+    }
   }
 }
 
-/* v <= r2 decided from an FP32 value v within e of the FP64 one and r2 =
- * rn32 of the FP64 threshold: 1 certainly, 0 certainly not, -1 too close.
- * The margins carry one extra unit roundoff for the rounding of the two
- * sums compared here; NaN or infinity give -1. */
+/* v <= r2 decided from an FP32 sum of squares v with margin e and r2 = rn32
+ * of the FP64 threshold: 1 certainly, 0 certainly not, -1 too close; NaN or
+ * infinity give -1 (an infinite r2 alone gives 1). */
 __device__ __forceinline__ int screen_le(float v, float e, float r2) {
-  const float er = 2.0f * kU * r2;
-  if (v + e < r2 - er) return 1;
-  if (v - e > r2 + er) return 0;
+  if (fmaf(v, 1.0f + kScreen, e) < r2) return 1;
+  if (fmaf(v, 1.0f - kScreen, -e) > r2) return 0;
   return -1;
 }
 
@@ -196,12 +269,11 @@ __device__ __forceinline__ int screen_le_t(float v, float ev, float t, float et)
 
 /* open_softening in FP32 for a source g at c = cm + offset (FP32, with
  * the per-axis inputs cm and o for the error bound) against node `node`:
- * 1 certainly true, 0 certainly false, -1 too close to call.  Errors as in
- * open_criterion_screened: per axis the FP32 inputs and their sums carry at
- * most delta = 6u (|cm| + |o| + |node's cm or box face|) against the FP64
+ * 1 certainly true, 0 certainly false, -1 too close to call.  Per
+ * axis the FP32 inputs and their sums carry at most delta = 6u (|cm| + |o| + |node's cm or box face|) against the FP64
  * values; the softening sums 2 s_g + 2 s_node carry at most 3u of their
  * value, so their square at most 7u (bounded here by 8u). */
-__device__ int open_softening_screened(const WalkArgs& a, float sg, const float* c,
+__device__ __noinline__ int open_softening_screened(const WalkArgs& a, float sg, const float* c,
                                        const float* cm, const float* o, int node) {
   const float4 nc = a.nodes[node].geo;
   const float sn = a.hexf[node].x;
@@ -233,7 +305,7 @@ __device__ int open_softening_screened(const WalkArgs& a, float sg, const float*
 
 /* open_softening for source g at replica code `off` against node `node`:
  * the FP32 screen, then the FP64 test when too close to call. */
-__device__ bool open_softening_fast(const WalkArgs& a, int g, int off, int node) {
+__device__ __noinline__ bool open_softening_fast(const WalkArgs& a, int g, int off, int node) {
   const float4 gf = a.nodes[g].geo;
   const float cm[3] = {gf.x, gf.y, gf.z};
   const float o[3] = {(float)((off & 7) - 3) * a.period32, (float)(((off >> 3) & 7) - 3) * a.period32,
@@ -250,7 +322,8 @@ __device__ bool open_softening_fast(const WalkArgs& a, int g, int off, int node)
 
 /* openCriterionNode (gravity.h:652-723), quadrupole and hexadecapole
  * forms: 1 open, -1 undecided, 0 accept. */
-__device__ int open_criterion(const WalkArgs& a, int g, int local, bool local_bucket, int off) {
+__device__ __noinline__ int open_criterion(const WalkArgs& a, int g, int local, bool local_bucket,
+                                          int off) {
   const int count = a.info[4 * (size_t)g + 3];
   if (count <= 6) return 1;
   const double* gg = a.geom + 6 * (size_t)g;
@@ -282,59 +355,51 @@ __device__ int open_criterion(const WalkArgs& a, int g, int local, bool local_bu
   return d2 <= rm * rm ? 1 : 0;
 }
 
-/* open_criterion screened in FP32.  Per axis the FP32 inputs (centre,
- * replica offset, box faces) and the FP32 sums and differences carry at
- * most u (3|cm| + 4|o| + 2|b|) of error against the FP64 values; delta =
- * 6u (|cm| + |o| + |lesser| + |greater|) covers that and the FP64 path's own
- * rounding (the 1e-30 floor covers conversions that land on FP32
- * subnormals).  Squares and the three-term sum add 2u of the total,
- * bounded here by 4u. */
-__device__ int open_criterion_screened(const WalkArgs& a, const WalkNode& nd, int g, int local,
+/* open_criterion screened in FP32 (the margins above), in the form the box's
+ * centre m and half extents h give: the distance outside the box per axis is
+ * |c - m| - h where positive, the far side's |c - m| + h.  kUnsure: to be
+ * repeated in FP64. */
+constexpr int kUnsure = 2;
+template <bool HEX>
+__device__ __forceinline__ int open_criterion_screened(const WalkArgs& a, const WalkNode& nd, int g, int local,
                                        bool local_bucket, int off) {
-  if (nd.link.w <= 6) return 1;
-  const float4 nf = nd.geo;
-  const float4 lo = a.boxf[2 * (size_t)local], hi = a.boxf[2 * (size_t)local + 1];
-  const float cm[3] = {nf.x, nf.y, nf.z};
-  const float o[3] = {(float)((off & 7) - 3) * a.period32,
-                      (float)(((off >> 3) & 7) - 3) * a.period32,
-                      (float)(((off >> 6) & 7) - 3) * a.period32};
-  const float bl[3] = {lo.x, lo.y, lo.z}, bh[3] = {hi.x, hi.y, hi.z};
-  float c[3], dl[3];
-  float d2 = 0.0f, e = 0.0f;
-#pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    c[k] = cm[k] + o[k];
-    dl[k] = 6.0f * kU * (fabsf(cm[k]) + fabsf(o[k]) + fabsf(bl[k]) + fabsf(bh[k])) + 1e-30f;
-    const float gk = fmaxf(0.0f, fmaxf(bl[k] - c[k], c[k] - bh[k]));
-    d2 += gk * gk;
-    e += 2.0f * gk * dl[k] + 3.0f * dl[k] * dl[k];
+  const float4 m = a.boxes[local].mid, h = a.boxes[local].half;
+  const unsigned mxy = __float_as_uint(m.w), mze = __float_as_uint(h.w);
+  float dx = nd.geo.x - m.x, dy = nd.geo.y - m.y, dz = nd.geo.z - m.z, e = bf_lo(mze);
+  if (off != kHere) {
+    dx += (float)((off & 7) - 3) * a.period32;
+    dy += (float)(((off >> 3) & 7) - 3) * a.period32;
+    dz += (float)(((off >> 6) & 7) - 3) * a.period32;
+    e += a.e_rep;
   }
-  e += 4.0f * kU * d2;
-  const int inter = screen_le(d2, e, nf.w);
-  if (inter < 0) return open_criterion(a, g, local, local_bucket, off);
+  dx = fabsf(dx + (bf_lo(nd.low_xy) - bf_lo(mxy)));
+  dy = fabsf(dy + (bf_hi(nd.low_xy) - bf_hi(mxy)));
+  dz = fabsf(dz + (bf_hi(nd.low_z) - bf_hi(mze)));
+  const float gx = fmaxf(0.0f, dx - h.x), gy = fmaxf(0.0f, dy - h.y), gz = fmaxf(0.0f, dz - h.z);
+  const float d2 = fmaf(gx, gx, fmaf(gy, gy, gz * gz));
+  const int inter = screen_le(d2, e, nd.geo.w);
+  if (inter < 0) return kUnsure;
   if (inter == 1) {
     if (local_bucket) return 1;
-    float f2 = 0.0f, ef = 0.0f;
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      const float mk = fmaxf(fabsf(c[k] - bl[k]), fabsf(bh[k] - c[k]));
-      f2 += mk * mk;
-      ef += 2.0f * mk * dl[k] + 3.0f * dl[k] * dl[k];
-    }
-    ef += 4.0f * kU * f2;
-    const int far = screen_le(f2, ef, nf.w);
-    if (far < 0) return open_criterion(a, g, local, local_bucket, off);
+    const float fx = dx + h.x, fy = dy + h.y, fz = dz + h.z;
+    const int far = screen_le(fmaf(fx, fx, fmaf(fy, fy, fz * fz)), e, nd.geo.w);
+    if (far < 0) return kUnsure;
     return far ? 1 : -1;
   }
   /* outside the opening sphere: accepted, unless the hexadecapole rules
    * open it: a softening sphere that meets the local node, and then the
    * monopole radius (both screened in FP32, FP64 when too close to call) */
-  if (a.order != 4) return 0;
+  if (!HEX) return 0;
+  const float cm[3] = {nd.geo.x, nd.geo.y, nd.geo.z};
+  const float o[3] = {(float)((off & 7) - 3) * a.period32,
+                      (float)(((off >> 3) & 7) - 3) * a.period32,
+                      (float)(((off >> 6) & 7) - 3) * a.period32};
+  const float c[3] = {cm[0] + o[0], cm[1] + o[1], cm[2] + o[2]};
   const int sof = open_softening_screened(a, a.hexf[g].x, c, cm, o, local);
-  if (sof < 0) return open_criterion(a, g, local, local_bucket, off);
+  if (sof < 0) return kUnsure;
   if (sof == 0) return 0;
   const int mono = screen_le(d2, e, a.hexf[g].y);
-  if (mono < 0) return open_criterion(a, g, local, local_bucket, off);
+  if (mono < 0) return kUnsure;
   return mono;
 }
 
@@ -350,286 +415,314 @@ __device__ __forceinline__ int warp_excl_scan(int v, int& total) {
   return x - v;
 }
 
-/* Append pass: before a step adds `total` entries to list k (cnt so far),
- * the bucket's chunks are extended to hold them (lane 0, one atomic; the
- * warp's table maps list ranks to chunks; -1 once the pool is short). */
-__device__ __forceinline__ void ensure_chunks(const WalkArgs& a, int k, int b, int* tab, int& nalloc,
-                                              long long cnt, int total) {
-  const int need = (int)((cnt + total + kChunk - 1) / kChunk);
-  if (need > nalloc) {  // uniform over the warp
-    if ((threadIdx.x & 31) == 0) {
-      const int m = need - nalloc;
-      long long c0 = -1;
-      if (need <= kMaxChunks) {
-        c0 = atomicAdd(a.pool_next + k, (unsigned)m);
-        if (c0 + m > a.pool_chunks[k]) c0 = -1;
-      }
-      if (c0 < 0) atomicExch(a.overflow, 1);
-      for (int i = 0; i < m && nalloc + i < kMaxChunks; ++i) {
-        tab[nalloc + i] = c0 < 0 ? -1 : (int)(c0 + i);
-        if (c0 >= 0) {
-          a.chunk_bucket[k][c0 + i] = b;
-          a.chunk_rank[k][c0 + i] = nalloc + i;
-        }
-      }
-    }
-    nalloc = need;
-    __syncwarp();
+/* Append pass: m more chunks of list k for bucket b, the first of rank
+ * `rank`.  Returns the first one's number, the others following it, or -1 when
+ * the pool is short.  Called by the whole warp. */
+__device__ __noinline__ int take_chunks(const WalkArgs& a, int k, int b, int rank, int m) {
+  const int lane = threadIdx.x & 31;
+  unsigned c = 0;
+  if (lane == 0) c = atomicAdd(a.pool_next + k, (unsigned)m);
+  c = __shfl_sync(0xffffffffu, c, 0);
+  if ((long long)c + m > a.pool_chunks[k]) {
+    if (lane == 0) atomicExch(a.overflow, 1);
+    return -1;
   }
+  for (int i = lane; i < m; i += 32) {
+    a.chunk_bucket[k][c + i] = b;
+    a.chunk_rank[k][c + i] = rank + i;
+  }
+  return (int)c;
 }
 
-/* Entry q of list k of this bucket into its chunk. */
-__device__ __forceinline__ void append_at(const WalkArgs& a, int k, const int* tab, long long q,
-                                          int2 e) {
-  const long long r = q / kChunk;
-  const int c = r < kMaxChunks ? tab[r] : -1;
-  if (c >= 0) a.pool[k][(size_t)c * kChunk + (q - r * kChunk)] = e;
+/* Local nodes of a walk: chain[0] the unit's node, upward to `top` (the root
+ * when top is negative).  Returns top's level, or -1 when the chain is longer
+ * than 64 or does not meet top.  Lane 0 climbs; the result is the warp's. */
+__device__ __forceinline__ int climb_chain(const int* __restrict__ parent, long long n_nodes, int bn,
+                                           int top, int* chain) {
+  int n = -1;
+  if ((threadIdx.x & 31) == 0) {
+    int x = bn;
+    for (int k = 0; k < 64 && x >= 0 && x < n_nodes; ++k) {
+      chain[k] = x;
+      if (x == top) {
+        n = k;
+        break;
+      }
+      x = parent[x];
+    }
+  }
+  n = __shfl_sync(0xffffffffu, n, 0);
+  __syncwarp();
+  return n;
 }
 
 /* PHASE 0: the whole walk of each bucket; 1: the shared walk of each group
  * down to its group node (prefix lists and frontier); 2: each bucket from
- * its group's frontier, after its group's prefix lists. */
-template <int MODE, int STACK, int PHASE>
-__global__ void __launch_bounds__(kWalkWarps * 32) walk_kernel(const WalkArgs a) {
+ * its group's frontier, after its group's prefix lists.
+ *
+ * Bound by instruction issue and by L1 wavefronts alike (66 % and 60 % of
+ * their peaks for the buckets of 2^20 clustered particles), so the step is
+ * short: a test of some 40 instructions on a 32-byte record per source node
+ * and one per local node, pushes and list positions from ballots (no scans),
+ * particles expanded only in steps that open a source bucket.  Shared memory
+ * is kept to the stack: each KB taken from L1 costs hits on the node records
+ * (with a table of chunks beside the stack and 96-byte records the L1 hit rate
+ * was 38 %, and the pass took as long as one of 35 % more instructions).
+ * 1000003 NFW particles in buckets of 16, the bucket pass: 1982 us with FP32
+ * boxes, per-axis margins and scans, 1447 us so; 2^23 in buckets of 32: the
+ * whole walk 14.1 ms, 11.1 ms so. */
+template <int MODE, int PHASE, bool HEX>
+__global__ void __launch_bounds__(kWalkWarps * 32, 8)
+    walk_kernel(const __grid_constant__ WalkArgs a, const int stack) {
   constexpr bool FILL = MODE == kFill;
-  __shared__ int2 stk[kWalkWarps][STACK];
-  __shared__ int chain[kWalkWarps][64];
-  __shared__ int ctab[MODE == kAppend ? kWalkWarps : 1][3][MODE == kAppend ? kMaxChunks : 1];
+  constexpr bool POOL = MODE == kAppend && PHASE != 1;   // entries to chunk pools
+  constexpr bool SLOT = MODE == kAppend && PHASE == 1;   // entries to the group's slots
+  extern __shared__ int2 stk[];  // kWalkWarps x stack
+  __shared__ int chain_[kWalkWarps][64];
+  __shared__ int2 runs_[MODE != kCount ? kWalkWarps : 1][MODE != kCount ? 32 : 1];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const unsigned full = 0xffffffffu;
+  const unsigned full = 0xffffffffu, below = (1u << lane) - 1u;
   const long long bl = ((long long)blockIdx.x * kWalkWarps + warp) * a.bucket_stride;
   if (bl >= (PHASE == 1 ? (long long)a.n_groups : (long long)a.n_buckets)) return;  // whole warp
   const int b = (int)bl;  // the unit: a bucket, or a group in phase 1
   const int bn = PHASE == 1 ? a.group_node[b] : a.bucket_node[b];
   if (bn < 0 || bn >= a.n_nodes) return;
   const int gid = PHASE == 2 ? a.bucket_group[b] : 0;
-  const int gnode = PHASE == 2 ? a.group_node[gid] : -1;
-  /* local nodes from the root down to this unit (and, phase 2, the level
-   * of the bucket's group node on that chain) */
-  int depth = 0, gdepth = -1;
-  if (lane == 0) {
-    int n = 0;
-    for (int x = bn; x >= 0 && x < a.n_nodes && n < 65; x = a.parent[x]) ++n;
-    if (n > 64) {
-      depth = -1;
-    } else {
-      int k = n - 1;
-      for (int x = bn; k >= 0; x = a.parent[x]) {
-        if (x == gnode) gdepth = k;
-        chain[warp][k--] = x;
-      }
-      depth = chain[warp][0] == 0 ? n - 1 : -1;
-    }
-  }
-  depth = __shfl_sync(full, depth, 0);
-  gdepth = __shfl_sync(full, gdepth, 0);
-  if (depth < 0 || (PHASE == 2 && gdepth < 0)) {
+  int* chain = chain_[warp];
+  const int top = climb_chain(a.parent, a.n_nodes, bn, PHASE == 2 ? a.group_node[gid] : 0, chain);
+  if (top < 0) {
     if (lane == 0) atomicExch(a.error, 1);
     return;
   }
   /* a group node with children is not a bucket: entries undecided at its
    * level go to the frontier instead of being opened */
   const bool unit_bucket = PHASE != 1 || (a.info[4 * (size_t)bn] < 0 && a.info[4 * (size_t)bn + 1] < 0);
-  long long oc = 0, op = 0, os = 0, of = 0;
+  /* where list k's entries go: the fill pass's offsets or the group's slots */
+  int2* base[3] = {nullptr, nullptr, nullptr};
+  int2* fbase = nullptr;
   if (FILL) {
-    oc = a.off_cells[b];
-    op = a.off_parts[b];
-    os = a.off_soft ? a.off_soft[b] : 0;
-    if (PHASE == 1) of = a.off_front[b];
+    base[0] = a.cells + a.off_cells[b];
+    base[1] = a.parts + a.off_parts[b];
+    if (PHASE != 1 && a.off_soft) base[2] = a.soft + a.off_soft[b];
+    if (PHASE == 1) fbase = a.front + a.off_front[b];
   }
+  if (SLOT) {
+    base[0] = a.cells + (size_t)b * a.slot[0];
+    base[1] = a.parts + (size_t)b * a.slot[1];
+    fbase = a.front + (size_t)b * a.slot[2];
+  }
+  int n[3] = {0, 0, 0}, nf = 0;     // entries so far
+  /* append pass, per list: entries that the chunks taken hold, and where entry
+   * q goes in the last chunk taken before this step (less that chunk's first
+   * entry) and in those taken in it; a negative pool position drops entries */
+  int room[3] = {0, 0, 0}, last[3] = {-1, -1, -1};
+  int split = 0, fresh = -1;
+  auto reserve = [&](int k, int total) {
+    if (POOL) {
+      split = room[k];
+      if (n[k] + total > room[k]) {  // uniform over the warp
+        const int m = (n[k] + total - room[k] + kChunk - 1) / kChunk;
+        fresh = take_chunks(a, k, b, room[k] / kChunk, m);
+        room[k] += m * kChunk;
+      }
+    }
+  };
+  auto put = [&](int k, int q, int2 e) {
+    if (FILL) base[k][q] = e;
+    if (SLOT && q < a.slot[k]) base[k][q] = e;
+    if (POOL) {
+      const int c = q < split ? last[k] : fresh < 0 ? -1 : fresh + (q - split) / kChunk;
+      if (c >= 0) a.pool[k][(size_t)c * kChunk + q % kChunk] = e;
+    }
+  };
+  auto done = [&](int k) {  // the step's entries are put
+    if (POOL && room[k] > split) last[k] = fresh < 0 ? -1 : fresh + (room[k] - split) / kChunk - 1;
+  };
+  int2* st = stk + warp * stack;
   int sp = 0;
-  long long fpos = 0, fend = 0;  // phase 2: the group's frontier, fed when the stack is empty
+  const int2* front = nullptr;  // phase 2: the group's frontier, fed when the stack is empty
+  int fpos = 0, fend = 0;
   if (PHASE == 2) {
-    fpos = a.off_front[gid];
-    fend = a.off_front[gid + 1];
+    front = a.glist[2] + (a.goff[2] ? a.goff[2][gid] : (long long)gid * a.slot[2]);
+    fend = a.gcnt[2][gid];
+    /* the group's prefix lists (entries accepted against the local nodes
+     * the group walk covered, the same for every bucket of the group) */
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const int2* pre = a.glist[k] + (a.goff[k] ? a.goff[k][gid] : (long long)gid * a.slot[k]);
+      const int cnt = a.gcnt[k][gid];
+      if (k == 0 && HEX) {
+        /* hexadecapole: the group's accepted cells split here into cells and
+         * softened cells, by openSoftening against this bucket, as the
+         * one-phase walk splits them when it accepts them */
+        for (int j0 = 0; j0 < cnt; j0 += 32) {
+          const int tot = cnt - j0 < 32 ? cnt - j0 : 32;
+          int2 e = make_int2(-1, 0);
+          bool soft = false;
+          if (lane < tot) {
+            e = pre[j0 + lane];
+            if (e.x >= 0 && e.x < a.n_nodes)
+              soft = open_softening_fast(a, e.x, (e.y >> 22) & 0x1ff, bn);
+          }
+          const unsigned mc = __ballot_sync(full, lane < tot && !soft);
+          const unsigned ms = __ballot_sync(full, lane < tot && soft);
+          reserve(0, __popc(mc));
+          if (MODE != kCount && lane < tot && !soft) put(0, n[0] + __popc(mc & below), e);
+          done(0);
+          n[0] += __popc(mc);
+          reserve(2, __popc(ms));
+          if (MODE != kCount && lane < tot && soft) put(2, n[2] + __popc(ms & below), e);
+          done(2);
+          n[2] += __popc(ms);
+        }
+        continue;
+      }
+      if (MODE != kCount) {
+        reserve(k, cnt);
+        for (int j = lane; j < cnt; j += 32) put(k, j, pre[j]);
+        done(k);
+      }
+      n[k] = cnt;
+    }
   } else {
     /* the root of every replica on the check list */
     const int nr = a.n_replicas, side = 2 * nr + 1, nrep = side * side * side;
-    if (nrep > STACK) {  // uniform; the host re-runs the launch with the larger stack
+    if (nrep > stack) {  // uniform; the host re-runs the walk with the larger stack
       if (lane == 0) atomicExch(a.error, 2);
       return;
     }
     for (int r = lane; r < nrep; r += 32) {
       const int x = r / (side * side) - nr, y = (r / side) % side - nr, z = r % side - nr;
-      stk[warp][r] = make_int2(0, (x + 3) | ((y + 3) << 3) | ((z + 3) << 6));
+      st[r] = make_int2(0, (top << 16) | (x + 3) | ((y + 3) << 3) | ((z + 3) << 6));
     }
     sp = nrep;
   }
-  long long nc = 0, np = 0, ns = 0, nf = 0;
-  int na[3] = {0, 0, 0};  // append pass: chunks taken per list
-  if (PHASE == 2) {
-    /* the group's prefix lists (entries accepted against the local nodes
-     * the group walk covered, the same for every bucket of the group) */
-    if (a.order == 4) {
-      /* hexadecapole: the group's accepted cells split here into cells and
-       * softened cells, by openSoftening against this bucket, as the
-       * one-phase walk splits them when it accepts them */
-      const unsigned below = (1u << lane) - 1u;
-      const long long p0 = a.pre_off[0][gid], cnt = a.pre_off[0][gid + 1] - p0;
-      for (long long j0 = 0; j0 < cnt; j0 += 32) {
-        const int tot = (int)(cnt - j0 < 32 ? cnt - j0 : 32);
-        int2 e = make_int2(-1, 0);
-        bool soft = false;
-        if (lane < tot) {
-          e = a.pre[0][p0 + j0 + lane];
-          if (e.x >= 0 && e.x < a.n_nodes) soft = open_softening_fast(a, e.x, (e.y >> 22) & 0x1ff, bn);
-        }
-        const unsigned mc = __ballot_sync(full, lane < tot && !soft);
-        const unsigned ms = __ballot_sync(full, lane < tot && soft);
-        if (MODE == kAppend) {
-          if (mc) ensure_chunks(a, 0, b, ctab[warp][0], na[0], nc, __popc(mc));
-          if (ms) ensure_chunks(a, 2, b, ctab[warp][2], na[2], ns, __popc(ms));
-        }
-        if (MODE != kCount && lane < tot) {
-          if (!soft) {
-            const long long q = nc + __popc(mc & below);
-            if (FILL) a.cells[oc + q] = e;
-            if (MODE == kAppend) append_at(a, 0, ctab[warp][0], q, e);
-          } else {
-            const long long q = ns + __popc(ms & below);
-            if (FILL) a.soft[os + q] = e;
-            if (MODE == kAppend) append_at(a, 2, ctab[warp][2], q, e);
-          }
-        }
-        nc += __popc(mc);
-        ns += __popc(ms);
-      }
-    }
-#pragma unroll
-    for (int k = 0; k < 2; ++k) {
-      if (k == 0 && a.order == 4) continue;  // split above
-      const long long p0 = a.pre_off[k][gid], cnt = a.pre_off[k][gid + 1] - p0;
-      long long& n_k = k == 0 ? nc : np;
-      if (MODE != kCount) {
-        for (long long j0 = 0; j0 < cnt; j0 += 32) {
-          const int tot = (int)(cnt - j0 < 32 ? cnt - j0 : 32);
-          if (MODE == kAppend) ensure_chunks(a, k, b, ctab[warp][k], na[k], n_k + j0, tot);
-          if (lane < tot) {
-            const int2 e = a.pre[k][p0 + j0 + lane];
-            if (FILL) (k == 0 ? a.cells[oc + n_k + j0 + lane] : a.parts[op + n_k + j0 + lane]) = e;
-            if (MODE == kAppend) append_at(a, k, ctab[warp][k], n_k + j0 + lane, e);
-          }
-        }
-      }
-      n_k += cnt;
-    }
-  }
   __syncwarp();
   while (sp > 0 || fpos < fend) {
-    int n;
     int2 e = make_int2(-1, 0);
     if (sp > 0) {
-      n = sp < 32 ? sp : 32;
-      const int top = sp - n;
-      if (lane < n) e = stk[warp][top + lane];
-      sp = top;
+      const int m = sp < 32 ? sp : 32;
+      sp -= m;
+      if (lane < m) e = st[sp + lane];
     } else {  // phase 2: the next frontier entries, tested one level below the group node
-      n = (int)(fend - fpos < 32 ? fend - fpos : 32);
-      if (lane < n) {
-        const int2 f = a.front[fpos + lane];
-        e = make_int2(f.x, ((gdepth + 1) << 16) | (f.y & 0xffff));
+      if (fpos + lane < fend) {
+        e = front[fpos + lane];
+        e.y = ((top - 1) << 16) | (e.y & 0xffff);
       }
-      fpos += n;
+      fpos += 32;
     }
     __syncwarp();  // popped before anything is pushed over them
     /* kind: 0 cell, 1 softened cell, 2 particles, 3 open, 4 defer, 5 frontier
      * (phase 1: undecided at the group node), -1 none */
-    int kind = -1, c0 = -1, c1 = -1, pfirst = 0, pcount = 0;
+    int kind = -1, na = -1, nb = -1;
     const int g = e.x, level = e.y >> 16, code = e.y & 0xffff;
-    if (g >= 0 && g < a.n_nodes && level <= depth) {  // memory safety
-      const int local = chain[warp][level];
-      const bool local_bucket = level == depth && unit_bucket;
+    if (g >= 0 && g < a.n_nodes && level >= 0 && level <= top) {  // memory safety
       const WalkNode nd = a.nodes[g];
-      const int open = open_criterion_screened(a, nd, g, local, local_bucket, code);
+      na = nd.a;
+      nb = nd.b;
+      const bool local_bucket = level == 0 && unit_bucket;
+      int open = open_criterion_screened<HEX>(a, nd, g, chain[level], local_bucket, code);
+      if (open == kUnsure) open = open_criterion(a, g, chain[level], local_bucket, code);
       if (open == 0) {
-        bool softened = false;
-        if (a.order == 4 && PHASE != 1)  // phase 2 splits the group's cells per bucket
-          softened = open_softening_fast(a, g, code, bn);
-        kind = softened ? 1 : 0;
-      } else if (nd.link.x < 0 && nd.link.y < 0) {  // a source bucket: its particles
+        kind = 0;
+        if (PHASE != 1 && HEX)  // phase 2 splits the group's cells per bucket
+          kind = open_softening_fast(a, g, code, bn) ? 1 : 0;
+      } else if (na < 0) {  // a source bucket: its particles
         kind = 2;
-        pfirst = nd.link.z;
-        pcount = nd.link.w;
       } else if (open == 1 || local_bucket) {
         kind = 3;
-        c0 = nd.link.x;
-        c1 = nd.link.y;
       } else {
-        kind = level == depth ? 5 : 4;  // 5 only in phase 1 (level == depth is a bucket otherwise)
+        kind = PHASE == 1 && level == 0 ? 5 : 4;  // at level 0 phases 0 and 2 decide
       }
     }
     /* pushes, in lane order; within a lane child 1 below child 0 */
-    const int npush = kind == 3 ? (c0 >= 0) + (c1 >= 0) : (kind == 4 ? 1 : 0);
-    int tpush;
-    int pos = sp + warp_excl_scan(npush, tpush);
-    if (sp + tpush > STACK) {  // uniform: every lane sees tpush
+    const bool two = kind == 3 && nb >= 0;
+    const bool push = kind == 3 || kind == 4;
+    const unsigned mq = __ballot_sync(full, push), m2 = __ballot_sync(full, two);
+    const int tpush = __popc(mq) + __popc(m2);
+    if (sp + tpush > stack) {  // uniform
       if (lane == 0) atomicExch(a.error, 2);
       break;
     }
-    if (kind == 3) {
-      if (c1 >= 0) stk[warp][pos++] = make_int2(c1, (level << 16) | code);
-      if (c0 >= 0) stk[warp][pos++] = make_int2(c0, (level << 16) | code);
-    } else if (kind == 4) {
-      stk[warp][pos] = make_int2(g, ((level + 1) << 16) | code);
+    if (push) {
+      const int pos = sp + __popc(mq & below) + __popc(m2 & below);
+      if (kind == 4) {
+        st[pos] = make_int2(g, ((level - 1) << 16) | code);
+      } else {
+        st[pos] = make_int2(two ? nb : na, (level << 16) | code);
+        if (two) st[pos + 1] = make_int2(na, (level << 16) | code);
+      }
     }
     sp += tpush;
     /* accepted cells, softened cells and particles, contiguous per step */
-    const unsigned below = (1u << lane) - 1u;
-    const unsigned mc = __ballot_sync(full, kind == 0), ms = __ballot_sync(full, kind == 1);
-    int tpart;
-    const int ppos = warp_excl_scan(kind == 2 ? pcount : 0, tpart);
-    if (MODE == kAppend) {
-      if (mc) ensure_chunks(a, 0, b, ctab[warp][0], na[0], nc, __popc(mc));
-      if (ms) ensure_chunks(a, 2, b, ctab[warp][2], na[2], ns, __popc(ms));
-      if (tpart) ensure_chunks(a, 1, b, ctab[warp][1], na[1], np, tpart);
+    const unsigned mc = __ballot_sync(full, kind == 0);
+    if (mc) {
+      reserve(0, __popc(mc));
+      if (MODE != kCount && kind == 0)
+        put(0, n[0] + __popc(mc & below), make_int2(g, code << 22));
+      done(0);
+      n[0] += __popc(mc);
     }
-    if (kind == 0) {
-      const long long q = nc + __popc(mc & below);
-      if (FILL) a.cells[oc + q] = make_int2(g, code << 22);
-      if (MODE == kAppend) append_at(a, 0, ctab[warp][0], q, make_int2(g, code << 22));
+    if (PHASE != 1 && HEX) {
+      const unsigned ms = __ballot_sync(full, kind == 1);
+      if (ms) {
+        reserve(2, __popc(ms));
+        if (MODE != kCount && kind == 1)
+          put(2, n[2] + __popc(ms & below), make_int2(g, code << 22));
+        done(2);
+        n[2] += __popc(ms);
+      }
     }
-    if (kind == 1) {
-      const long long q = ns + __popc(ms & below);
-      if (FILL) a.soft[os + q] = make_int2(g, code << 22);
-      if (MODE == kAppend) append_at(a, 2, ctab[warp][2], q, make_int2(g, code << 22));
-    }
-    if (MODE != kCount && tpart) {
-      /* the step's particle entries, 32 at a time: entry j belongs to the
-       * first lane whose run ends after j (a binary search over the lanes'
-       * inclusive ends), which lies ppos(owner) into that lane's run */
-      const int incl = ppos + (kind == 2 ? pcount : 0);
-      for (int j0 = 0; j0 < tpart; j0 += 32) {
-        const int j = j0 + lane;
-        int owner = 0;
-#pragma unroll
-        for (int bit = 16; bit > 0; bit >>= 1)
-          if (__shfl_sync(full, incl, owner + bit - 1) <= j) owner += bit;
-        const int o_pos = __shfl_sync(full, ppos, owner);
-        const int o_first = __shfl_sync(full, pfirst, owner);
-        const int o_code = __shfl_sync(full, code, owner);
-        if (j < tpart) {
-          const int2 e = make_int2(o_first + (j - o_pos), o_code << 22);
-          if (FILL) a.parts[op + np + j] = e;
-          if (MODE == kAppend) append_at(a, 1, ctab[warp][1], np + j, e);
+    const int pcount = kind == 2 && nb > 0 ? nb : 0;
+    const unsigned mp = __ballot_sync(full, pcount > 0);
+    if (mp) {
+      if (MODE == kCount) {
+        n[1] += __reduce_add_sync(full, pcount);
+      } else {
+        /* the step's particle entries, 32 at a time: the runs compacted in
+         * shared memory, entry j in the run of rank (runs starting at or
+         * before j) - 1 */
+        int tpart;
+        const int ppos = warp_excl_scan(pcount, tpart);
+        if (pcount > 0)
+          runs_[warp][__popc(mp & below)] = make_int2(~na - ppos, code << 22);
+        reserve(1, tpart);
+        __syncwarp();
+        int rank0 = -1;  // runs starting before this window, less one
+        for (int j0 = 0; j0 < tpart; j0 += 32) {
+          const unsigned at = (unsigned)(ppos - j0);
+          const unsigned mw = __reduce_or_sync(full, pcount > 0 && at < 32u ? 1u << at : 0u);
+          const int j = j0 + lane;
+          if (j < tpart) {
+            const int2 r = runs_[warp][rank0 + __popc(mw & (below | (1u << lane)))];
+            put(1, n[1] + j, make_int2(r.x + j, r.y));
+          }
+          rank0 += __popc(mw);
         }
+        done(1);
+        n[1] += tpart;
       }
     }
     if (PHASE == 1) {
       const unsigned mf = __ballot_sync(full, kind == 5);
-      if (FILL && kind == 5) a.front[of + nf + __popc(mf & below)] = make_int2(g, code);
-      nf += __popc(mf);
+      if (mf) {
+        const int q = nf + __popc(mf & below);
+        if (kind == 5 && (FILL || (SLOT && q < a.slot[2]))) fbase[q] = make_int2(g, code);
+        nf += __popc(mf);
+      }
     }
-    nc += __popc(mc);
-    ns += __popc(ms);
-    np += tpart;
     __syncwarp();  // pushes visible to the next pops
   }
   if (!FILL && lane == 0) {
+    if (SLOT && (n[0] > a.slot[0] || n[1] > a.slot[1] || nf > a.slot[2])) {
+      atomicExch(a.slot_over, 1);  // walked again by count and fill; nothing reads past the slots
+      n[0] = n[1] = nf = 0;
+    }
     const int i = b / a.bucket_stride;
-    a.n_cells[i] = (int)nc;
-    a.n_parts[i] = (int)np;
-    if (a.n_soft) a.n_soft[i] = (int)ns;
-    if (PHASE == 1) a.n_front[i] = (int)nf;
+    a.n_cells[i] = n[0];
+    a.n_parts[i] = n[1];
+    if (PHASE != 1 && a.n_soft) a.n_soft[i] = n[2];
+    if (PHASE == 1) a.n_front[i] = nf;
   }
 }
 
@@ -669,7 +762,7 @@ struct FusedArgs {
  * a 168-register budget of 12 warps per SM was slower still). */
 template <int STACK, int WARPS>
 __global__ void __launch_bounds__(WARPS * 32, kFusedWarpsPerSM / WARPS)
-    walk_eval_kernel(const WalkArgs a, const FusedArgs f) {
+    walk_eval_kernel(const __grid_constant__ WalkArgs a, const FusedArgs f) {
   __shared__ int2 stk[WARPS][STACK];
   __shared__ int chain[WARPS][64];
   __shared__ int2 pcell[WARPS][64];  // accepted cells waiting for a block
@@ -695,27 +788,10 @@ __global__ void __launch_bounds__(WARPS * 32, kFusedWarpsPerSM / WARPS)
       if (lane == 0) atomicExch(a.error, 1);
       continue;
     }
-    const int gnode = a.group_node[gid];
-    int depth = 0, gdepth = -1;
-    if (lane == 0) {
-      int n = 0;
-      for (int x = bn; x >= 0 && x < a.n_nodes && n < 65; x = a.parent[x]) ++n;
-      if (n > 64) {
-        depth = -1;
-      } else {
-        int k = n - 1;
-        for (int x = bn; k >= 0; x = a.parent[x]) {
-          if (x == gnode) gdepth = k;
-          chain[warp][k--] = x;
-        }
-        depth = chain[warp][0] == 0 ? n - 1 : -1;
-      }
-    }
-    depth = __shfl_sync(kFull, depth, 0);
-    gdepth = __shfl_sync(kFull, gdepth, 0);
+    const int top = climb_chain(a.parent, a.n_nodes, bn, a.group_node[gid], chain[warp]);
     const long long tbase = a.info[4 * (size_t)bn + 2];
     const int n = a.info[4 * (size_t)bn + 3];
-    if (depth < 0 || gdepth < 0) {
+    if (top < 0) {
       if (lane == 0) atomicExch(a.error, 1);
       continue;
     }
@@ -820,9 +896,10 @@ __global__ void __launch_bounds__(WARPS * 32, kFusedWarpsPerSM / WARPS)
         __syncwarp();  // the stage is rewritten by the next block
       };
 
-      long long pc_pos = a.pre_off[0][gid], pc_end = a.pre_off[0][gid + 1];
-      long long pp_pos = a.pre_off[1][gid], pp_end = a.pre_off[1][gid + 1];
-      long long fpos = a.off_front[gid], fend = a.off_front[gid + 1];
+      auto first = [&](int k) { return a.goff[k] ? a.goff[k][gid] : (long long)gid * a.slot[k]; };
+      long long pc_pos = first(0), pc_end = pc_pos + a.gcnt[0][gid];
+      long long pp_pos = first(1), pp_end = pp_pos + a.gcnt[1][gid];
+      long long fpos = first(2), fend = fpos + a.gcnt[2][gid];
       int sp_ = 0;       // walk stack entries
       int npc = 0;       // pending cells
       int nrun = 0;      // pending runs
@@ -837,13 +914,13 @@ __global__ void __launch_bounds__(WARPS * 32, kFusedWarpsPerSM / WARPS)
         if (pc_pos < pc_end) {
           const int ne = (int)min(32LL, pc_end - pc_pos);
           v = lane < ne;
-          if (v) ent = a.pre[0][pc_pos + lane];
+          if (v) ent = a.glist[0][pc_pos + lane];
           pc_pos += ne;
           which = 0;
         } else if (pp_pos < pp_end) {
           const int ne = (int)min(32LL, pp_end - pp_pos);
           v = lane < ne;
-          if (v) ent = a.pre[1][pp_pos + lane];
+          if (v) ent = a.glist[1][pp_pos + lane];
           pp_pos += ne;
           which = 1;
         } else if (npc >= 32 || (walked && npc > 0)) {
@@ -916,29 +993,30 @@ __global__ void __launch_bounds__(WARPS * 32, kFusedWarpsPerSM / WARPS)
         } else {
           nst = (int)(fend - fpos < 32 ? fend - fpos : 32);
           if (lane < nst) {
-            const int2 fr = a.front[fpos + lane];
-            e = make_int2(fr.x, ((gdepth + 1) << 16) | (fr.y & 0xffff));
+            const int2 fr = a.glist[2][fpos + lane];
+            e = make_int2(fr.x, ((top - 1) << 16) | (fr.y & 0xffff));
           }
           fpos += nst;
         }
         __syncwarp();
         int kind = -1, c0 = -1, c1 = -1, pfirst = 0, pcount = 0;
         const int src = e.x, level = e.y >> 16, code = e.y & 0xffff;
-        if (src >= 0 && src < a.n_nodes && level <= depth) {
+        if (src >= 0 && src < a.n_nodes && level >= 0 && level <= top) {
           const int local = chain[warp][level];
-          const bool local_bucket = level == depth;
+          const bool local_bucket = level == 0;
           const WalkNode nd = a.nodes[src];
-          const int open = open_criterion_screened(a, nd, src, local, local_bucket, code);
+          int open = open_criterion_screened<false>(a, nd, src, local, local_bucket, code);
+          if (open == kUnsure) open = open_criterion(a, src, local, local_bucket, code);
           if (open == 0) {
             kind = 0;
-          } else if (nd.link.x < 0 && nd.link.y < 0) {
+          } else if (nd.a < 0) {
             kind = 2;
-            pfirst = nd.link.z;
-            pcount = nd.link.w;
+            pfirst = ~nd.a;
+            pcount = nd.b;
           } else if (open == 1 || local_bucket) {
             kind = 3;
-            c0 = nd.link.x;
-            c1 = nd.link.y;
+            c0 = nd.a;
+            c1 = nd.b;
           } else {
             kind = 4;
           }
@@ -954,7 +1032,7 @@ __global__ void __launch_bounds__(WARPS * 32, kFusedWarpsPerSM / WARPS)
           if (c1 >= 0) stk[warp][pos++] = make_int2(c1, (level << 16) | code);
           if (c0 >= 0) stk[warp][pos++] = make_int2(c0, (level << 16) | code);
         } else if (kind == 4) {
-          stk[warp][pos] = make_int2(src, ((level + 1) << 16) | code);
+          stk[warp][pos] = make_int2(src, ((level - 1) << 16) | code);
         }
         sp_ += tpush;
         const unsigned mc = __ballot_sync(kFull, kind == 0);
@@ -1016,12 +1094,18 @@ __global__ void gather_chunks_kernel(const int2* __restrict__ pool, const int* _
   }
 }
 
-/* Exclusive scan of n int counts into off64[0..n] and off32[0..n]: per-tile
- * sums, a one-block scan of the tile sums, then per-tile scans. */
+/* Exclusive scans of gridDim.y rows of n int counts (row k at in + k n) into
+ * off64 + k (n + 1) and off32[k], n + 1 values each: per-tile sums, a
+ * one-block scan of each row's tile sums, then per-tile scans. */
 constexpr int kScanThreads = 1024, kScanPer = 4, kScanTile = kScanThreads * kScanPer;
+
+struct ScanOut {
+  int* off32[3];
+};
 
 __global__ void scan_tile_sums_kernel(const int* __restrict__ in, int n, long long* __restrict__ ts) {
   __shared__ long long part[kScanThreads / 32];
+  in += (size_t)blockIdx.y * n;
   const long long base = (long long)blockIdx.x * kScanTile + threadIdx.x * kScanPer;
   long long v = 0;
   for (int k = 0; k < kScanPer; ++k)
@@ -1032,7 +1116,7 @@ __global__ void scan_tile_sums_kernel(const int* __restrict__ in, int n, long lo
   if (threadIdx.x < 32) {
     long long w = part[threadIdx.x];
     for (int o = 16; o > 0; o >>= 1) w += __shfl_xor_sync(0xffffffffu, w, o);
-    if (threadIdx.x == 0) ts[blockIdx.x] = w;
+    if (threadIdx.x == 0) ts[(size_t)blockIdx.y * gridDim.x + blockIdx.x] = w;
   }
 }
 
@@ -1062,6 +1146,7 @@ __device__ long long block_exclusive_scan(long long v, long long* sh, long long&
 
 __global__ void scan_tiles_kernel(long long* __restrict__ ts, int nt) {
   __shared__ long long sh[32];
+  ts += (size_t)blockIdx.y * nt;
   long long carry = 0;
   for (int b0 = 0; b0 < nt; b0 += kScanThreads) {
     const int i = b0 + threadIdx.x;
@@ -1074,8 +1159,11 @@ __global__ void scan_tiles_kernel(long long* __restrict__ ts, int nt) {
 }
 
 __global__ void scan_apply_kernel(const int* __restrict__ in, int n, const long long* __restrict__ ts,
-                                  long long* __restrict__ off64, int* __restrict__ off32) {
+                                  long long* __restrict__ off64, const ScanOut out) {
   __shared__ long long sh[32];
+  in += (size_t)blockIdx.y * n;
+  off64 += (size_t)blockIdx.y * (n + 1);
+  int* off32 = out.off32[blockIdx.y];
   const long long base = (long long)blockIdx.x * kScanTile + threadIdx.x * kScanPer;
   int v[kScanPer];
   long long sum = 0;
@@ -1084,18 +1172,29 @@ __global__ void scan_apply_kernel(const int* __restrict__ in, int n, const long 
     sum += v[k];
   }
   long long tot;
-  long long run = ts[blockIdx.x] + block_exclusive_scan(sum, sh, tot);
+  long long run = ts[(size_t)blockIdx.y * gridDim.x + blockIdx.x] + block_exclusive_scan(sum, sh, tot);
   for (int k = 0; k < kScanPer; ++k) {
     if (base + k < n) {
       off64[base + k] = run;
-      off32[base + k] = (int)run;
+      if (off32) off32[base + k] = (int)run;
     }
     run += v[k];
     if (base + k == n - 1) {
       off64[n] = run;
-      off32[n] = (int)run;
+      if (off32) off32[n] = (int)run;
     }
   }
+}
+
+/* Tiles of one row, and the scans of `rows` rows (ts: rows x tiles). */
+inline int scan_tiles(int n) { return (n + kScanTile - 1) / kScanTile; }
+inline void launch_scans(const int* in, int n, int rows, long long* ts, long long* off64,
+                         const ScanOut& out, cudaStream_t s) {
+  const dim3 grid((unsigned)scan_tiles(n), (unsigned)rows);
+  scan_tile_sums_kernel<<<grid, kScanThreads, 0, s>>>(in, n, ts);
+  scan_tiles_kernel<<<dim3(1, (unsigned)rows), kScanThreads, 0, s>>>(ts, (int)grid.x);
+  scan_apply_kernel<<<grid, kScanThreads, 0, s>>>(in, n, ts, off64, out);
+  count_launch(3);
 }
 
 /* ---- groups for the two-phase walk ---- */
@@ -1111,20 +1210,22 @@ __global__ void bucket_first_kernel(const int* __restrict__ bucket_node, const i
   }
 }
 
-/* Buckets whose first particle lies in [lo, hi): the buckets of the node
- * covering those particles. */
-__device__ __forceinline__ int buckets_in(const int* bfirst, int nb, int lo, int hi) {
-  int a0 = 0, a1 = nb;  // first index with bfirst >= lo
+/* Whether the node that covers particles [lo, hi), bucket b's among them,
+ * holds more than gmax buckets.  Its buckets are those whose first particle
+ * lies in [lo, hi); only gmax of them to either side of b need be looked at. */
+__device__ __forceinline__ bool more_buckets(const int* bfirst, int nb, int b, int gmax, int lo,
+                                             int hi) {
+  int a0 = b - gmax > 0 ? b - gmax : 0, a1 = b;  // first index with bfirst >= lo, if that far
   while (a0 < a1) {
     const int m = (a0 + a1) >> 1;
     if (bfirst[m] < lo) a0 = m + 1; else a1 = m;
   }
-  int b0 = a0, b1 = nb;  // first index with bfirst >= hi
+  int b0 = b, b1 = (long long)b + gmax + 1 < nb ? b + gmax + 1 : nb;  // first with bfirst >= hi
   while (b0 < b1) {
     const int m = (b0 + b1) >> 1;
     if (bfirst[m] < hi) b0 = m + 1; else b1 = m;
   }
-  return b0 - a0;
+  return b0 - a0 > gmax;
 }
 
 /* Each bucket's group node: its highest ancestor whose subtree holds at
@@ -1140,7 +1241,7 @@ __global__ void bucket_group_node_kernel(const int* __restrict__ bucket_node,
       const int q = parent[x];
       if (q < 0 || q >= n_nodes) break;
       const int lo = info[4 * (size_t)q + 2], cnt = info[4 * (size_t)q + 3];
-      if (buckets_in(bfirst, nb, lo, lo + cnt) > gmax) break;
+      if (more_buckets(bfirst, nb, (int)b, gmax, lo, lo + cnt)) break;
       x = q;
     }
     gn[b] = x;
@@ -1179,23 +1280,27 @@ static bool walk_args_ok(const ChangaTreeView* t, const ChangaWalkParams* p) {
 }
 
 /* Node records and boxes for the screened tests (stream-ordered scratch,
- * freed by the caller). */
+ * freed by the caller).  The block starts with the error word and, at the
+ * next int, the word that a group which outgrew its slots sets. */
 static int walk_setup(const ChangaTreeView* t, const ChangaWalkParams* p, WalkArgs& a, char** block,
                       cudaStream_t s) {
   prepare_pool();
   const size_t nn = (size_t)t->n_nodes;
+  const bool hex = p->order == 4;
   CHG_CUDA(cudaMallocAsync((void**)block,
-                           256 + nn * (sizeof(WalkNode) + 2 * sizeof(float4) + sizeof(float2)), s));
+                           256 + nn * (sizeof(WalkNode) + sizeof(WalkBox) +
+                                       (hex ? 2 * sizeof(float4) + sizeof(float2) : 0)), s));
   int* err = (int*)*block;
   WalkNode* nodes = (WalkNode*)(*block + 256);
-  float4* boxf = (float4*)(nodes + nn);
-  float2* hexf = (float2*)(boxf + 2 * nn);
-  CHG_CUDA(cudaMemsetAsync(err, 0, sizeof(int), s));
+  WalkBox* boxes = (WalkBox*)(nodes + nn);
+  float4* boxf = hex ? (float4*)(boxes + nn) : nullptr;
+  float2* hexf = hex ? (float2*)(boxf + 2 * nn) : nullptr;
+  CHG_CUDA(cudaMemsetAsync(err, 0, 256, s));
   long long g = (t->n_nodes + 255) / 256;
   const long long cap = (long long)sm_count() * 8;
   walk_prep_kernel<<<(int)(g < cap ? g : cap), 256, 0, s>>>(
       t->geom, t->bbox, t->info, t->n_nodes, p->theta,
-      p->theta * p->theta * p->theta * p->theta, nodes, boxf, hexf);
+      p->theta * p->theta * p->theta * p->theta, nodes, boxes, boxf, hexf);
   count_launch();
   a = WalkArgs{};
   a.geom = t->geom;
@@ -1211,10 +1316,15 @@ static int walk_setup(const ChangaTreeView* t, const ChangaWalkParams* p, WalkAr
   a.order = p->order;
   a.n_replicas = p->n_replicas;
   a.error = err;
+  a.slot_over = err + 1;
   a.nodes = nodes;
+  a.boxes = boxes;
   a.boxf = boxf;
   a.hexf = hexf;
   a.period32 = (float)p->period;
+  /* the margin of an offset of n_replicas periods: twice 3 (2^13 + 2) (4 u o)^2 */
+  const double eo = 4.0 * kU * p->n_replicas * p->period;
+  a.e_rep = (float)(1.001 * kScreenE * eo * eo);
   a.bucket_stride = 1;
   return 0;
 }
@@ -1224,45 +1334,49 @@ static int walk_setup(const ChangaTreeView* t, const ChangaWalkParams* p, WalkAr
 static std::atomic<int> g_test_small_stack{0};
 static std::atomic<long long> g_stack_reruns{0};  // launches re-run with the large stack
 
-template <int STACK, int PHASE>
-static void walk_launch_phase(const WalkArgs& a, int mode, int grid, cudaStream_t s) {
-  if (mode == kFill) walk_kernel<kFill, STACK, PHASE><<<grid, kWalkWarps * 32, 0, s>>>(a);
-  else if (mode == kAppend && PHASE != 1)
-    walk_kernel<(PHASE != 1 ? kAppend : kCount), STACK, PHASE><<<grid, kWalkWarps * 32, 0, s>>>(a);
-  else walk_kernel<kCount, STACK, PHASE><<<grid, kWalkWarps * 32, 0, s>>>(a);
+template <int PHASE, bool HEX>
+static void walk_launch(const WalkArgs& a, int mode, int stack, int grid, cudaStream_t s) {
+  const int threads = kWalkWarps * 32;
+  const size_t smem = (size_t)kWalkWarps * stack * sizeof(int2);
+  if (mode == kFill) walk_kernel<kFill, PHASE, HEX><<<grid, threads, smem, s>>>(a, stack);
+  else if (mode == kAppend) walk_kernel<kAppend, PHASE, HEX><<<grid, threads, smem, s>>>(a, stack);
+  else walk_kernel<kCount, PHASE, HEX><<<grid, threads, smem, s>>>(a, stack);
   count_launch();
 }
 
-template <int STACK>
-static void walk_launch_mode(const WalkArgs& a, int mode, int phase, int grid, cudaStream_t s) {
-  if (phase == 1) walk_launch_phase<STACK, 1>(a, mode, grid, s);
-  else if (phase == 2) walk_launch_phase<STACK, 2>(a, mode, grid, s);
-  else walk_launch_phase<STACK, 0>(a, mode, grid, s);
-}
-
-/* One traversal.  The per-warp stack of kWarpStack entries keeps the
+/* How a walk runs.  The per-warp stack of kWarpStack entries keeps the
  * blocks' shared memory small enough for register-bound residency; a warp
- * that would exhaust it sets error 2 and stops, and the whole launch then
- * runs once more with kWarpStackLarge entries (every output of a launch is
- * rewritten by the re-run: per-bucket counts and entries, and in append
- * mode the pools, whose counters are reset first). */
-static void walk_run(const WalkArgs& a, int mode, cudaStream_t s, int phase = 0) {
+ * that would exhaust it sets error 2 and stops, and the walk then runs once
+ * more with kWarpStackLarge entries.  A group that outgrows its slots sets
+ * the second word, and the groups' lists are then counted and filled.  The
+ * host reads both words where it waits for the walk's totals anyway. */
+struct WalkTry {
+  bool large = false, slots = true;
+  bool again(const int* err) {
+    if (err[0] == 2 && !large) {
+      large = true;
+      g_stack_reruns.fetch_add(1);
+      return true;
+    }
+    if (err[0] == 0 && err[1] != 0 && slots) {
+      slots = false;
+      return true;
+    }
+    return false;
+  }
+};
+
+/* One traversal. */
+static void walk_run(const WalkArgs& a, int mode, cudaStream_t s, int phase, bool large) {
   const long long units = phase == 1 ? a.n_groups : a.n_buckets;
   const long long warps = (units + a.bucket_stride - 1) / a.bucket_stride;
   const int grid = (int)((warps + kWalkWarps - 1) / kWalkWarps);
   if (grid <= 0) return;
-  if (g_test_small_stack.load()) walk_launch_mode<64>(a, mode, phase, grid, s);
-  else walk_launch_mode<kWarpStack>(a, mode, phase, grid, s);
-  int h = 0;
-  if (cudaMemcpyAsync(&h, a.error, sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
-      cudaStreamSynchronize(s) != cudaSuccess || h != 2)
-    return;  // launch errors surface at the caller's next check
-  if (cudaMemsetAsync(a.error, 0, sizeof(int), s) != cudaSuccess) return;
-  if (mode == kAppend && a.pool_next &&
-      cudaMemsetAsync(a.pool_next, 0, 64, s) != cudaSuccess)  // pool counters, overflow flag
-    return;
-  walk_launch_mode<kWarpStackLarge>(a, mode, phase, grid, s);
-  g_stack_reruns.fetch_add(1);
+  const int stack = large ? kWarpStackLarge : g_test_small_stack.load() ? 64 : kWarpStack;
+  const bool hex = a.order == 4;
+  if (phase == 1) hex ? walk_launch<1, true>(a, mode, stack, grid, s) : walk_launch<1, false>(a, mode, stack, grid, s);
+  else if (phase == 2) hex ? walk_launch<2, true>(a, mode, stack, grid, s) : walk_launch<2, false>(a, mode, stack, grid, s);
+  else hex ? walk_launch<0, true>(a, mode, stack, grid, s) : walk_launch<0, false>(a, mode, stack, grid, s);
 }
 
 static int walk_error(int h_err) {
@@ -1275,7 +1389,7 @@ static int walk_error(int h_err) {
                       __FILE__, __LINE__);
 }
 
-static int walk_launch(const ChangaTreeView* t, const ChangaWalkParams* p, bool fill, int* nc,
+static int walk_pass(const ChangaTreeView* t, const ChangaWalkParams* p, bool fill, int* nc,
                        int* np, int* ns, const long long* oc, const long long* op,
                        const long long* os, ILCell* cells, ILCell* parts, ILCell* soft,
                        cudaStream_t s) {
@@ -1294,20 +1408,25 @@ static int walk_launch(const ChangaTreeView* t, const ChangaWalkParams* p, bool 
   a.cells = (int2*)cells;
   a.parts = (int2*)parts;
   a.soft = (int2*)soft;
-  walk_run(a, fill ? kFill : kCount, s);
-  CHG_CUDA(cudaGetLastError());
-  int h_err = 0;
-  CHG_CUDA(cudaMemcpyAsync(&h_err, a.error, sizeof(int), cudaMemcpyDeviceToHost, s));
+  WalkTry how;
+  int h_err[2] = {0, 0};
+  for (;;) {
+    walk_run(a, fill ? kFill : kCount, s, 0, how.large);
+    CHG_CUDA(cudaGetLastError());
+    CHG_CUDA(cudaMemcpyAsync(h_err, a.error, sizeof(h_err), cudaMemcpyDeviceToHost, s));
+    CHG_CUDA(cudaStreamSynchronize(s));
+    if (!how.again(h_err)) break;
+    CHG_CUDA(cudaMemsetAsync(a.error, 0, 256, s));
+  }
   CHG_CUDA(cudaFreeAsync(block, s));
-  CHG_CUDA(cudaStreamSynchronize(s));
-  return h_err ? walk_error(h_err) : 0;
+  return h_err[0] ? walk_error(h_err[0]) : 0;
 }
 
 extern "C" int changa_walk_count(const ChangaTreeView* tree, const ChangaWalkParams* p,
                                  int* n_cells, int* n_parts, int* n_soft, cudaStream_t s) {
   if (!n_cells || !n_parts || (p && p->order == 4 && !n_soft))
     return record_error(CHANGA_E_INVALID_ARG, "walk_count: outputs", __FILE__, __LINE__);
-  return walk_launch(tree, p, false, n_cells, n_parts, n_soft, nullptr, nullptr, nullptr, nullptr,
+  return walk_pass(tree, p, false, n_cells, n_parts, n_soft, nullptr, nullptr, nullptr, nullptr,
                      nullptr, nullptr, s);
 }
 
@@ -1318,23 +1437,27 @@ extern "C" int changa_walk_fill(const ChangaTreeView* tree, const ChangaWalkPara
   if (!off_cells || !off_parts || !cells || !parts ||
       (p && p->order == 4 && (!off_soft || !soft)))
     return record_error(CHANGA_E_INVALID_ARG, "walk_fill: outputs", __FILE__, __LINE__);
-  return walk_launch(tree, p, true, nullptr, nullptr, nullptr, off_cells, off_parts, off_soft,
+  return walk_pass(tree, p, true, nullptr, nullptr, nullptr, off_cells, off_parts, off_soft,
                      cells, parts, soft, s);
 }
 
 /* ---- both passes and the prefix sums, lists owned by the result ---- */
 
-/* append-pass pool size over the sampled estimate of the entries */
+/* append-pass pool size over the estimate of the entries */
 static std::atomic<double> g_pool_factor{1.2};
 
 extern "C" void changa_walk_set_pool_factor(double f) { g_pool_factor.store(f > 0 ? f : 0.0); }
 
 extern "C" void changa_walk_set_test_small_stack(int on) { g_test_small_stack.store(on ? 1 : 0); }
 
-/* Two-phase walk: groups of at most g_group_max buckets, for quadrupole
- * walks of at least g_group_min buckets (0 turns it off). */
+/* Two-phase walk: groups of at most g_group_max buckets, for walks of at
+ * least g_group_min buckets (0 turns it off).  Below some 10000 buckets the
+ * groups are too few to fill the GPU and the two phases cost more than the
+ * shared part saves; us a walk, one phase / two (open and periodic trees):
+ * 5524 buckets 482 / 555, 10086 605 / 638, 10447 645 / 654, 11944 746 / 706,
+ * 23834 1422 / 1058. */
 static std::atomic<int> g_group_max{32};
-static std::atomic<int> g_group_min{4096};
+static std::atomic<int> g_group_min{10240};
 
 extern "C" void changa_walk_set_groups(int max_buckets, int min_tree_buckets) {
   g_group_max.store(max_buckets > 0 ? max_buckets : 0);
@@ -1375,96 +1498,132 @@ struct Scratch {
   }
 };
 
-/* Groups of at most gmax buckets and phase 1 of the two-phase walk.
- * Phase 1 walks each group's node once: its chain down to the group node
- * is shared by all the group's buckets, so the entries accepted on it (the
- * group's prefix lists) and those still undecided at the group node (its
- * frontier) are the same for each of them.  Fills a's group fields and the
- * phase 2 inputs (prefix lists, frontier), in scratch of sc. */
-static int walk_phase1(WalkArgs& a, const ChangaTreeView* t, int gmax, Scratch& sc,
+/* The groups of a two-phase walk (device arrays in scratch). */
+struct WalkGroups {
+  int n = 0;
+  int* bucket_group = nullptr;
+  int* node = nullptr;
+  int* cnt = nullptr;       // 3 n: prefix cells, prefix particles, frontier
+  int2* slots = nullptr;    // the append pass's slots, when taken
+};
+
+/* Groups of at most gmax buckets; waits for their number. */
+static int walk_groups(WalkGroups& gr, const ChangaTreeView* t, int gmax, Scratch& sc,
                        cudaStream_t s) {
   const int nb = t->n_buckets;
-  const int tiles = (nb + kScanTile - 1) / kScanTile;
-  long long* ts = (long long*)sc.alloc((size_t)tiles * sizeof(long long));
-  if (!ts) return record_error(cudaErrorMemoryAllocation, "walk: memory", __FILE__, __LINE__);
-  int h_err = 0;
-  int* bfirst = (int*)sc.alloc((size_t)nb * sizeof(int));
-  int* gn = (int*)sc.alloc((size_t)nb * sizeof(int));
-  int* flag = (int*)sc.alloc((size_t)nb * sizeof(int));
-  long long* gex = (long long*)sc.alloc((size_t)(nb + 1) * sizeof(long long));
-  int* gex32 = (int*)sc.alloc((size_t)(nb + 1) * sizeof(int));
-  int* bucket_group = (int*)sc.alloc((size_t)nb * sizeof(int));
-  int* group_node = (int*)sc.alloc((size_t)nb * sizeof(int));
-  if (!bfirst || !gn || !flag || !gex || !gex32 || !bucket_group || !group_node)
-    return record_error(cudaErrorMemoryAllocation, "walk: memory", __FILE__, __LINE__);
+  const size_t nbp = ((size_t)nb + 2) & ~size_t(1);
+  char* q = (char*)sc.alloc((size_t)scan_tiles(nb) * sizeof(long long) + nbp * (8 + 5 * 4));
+  if (!q) return record_error(cudaErrorMemoryAllocation, "walk: memory", __FILE__, __LINE__);
+  long long* ts = (long long*)q;
+  long long* gex = ts + scan_tiles(nb);
+  int* bfirst = (int*)(gex + nbp);
+  int* gn = bfirst + nbp;
+  int* flag = gn + nbp;
+  gr.bucket_group = flag + nbp;
+  gr.node = gr.bucket_group + nbp;
   const long long gb = ((long long)nb + 255) / 256, cap = (long long)sm_count() * 8;
   const int grid = (int)(gb < cap ? gb : cap);
   bucket_first_kernel<<<grid, 256, 0, s>>>(t->bucket_node, t->info, t->n_nodes, nb, bfirst);
   bucket_group_node_kernel<<<grid, 256, 0, s>>>(t->bucket_node, t->parent, t->info, bfirst,
                                                 t->n_nodes, nb, gmax, gn);
   group_flag_kernel<<<grid, 256, 0, s>>>(gn, nb, flag);
-  scan_tile_sums_kernel<<<tiles, kScanThreads, 0, s>>>(flag, nb, ts);
-  scan_tiles_kernel<<<1, kScanThreads, 0, s>>>(ts, tiles);
-  scan_apply_kernel<<<tiles, kScanThreads, 0, s>>>(flag, nb, ts, gex, gex32);
-  group_ids_kernel<<<grid, 256, 0, s>>>(gn, flag, gex, nb, bucket_group, group_node);
-  count_launch(7);
-  long long ng_ll = 0;
-  if (cudaMemcpyAsync(&ng_ll, gex + nb, sizeof(long long), cudaMemcpyDeviceToHost, s) !=
-          cudaSuccess ||
-      cudaStreamSynchronize(s) != cudaSuccess || ng_ll <= 0 || ng_ll > nb)
+  launch_scans(flag, nb, 1, ts, gex, ScanOut{}, s);
+  group_ids_kernel<<<grid, 256, 0, s>>>(gn, flag, gex, nb, gr.bucket_group, gr.node);
+  count_launch(4);
+  long long ng = 0;
+  if (cudaMemcpyAsync(&ng, gex + nb, sizeof(long long), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+      cudaStreamSynchronize(s) != cudaSuccess || ng <= 0 || ng > nb)
     return record_error((int)cudaGetLastError(), "walk: groups", __FILE__, __LINE__);
-  const int ng = (int)ng_ll;
-  int* gcnt = (int*)sc.alloc((size_t)3 * ng * sizeof(int));
-  long long* goff = (long long*)sc.alloc((size_t)3 * (ng + 1) * sizeof(long long));
-  int* goff32 = (int*)sc.alloc((size_t)3 * (ng + 1) * sizeof(int));
-  if (!gcnt || !goff || !goff32)
+  gr.n = (int)ng;
+  gr.cnt = (int*)sc.alloc((size_t)3 * gr.n * sizeof(int));
+  if (!gr.cnt) return record_error(cudaErrorMemoryAllocation, "walk: memory", __FILE__, __LINE__);
+  return 0;
+}
+
+/* Entries of a group's slots, 48 KB in all.  The largest of 20000 groups of 32
+ * buckets of at most 32 (2^23 NFW particles, theta 0.7): 686 cells, 1507
+ * particles, 175 in the frontier; of 5600 at theta 0.5: 1292, 2219, 365. */
+constexpr int kSlotCells = 2048, kSlotParts = 3072, kSlotFront = 1024;
+
+/* Phase 1 of the two-phase walk: each group's node walked once.  Its chain
+ * down to the group node is shared by all the group's buckets, so the
+ * entries accepted on it (the group's prefix lists) and those still
+ * undecided at the group node (its frontier) are the same for each of them.
+ * Fills a's group fields and the phase 2 inputs, in scratch of sc.  With
+ * slots nothing is waited for. */
+static int walk_phase1(WalkArgs& a, WalkGroups& gr, WalkTry& how, Scratch& sc, cudaStream_t s) {
+  const int ng = gr.n;
+  const auto no_memory = [&] {
     return record_error(cudaErrorMemoryAllocation, "walk: memory", __FILE__, __LINE__);
-  a.group_node = group_node;
+  };
+  if (cudaMemsetAsync(a.error, 0, 256, s) != cudaSuccess ||
+      cudaMemsetAsync(gr.cnt, 0, (size_t)3 * ng * sizeof(int), s) != cudaSuccess)
+    return record_error((int)cudaGetLastError(), "walk: group reset", __FILE__, __LINE__);
+  a.group_node = gr.node;
   a.n_groups = ng;
-  a.bucket_group = bucket_group;
-  a.n_cells = gcnt;
-  a.n_parts = gcnt + ng;
+  a.bucket_group = gr.bucket_group;
+  a.n_cells = gr.cnt;
+  a.n_parts = gr.cnt + ng;
+  a.n_front = gr.cnt + 2 * (size_t)ng;
   a.n_soft = nullptr;
-  a.n_front = gcnt + 2 * (size_t)ng;
-  walk_run(a, kCount, s, 1);
-  const int gtiles = (ng + kScanTile - 1) / kScanTile;
-  for (int k = 0; k < 3; ++k) {
-    scan_tile_sums_kernel<<<gtiles, kScanThreads, 0, s>>>(gcnt + (size_t)k * ng, ng, ts);
-    scan_tiles_kernel<<<1, kScanThreads, 0, s>>>(ts, gtiles);
-    scan_apply_kernel<<<gtiles, kScanThreads, 0, s>>>(gcnt + (size_t)k * ng, ng, ts,
-                                                      goff + (size_t)k * (ng + 1),
-                                                      goff32 + (size_t)k * (ng + 1));
-    count_launch(3);
-  }
-  long long gtot[3] = {0, 0, 0};
-  for (int k = 0; k < 3; ++k)
-    cudaMemcpyAsync(&gtot[k], goff + (size_t)k * (ng + 1) + ng, sizeof(long long),
-                    cudaMemcpyDeviceToHost, s);
-  cudaMemcpyAsync(&h_err, a.error, sizeof(int), cudaMemcpyDeviceToHost, s);
-  if (cudaStreamSynchronize(s) != cudaSuccess)
-    return record_error((int)cudaGetLastError(), "walk: group count", __FILE__, __LINE__);
-  if (h_err) return walk_error(h_err);
-  int2* pre_cells = (int2*)sc.alloc((size_t)(gtot[0] > 0 ? gtot[0] : 1) * sizeof(int2));
-  int2* pre_parts = (int2*)sc.alloc((size_t)(gtot[1] > 0 ? gtot[1] : 1) * sizeof(int2));
-  int2* front = (int2*)sc.alloc((size_t)(gtot[2] > 0 ? gtot[2] : 1) * sizeof(int2));
-  if (!pre_cells || !pre_parts || !front)
-    return record_error(cudaErrorMemoryAllocation, "walk: memory", __FILE__, __LINE__);
-  a.off_cells = goff;
-  a.off_parts = goff + (ng + 1);
   a.off_soft = nullptr;
-  a.off_front = goff + 2 * (size_t)(ng + 1);
-  a.cells = pre_cells;
-  a.parts = pre_parts;
   a.soft = nullptr;
-  a.front = front;
-  walk_run(a, kFill, s, 1);
+  a.slot[0] = kSlotCells;
+  a.slot[1] = kSlotParts;
+  a.slot[2] = kSlotFront;
+  for (int k = 0; k < 3; ++k) {
+    a.gcnt[k] = gr.cnt + (size_t)k * ng;
+    a.goff[k] = nullptr;
+  }
+  if (how.slots && !gr.slots) {
+    gr.slots = (int2*)sc.alloc((size_t)ng * (kSlotCells + kSlotParts + kSlotFront) * sizeof(int2));
+    if (!gr.slots) {
+      cudaGetLastError();  // no room for the slots: count and fill
+      how.slots = false;
+    }
+  }
+  if (how.slots) {
+    a.cells = gr.slots;
+    a.parts = a.cells + (size_t)ng * kSlotCells;
+    a.front = a.parts + (size_t)ng * kSlotParts;
+    walk_run(a, kAppend, s, 1, how.large);
+  } else {
+    walk_run(a, kCount, s, 1, how.large);
+    const int gt = scan_tiles(ng);
+    long long* ts = (long long*)sc.alloc((size_t)3 * (gt + ng + 1) * sizeof(long long));
+    if (!ts) return no_memory();
+    long long* off = ts + 3 * (size_t)gt;
+    launch_scans(gr.cnt, ng, 3, ts, off, ScanOut{}, s);
+    long long tot[3] = {0, 0, 0};
+    int h_err = 0;
+    for (int k = 0; k < 3; ++k)
+      cudaMemcpyAsync(&tot[k], off + (size_t)k * (ng + 1) + ng, sizeof(long long),
+                      cudaMemcpyDeviceToHost, s);
+    cudaMemcpyAsync(&h_err, a.error, sizeof(int), cudaMemcpyDeviceToHost, s);
+    if (cudaStreamSynchronize(s) != cudaSuccess)
+      return record_error((int)cudaGetLastError(), "walk: group count", __FILE__, __LINE__);
+    if (h_err == 2 && !how.large) {
+      how.large = true;
+      g_stack_reruns.fetch_add(1);
+      return walk_phase1(a, gr, how, sc, s);
+    }
+    if (h_err) return walk_error(h_err);
+    a.cells = (int2*)sc.alloc((size_t)(tot[0] + tot[1] + tot[2] + 1) * sizeof(int2));
+    if (!a.cells) return no_memory();
+    a.parts = a.cells + tot[0];
+    a.front = a.parts + tot[1];
+    for (int k = 0; k < 3; ++k) a.goff[k] = off + (size_t)k * (ng + 1);
+    a.off_cells = a.goff[0];
+    a.off_parts = a.goff[1];
+    a.off_front = a.goff[2];
+    walk_run(a, kFill, s, 1, how.large);
+  }
   /* phase 2 reads the group outputs */
-  a.pre_off[0] = goff;
-  a.pre_off[1] = goff + (ng + 1);
-  a.pre[0] = pre_cells;
-  a.pre[1] = pre_parts;
-  a.off_cells = a.off_parts = a.off_soft = nullptr;
-  a.cells = a.parts = a.soft = nullptr;
+  a.glist[0] = a.cells;
+  a.glist[1] = a.parts;
+  a.glist[2] = a.front;
+  a.off_cells = a.off_parts = a.off_front = nullptr;
+  a.cells = a.parts = a.front = nullptr;
   a.n_front = nullptr;
   return 0;
 }
@@ -1492,94 +1651,107 @@ extern "C" int changa_walk(const ChangaTreeView* t, const ChangaWalkParams* p,
     }
     return rc;
   };
-  auto alloc = [&](size_t bytes) { return sc.alloc(bytes); };
-  int* cnt = (int*)alloc((size_t)3 * nb * sizeof(int));
-  const int tiles = (nb + kScanTile - 1) / kScanTile;
-  long long* ts = (long long*)alloc((size_t)tiles * sizeof(long long));
-  long long* off = (long long*)alloc((size_t)3 * (nb + 1) * sizeof(long long));
-  unsigned int* ctr = (unsigned int*)alloc(64);
-  if (!cnt || !ts || !off || !ctr)
-    return finish(record_error(cudaErrorMemoryAllocation, "walk: memory", __FILE__, __LINE__));
-  int h_err = 0;
+  auto no_memory = [&](const char* what) {
+    return finish(record_error(cudaErrorMemoryAllocation, what, __FILE__, __LINE__));
+  };
+  /* pool counters, tile sums, offsets, counts */
+  const int tiles = scan_tiles(nb);
+  char* q = (char*)sc.alloc(256 + (size_t)3 * (tiles + nb + 1) * sizeof(long long) +
+                            (size_t)3 * nb * sizeof(int));
+  if (!q) return no_memory("walk: memory");
+  unsigned int* ctr = (unsigned int*)q;
+  long long* ts = (long long*)(q + 256);
+  long long* off = ts + (size_t)3 * tiles;
+  int* cnt = (int*)(off + (size_t)3 * (nb + 1));
+  ScanOut markers{};
+  for (int k = 0; k < nl; ++k) {
+    if (cudaMallocAsync((void**)&out->markers[k], (size_t)(nb + 1) * sizeof(int), s) != cudaSuccess)
+      return no_memory("walk: markers");
+    markers.off32[k] = out->markers[k];
+  }
   /* Walks of many buckets run in two phases (walk_phase1); phase 2 walks
    * each bucket from its group's frontier, its lists starting with the
    * group's prefix. */
-  int phase = 0;
+  WalkGroups gr;
   const int gmax = g_group_max.load();
-  if (gmax > 0 && g_group_min.load() > 0 && nb >= g_group_min.load()) {
-    if (int rc = walk_phase1(a, t, gmax, sc, s)) return finish(rc);
-    phase = 2;
-  }
-  /* Large trees: one traversal appends the entries into pools of chunks
-   * sized from a sampled count (every 16th bucket); small trees (where the
-   * sample's fixed costs dominate) count, then fill. */
-  bool appended = false;
+  const int phase = gmax > 0 && g_group_min.load() > 0 && nb >= g_group_min.load() ? 2 : 0;
+  if (phase == 2)
+    if (int rc = walk_groups(gr, t, gmax, sc, s)) return finish(rc);
+  /* One traversal appends the entries into pools of chunks; a pool that
+   * falls short costs a fill pass, and the counts are right either way.
+   * Large trees size the pools from a count of one bucket in `stride` (some
+   * kSample of them: their mean is within a few percent, and the pools hold
+   * a fifth more); small trees, where that count would cost as much as what
+   * it saves, take kGuess entries per bucket and list. */
+  constexpr int kSampleMin = 16384, kSample = 2048, kGuess = 1024;
+  bool pools = false, tried = false;
   long long chunks[3] = {0, 0, 0};
-  if (nb >= 16384) {
-    const int stride = 16, nsamp = (nb + stride - 1) / stride;
-    int* samp = (int*)alloc((size_t)3 * nsamp * sizeof(int));
-    if (!samp)
-      return finish(record_error(cudaErrorMemoryAllocation, "walk: memory", __FILE__, __LINE__));
-    a.n_cells = samp;
-    a.n_parts = samp + nsamp;
-    a.n_soft = nl == 3 ? samp + 2 * nsamp : nullptr;
-    a.bucket_stride = stride;
-    walk_run(a, kCount, s, phase);
-    a.bucket_stride = 1;
-    std::vector<int> hs((size_t)nl * nsamp);
-    if (cudaMemcpyAsync(hs.data(), samp, hs.size() * sizeof(int), cudaMemcpyDeviceToHost, s) !=
-            cudaSuccess ||
-        cudaStreamSynchronize(s) != cudaSuccess)
-      return finish(record_error((int)cudaGetLastError(), "walk: sample", __FILE__, __LINE__));
-    bool ok = true;
-    for (int k = 0; k < nl && ok; ++k) {
-      double sum = 0;
-      for (int i = 0; i < nsamp; ++i) sum += hs[(size_t)k * nsamp + i];
-      chunks[k] = (long long)(sum * ((double)nb / nsamp) * g_pool_factor.load() / kChunk) + nb + 256;
-      a.pool[k] = (int2*)alloc((size_t)chunks[k] * kChunk * sizeof(int2));
-      a.chunk_bucket[k] = (int*)alloc((size_t)chunks[k] * sizeof(int));
-      a.chunk_rank[k] = (int*)alloc((size_t)chunks[k] * sizeof(int));
-      a.pool_chunks[k] = chunks[k];
-      ok = a.pool[k] && a.chunk_bucket[k] && a.chunk_rank[k];
+  long long tot[3];
+  unsigned int hc[16];
+  int h_err[2];
+  WalkTry how;
+  for (;;) {
+    if (phase == 2) {
+      if (int rc = walk_phase1(a, gr, how, sc, s)) return finish(rc);
+    } else if (cudaMemsetAsync(a.error, 0, 256, s) != cudaSuccess) {
+      return finish(record_error((int)cudaGetLastError(), "walk: reset", __FILE__, __LINE__));
     }
-    if (ok && cudaMemsetAsync(ctr, 0, 64, s) == cudaSuccess) {
+    if (!tried) {
+      double est[3] = {(double)kGuess * nb, (double)kGuess * nb, (double)kGuess * nb};
+      if (nb >= kSampleMin) {
+        const int stride = std::max(16, nb / kSample), nsamp = (nb + stride - 1) / stride;
+        a.n_cells = cnt;
+        a.n_parts = cnt + nsamp;
+        a.n_soft = nl == 3 ? cnt + 2 * nsamp : nullptr;
+        a.bucket_stride = stride;
+        walk_run(a, kCount, s, phase, how.large);
+        a.bucket_stride = 1;
+        std::vector<int> hs((size_t)nl * nsamp);
+        if (cudaMemcpyAsync(hs.data(), cnt, hs.size() * sizeof(int), cudaMemcpyDeviceToHost, s) !=
+                cudaSuccess ||
+            cudaMemcpyAsync(h_err, a.error, sizeof(h_err), cudaMemcpyDeviceToHost, s) !=
+                cudaSuccess ||
+            cudaStreamSynchronize(s) != cudaSuccess)
+          return finish(record_error((int)cudaGetLastError(), "walk: sample", __FILE__, __LINE__));
+        if (how.again(h_err)) continue;
+        if (h_err[0]) return finish(walk_error(h_err[0]));
+        for (int k = 0; k < nl; ++k) {
+          est[k] = 0;
+          for (int i = 0; i < nsamp; ++i) est[k] += hs[(size_t)k * nsamp + i];
+          est[k] *= (double)nb / nsamp;
+        }
+      }
+      tried = pools = true;
+      for (int k = 0; k < nl && pools; ++k) {
+        chunks[k] = (long long)(est[k] * g_pool_factor.load() / kChunk) + nb + 256;
+        a.pool[k] = (int2*)sc.alloc((size_t)chunks[k] * kChunk * sizeof(int2));
+        a.chunk_bucket[k] = (int*)sc.alloc((size_t)chunks[k] * 2 * sizeof(int));
+        a.chunk_rank[k] = a.chunk_bucket[k] + chunks[k];
+        a.pool_chunks[k] = chunks[k];
+        pools = a.pool[k] && a.chunk_bucket[k];
+      }
+      if (!pools) cudaGetLastError();  // pools that did not fit: count and fill instead
       a.pool_next = ctr;
       a.overflow = reinterpret_cast<int*>(ctr + 8);
-      a.n_cells = cnt;
-      a.n_parts = cnt + nb;
-      a.n_soft = nl == 3 ? cnt + 2 * (size_t)nb : nullptr;
-      walk_run(a, kAppend, s, phase);
-      appended = true;
-    } else {
-      cudaGetLastError();  // a pool that did not fit: count and fill instead
     }
-  }
-  if (!appended) {
     a.n_cells = cnt;
     a.n_parts = cnt + nb;
     a.n_soft = nl == 3 ? cnt + 2 * (size_t)nb : nullptr;
-    walk_run(a, kCount, s, phase);
+    if (cudaMemsetAsync(ctr, 0, 64, s) != cudaSuccess)
+      return finish(record_error((int)cudaGetLastError(), "walk: reset", __FILE__, __LINE__));
+    walk_run(a, pools ? kAppend : kCount, s, phase, how.large);
+    /* offsets (and the int32 markers) of every list */
+    launch_scans(cnt, nb, nl, ts, off, markers, s);
+    for (int k = 0; k < nl; ++k)
+      cudaMemcpyAsync(&tot[k], off + (size_t)k * (nb + 1) + nb, sizeof(long long),
+                      cudaMemcpyDeviceToHost, s);
+    cudaMemcpyAsync(hc, ctr, 64, cudaMemcpyDeviceToHost, s);
+    cudaMemcpyAsync(h_err, a.error, sizeof(h_err), cudaMemcpyDeviceToHost, s);
+    if (cudaStreamSynchronize(s) != cudaSuccess)
+      return finish(record_error((int)cudaGetLastError(), "walk: count", __FILE__, __LINE__));
+    if (!how.again(h_err)) break;
   }
-  /* offsets (and the int32 markers) of every list */
-  for (int k = 0; k < nl; ++k) {
-    if (cudaMallocAsync((void**)&out->markers[k], (size_t)(nb + 1) * sizeof(int), s) != cudaSuccess)
-      return finish(record_error(cudaErrorMemoryAllocation, "walk: markers", __FILE__, __LINE__));
-    scan_tile_sums_kernel<<<tiles, kScanThreads, 0, s>>>(cnt + (size_t)k * nb, nb, ts);
-    scan_tiles_kernel<<<1, kScanThreads, 0, s>>>(ts, tiles);
-    scan_apply_kernel<<<tiles, kScanThreads, 0, s>>>(cnt + (size_t)k * nb, nb, ts,
-                                                     off + (size_t)k * (nb + 1), out->markers[k]);
-    count_launch(3);
-  }
-  long long tot[3] = {0, 0, 0};
-  unsigned int hc[16] = {0};
-  for (int k = 0; k < nl; ++k)
-    cudaMemcpyAsync(&tot[k], off + (size_t)k * (nb + 1) + nb, sizeof(long long),
-                    cudaMemcpyDeviceToHost, s);
-  cudaMemcpyAsync(hc, ctr, 64, cudaMemcpyDeviceToHost, s);
-  cudaMemcpyAsync(&h_err, a.error, sizeof(int), cudaMemcpyDeviceToHost, s);
-  if (cudaStreamSynchronize(s) != cudaSuccess)
-    return finish(record_error((int)cudaGetLastError(), "walk: count", __FILE__, __LINE__));
-  if (h_err) return finish(walk_error(h_err));
+  if (h_err[0]) return finish(walk_error(h_err[0]));
   for (int k = 0; k < nl; ++k) {
     if (tot[k] >= (1LL << 31) - 1)
       return finish(record_error(CHANGA_E_TOO_LARGE, "walk: list exceeds int32 markers", __FILE__,
@@ -1587,10 +1759,10 @@ extern "C" int changa_walk(const ChangaTreeView* t, const ChangaWalkParams* p,
     out->n_entries[k] = tot[k];
     if (cudaMallocAsync((void**)&out->list[k], (size_t)(tot[k] > 0 ? tot[k] : 1) * sizeof(ILCell),
                         s) != cudaSuccess)
-      return finish(record_error(cudaErrorMemoryAllocation, "walk: lists", __FILE__, __LINE__));
+      return no_memory("walk: lists");
   }
-  const bool overflow = appended && hc[8] != 0;
-  if (appended && !overflow) {
+  const bool overflow = pools && hc[8] != 0;
+  if (pools && !overflow) {
     for (int k = 0; k < nl; ++k) {
       const long long used = (long long)hc[k] < chunks[k] ? (long long)hc[k] : chunks[k];
       if (used == 0) continue;
@@ -1602,20 +1774,20 @@ extern "C" int changa_walk(const ChangaTreeView* t, const ChangaWalkParams* p,
       count_launch();
     }
   } else {
-    /* entries by a second traversal (small trees, or pools that ran short) */
+    /* entries by a second traversal (pools that ran short or did not fit) */
     a.off_cells = off;
     a.off_parts = off + (nb + 1);
     a.off_soft = nl == 3 ? off + 2 * (size_t)(nb + 1) : nullptr;
     a.cells = (int2*)out->list[0];
     a.parts = (int2*)out->list[1];
     a.soft = nl == 3 ? (int2*)out->list[2] : nullptr;
-    walk_run(a, kFill, s, phase);
-    cudaMemcpyAsync(&h_err, a.error, sizeof(int), cudaMemcpyDeviceToHost, s);
+    walk_run(a, kFill, s, phase, how.large);
+    cudaMemcpyAsync(h_err, a.error, sizeof(h_err), cudaMemcpyDeviceToHost, s);
   }
-  out->passes = appended ? (overflow ? 3 : 1) : 2;
+  out->passes = !pools ? 2 : overflow ? 3 : 1;
   if (cudaStreamSynchronize(s) != cudaSuccess)
     return finish(record_error((int)cudaGetLastError(), "walk: entries", __FILE__, __LINE__));
-  if (h_err) return finish(walk_error(h_err));
+  if (h_err[0]) return finish(walk_error(h_err[0]));
   return finish(0);
 }
 
@@ -1665,7 +1837,8 @@ extern "C" int changa_walk_forces(const ChangaTreeView* t, const ChangaWalkParam
       (e = launch_pack_parts(parts, n_parts, ppk, s)) != cudaSuccess)
     return finish(record_error((int)e, "walk_forces: pack", __FILE__, __LINE__));
   const int gmax = g_group_max.load() > 0 ? g_group_max.load() : 32;
-  if (int rc = walk_phase1(a, t, gmax, sc, s)) return finish(rc);
+  WalkGroups gr;
+  if (int rc = walk_groups(gr, t, gmax, sc, s)) return finish(rc);
   FusedArgs f{};
   f.cells.src = pc;
   f.cells.n_src = t->n_nodes;
@@ -1677,29 +1850,25 @@ extern "C" int changa_walk_forces(const ChangaTreeView* t, const ChangaWalkParam
   f.parts.fperiod_d = p->period;
   f.vars = vars;
   f.queue = queue;
-  /* a warp that would exhaust its stack stops with error 2; the launch
-   * then runs again with the larger stack and rewrites every target */
-  int h_err = 0;
-  for (int attempt = 0; attempt < 2; ++attempt) {
-    if ((e = cudaMemsetAsync(queue, 0, sizeof(unsigned int), s)) != cudaSuccess ||
-        (e = cudaMemsetAsync(a.error, 0, sizeof(int), s)) != cudaSuccess)
+  /* A warp that would exhaust its stack stops with error 2; both phases then
+   * run again with the larger stack, and every target is rewritten.  So do
+   * they with counted group lists when a group outgrew its slots. */
+  WalkTry how;
+  int h_err[2] = {0, 0};
+  do {
+    if ((e = cudaMemsetAsync(queue, 0, sizeof(unsigned int), s)) != cudaSuccess)
       return finish(record_error((int)e, "walk_forces: reset", __FILE__, __LINE__));
-    if (attempt == 1) {
-      e = launch_walk_eval<kWarpStackLarge, 2>(a, f, s);
-      g_stack_reruns.fetch_add(1);
-    } else if (g_test_small_stack.load()) {
-      e = launch_walk_eval<32, kFusedWarps>(a, f, s);  // runs out on the first opening steps
-    } else {
-      e = launch_walk_eval<kWarpStack, kFusedWarps>(a, f, s);
-    }
+    if (int rc = walk_phase1(a, gr, how, sc, s)) return finish(rc);
+    if (how.large) e = launch_walk_eval<kWarpStackLarge, 2>(a, f, s);
+    else if (g_test_small_stack.load()) e = launch_walk_eval<32, kFusedWarps>(a, f, s);  // runs out at once
+    else e = launch_walk_eval<kWarpStack, kFusedWarps>(a, f, s);
     if (e != cudaSuccess) return finish(record_error((int)e, "walk_forces: launch", __FILE__, __LINE__));
-    if ((e = cudaMemcpyAsync(&h_err, a.error, sizeof(int), cudaMemcpyDeviceToHost, s)) !=
+    if ((e = cudaMemcpyAsync(h_err, a.error, sizeof(h_err), cudaMemcpyDeviceToHost, s)) !=
             cudaSuccess ||
         (e = cudaStreamSynchronize(s)) != cudaSuccess)
       return finish(record_error((int)e, "walk_forces: status", __FILE__, __LINE__));
-    if (h_err != 2) break;
-  }
-  if (h_err) return finish(walk_error(h_err));
+  } while (how.again(h_err));
+  if (h_err[0]) return finish(walk_error(h_err[0]));
   if (ewald && (e = launch_ewald_fp(kMix, parts, n_parts, nullptr, n_parts, *ewald, vars, s)) !=
                    cudaSuccess)
     return finish(record_error((int)e, "walk_forces: ewald", __FILE__, __LINE__));

@@ -377,17 +377,17 @@ int changa_walk_fill(const ChangaTreeView *tree, const ChangaWalkParams *p,
                      const long long *off_soft, ILCell *cells, ILCell *parts, ILCell *soft,
                      cudaStream_t stream);
 
-/* The whole walk in one call.  Trees of 16384 buckets or more take one
- * traversal: a count of every 16th bucket sizes pools of 256-entry chunks,
- * one pass counts every bucket's lists and appends their entries chunk by
- * chunk, and a gather puts the chunks in list order (a fill pass replaces
- * the gather if a pool ran short).  Smaller trees count, then fill.  The
+/* The whole walk in one call.  One pass counts every bucket's lists and
+ * appends their entries to pools of 256-entry chunks, and a gather puts the
+ * chunks in list order (a fill pass replaces the gather if a pool ran short).
+ * For trees of 16384 buckets or more a count of some 2000 buckets sizes the
+ * pools; smaller trees take room for 1024 entries per bucket and list.  The
  * lists and markers are device arrays owned by the result until
  * changa_walk_lists_free: list k (0 cells, 1 particles, 2 softened cells
  * when order is 4) holds n_entries[k] ILCells, bucket b's entries at
  * markers[k][b] .. markers[k][b + 1], in the same order as count + fill
- * write them.  passes: 1 (append + gather), 2 (count + fill), 3 (append,
- * then fill).  Returns after the stream has finished. */
+ * write them.  passes: 1 (append + gather), 2 (count + fill, when the
+ * pools cannot be had), 3 (append, then fill).  Returns after the stream has finished. */
 typedef struct ChangaWalkLists {
   int n_buckets;
   int order;
@@ -399,7 +399,7 @@ typedef struct ChangaWalkLists {
 int changa_walk(const ChangaTreeView *tree, const ChangaWalkParams *p, ChangaWalkLists *out,
                 cudaStream_t stream);
 void changa_walk_lists_free(ChangaWalkLists *out);
-/* Append-pass pool capacity as a multiple of the sampled estimate of the
+/* Append-pass pool capacity as a multiple of the estimate of the
  * entries (default 1.2; 0 leaves one chunk per bucket and list, so lists
  * longer than one chunk end in the fill pass). */
 void changa_walk_set_pool_factor(double factor);
@@ -414,7 +414,7 @@ long long changa_walk_stack_reruns(void);
  * (the highest node whose subtree holds no more), down to the group node,
  * which the group's buckets share; then each bucket from the entries still
  * undecided there.  The lists hold the same entries as the one-phase walk.
- * Defaults 32 and 4096; 0 for either walks every bucket from the root. */
+ * Defaults 32 and 10240; 0 for either walks every bucket from the root. */
 void changa_walk_set_groups(int max_buckets, int min_tree_buckets);
 
 /* Walk and forces in one pass, with no interaction lists (FP32-mixed form,
