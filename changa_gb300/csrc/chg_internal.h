@@ -31,6 +31,10 @@ struct ListArgs {
   float fperiod_f;
   double fperiod_d;
   unsigned int* queue;  // work counter, zero at launch
+  /* the launch before this one in the stream is a list kernel of the same
+   * evaluation (same vars, its inputs ready before that one began): this one
+   * may start as that one drains */
+  bool after_list = false;
 };
 
 /* Packed FP32-mixed layouts (built by pack kernels from FP64 inputs):
@@ -61,11 +65,16 @@ unsigned long long tma_launches();
 cudaError_t read_device_status(unsigned* bits);
 cudaError_t launch_pack_cells(const double* moments, long long n, float4* out, cudaStream_t s);
 cudaError_t launch_pack_parts(const double* parts, long long n, float4* out, cudaStream_t s);
+/* Both (cells of 12 doubles, or of 27 for the hexadecapole form) and kQueueInts
+ * zero words at queue, in one launch. */
+constexpr int kQueueInts = 192;
+cudaError_t launch_pack_step(bool hex, const double* moments, long long n_moments, float4* cells,
+                             const double* parts, long long n_parts, float4* packed,
+                             unsigned int* queue, cudaStream_t s);
 cudaError_t launch_zero_vars_f32(VariablePartData* v, long long n, cudaStream_t s);
 /* hexadecapole build: cell lists over 27-double (kF64) or packed (kMix)
  * moments; the pack; cells as point-mass particles {M, soft, cm} */
 cudaError_t launch_list_hex(int form, const ListArgs& a, cudaStream_t s);
-cudaError_t launch_pack_cells_hex(const double* moments, long long n, float4* out, cudaStream_t s);
 cudaError_t launch_cells_as_parts(const double* moments, int stride, long long n, double* out,
                                   cudaStream_t s);
 
@@ -78,7 +87,7 @@ cudaError_t launch_ewald_f32(const CompactPartData* parts, VariablePartData* var
 /* hex: the hexadecapole build's expansion (p.momc required) */
 cudaError_t launch_ewald_fp(int form, const double* parts, long long n_parts, const int* idx,
                             long long n_idx, const ChangaEwaldParams& p, double* vars,
-                            cudaStream_t s, bool hex = false);
+                            cudaStream_t s, bool hex = false, bool after_list = false);
 
 /* adjoint of the Ewald term (quadrupole root expansion, FP64): adds the
  * vector-Jacobian product of lam . a_ewald to grad (n x 4 {dL/dx, dL/dm});
@@ -111,6 +120,49 @@ struct TimingScope {
   cudaStream_t s;
   void* start;
 };
+
+#ifdef __CUDACC__
+/* Launches of one evaluation that only meet in the sums they add to vars
+ * overlap: the first lets its successor start once every one of its own
+ * blocks has (open_to_next), the successor's blocks take the places that it
+ * frees as it drains, and wait for its end (wait_for_last) before they touch
+ * vars.  Without the attribute of launch_after both are no-operations.  A
+ * kernel launched so has wait_for_last in every path that adds to vars.  us a
+ * step, one after another / so: 32768 Plummer particles 125 / 107, 6000 of
+ * them 52 / 40, 1200 37 / 25; 12000 periodic with Ewald 87 / 51; 2^20 with
+ * Ewald 2490 / 2350. */
+__device__ __forceinline__ void open_to_next() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void wait_for_last() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+/* The share of an SM's L1 kept as shared memory, in percent, asked for by every
+ * kernel that overlaps another: an SM that must change its split first drains,
+ * which cost more than the overlap gave (1200 periodic particles 82 us a step
+ * with the runtime's choice per kernel, 35 with one split; 75 without
+ * overlap).  60 holds each kernel's resident blocks, but the FP64 Ewald
+ * kernel's, so the FP64 form asks for all of it. */
+constexpr int kCarveoutFp32 = 60, kCarveoutFp64 = 100;
+template <typename K>
+inline void set_carveout(K kernel, int percent) {
+  cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, percent);
+}
+
+template <typename... P, typename... A>
+cudaError_t launch_after(void (*kernel)(P...), int grid, int threads, cudaStream_t s, bool overlap,
+                         A&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.stream = s;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = overlap ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+#endif
 
 }  // namespace chg
 

@@ -532,6 +532,7 @@ __global__ void __launch_bounds__(128) ewald_f64_kernel(const double* __restrict
     }
   }
   if (!live) return;
+  wait_for_last();
   double* v = vars + 5 * j;
   v[0] += ax;
   v[1] += ay;
@@ -868,6 +869,7 @@ __global__ void __launch_bounds__(kMixWarps * 32) ewald_mix_kernel(
     kz = fmaf(h.z, t, kz);
   }
   const float tl = P.twopi_over_L;
+  wait_for_last();
   double* v = vars + 5 * j;
   v[0] += (double)fx + (double)(tl * kx);
   v[1] += (double)fy + (double)(tl * ky);
@@ -948,7 +950,7 @@ static int ewald_threads(long long n) { return n <= 128ll * sm_count() ? 32 : 12
 
 cudaError_t launch_ewald_fp(int form, const double* parts, long long n_parts, const int* idx,
                             long long n_idx, const ChangaEwaldParams& p, double* vars,
-                            cudaStream_t s, bool hex) {
+                            cudaStream_t s, bool hex, bool after_list) {
   if (n_idx <= 0) return cudaSuccess;
   if (p.nEwhLoop < 0 || p.nEwhLoop > CHANGA_MAX_EWH || (p.nEwhLoop > 0 && !p.ewt) || !(p.L > 0) ||
       (hex && !p.momc))
@@ -986,11 +988,13 @@ cudaError_t launch_ewald_fp(int form, const double* parts, long long n_parts, co
     if (hex) fill_hex_root(p.momc, P.hex);
     const int threads = ewald_threads(n_idx);
     const int blocks = (int)((n_idx + threads - 1) / threads);
+    static const bool split = (set_carveout(ewald_f64_kernel<true>, kCarveoutFp64),
+                               set_carveout(ewald_f64_kernel<false>, kCarveoutFp64), true);
+    (void)split;
     TimingScope ts(kKidEwaldF64, s);
-    if (hex) ewald_f64_kernel<true><<<blocks, threads, 0, s>>>(parts, n_parts, idx, n_idx, vars, P);
-    else ewald_f64_kernel<false><<<blocks, threads, 0, s>>>(parts, n_parts, idx, n_idx, vars, P);
     count_launch();
-    return cudaGetLastError();
+    return launch_after(hex ? ewald_f64_kernel<true> : ewald_f64_kernel<false>, blocks, threads, s,
+                        after_list && !ts.start, parts, n_parts, idx, n_idx, vars, P);
   }
   if (nE > kMixMaxReps) return cudaErrorInvalidValue;
   EwaldMixArgs P;
@@ -1025,11 +1029,13 @@ cudaError_t launch_ewald_fp(int form, const double* parts, long long n_parts, co
   if (hex) fill_hex_root(p.momc, P.hex);
   const int threads = ewald_threads(n_idx);
   const int blocks = (int)((n_idx + threads - 1) / threads);
+  static const bool split = (set_carveout(ewald_mix_kernel<true>, kCarveoutFp32),
+                             set_carveout(ewald_mix_kernel<false>, kCarveoutFp32), true);
+  (void)split;
   TimingScope ts(kKidEwaldMix, s);
-  if (hex) ewald_mix_kernel<true><<<blocks, threads, 0, s>>>(parts, n_parts, idx, n_idx, vars, P);
-  else ewald_mix_kernel<false><<<blocks, threads, 0, s>>>(parts, n_parts, idx, n_idx, vars, P);
   count_launch();
-  return cudaGetLastError();
+  return launch_after(hex ? ewald_mix_kernel<true> : ewald_mix_kernel<false>, blocks, threads, s,
+                      after_list && !ts.start, parts, n_parts, idx, n_idx, vars, P);
 }
 
 namespace {

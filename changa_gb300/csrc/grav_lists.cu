@@ -187,6 +187,7 @@ __global__ void __launch_bounds__(kThreads, 2) list_kernel_hex(const ListArgs a)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   T* st = stage[warp];
 
+  open_to_next();
   for (;;) {
     int b = 0;
     if (lane == 0) b = (int)atomicAdd(a.queue, 1u);
@@ -2014,6 +2015,7 @@ __global__ void __launch_bounds__(kThreads, MINB) list_kernel_hex2(const ListArg
   __shared__ double red[kWarps][5][32];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
+  open_to_next();
   for (;;) {
     int b = 0;
     if (lane == 0) b = (int)atomicAdd(a.queue, 1u);
@@ -2136,52 +2138,74 @@ __global__ void __launch_bounds__(kThreads, MINB) list_kernel_hex2(const ListArg
   }
 }
 
-__global__ void pack_cells_kernel(const double* __restrict__ m, long long n, float4* __restrict__ out) {
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
-       i += (long long)gridDim.x * blockDim.x) {
-    const double* r = m + 12 * i;
-    const double x = r[3], y = r[4], z = r[5];
-    const float hx = (float)x, hy = (float)y, hz = (float)z;
-    out[4 * i + 0] = make_float4(hx, hy, hz, (float)r[2]);
-    out[4 * i + 1] = make_float4((float)(x - (double)hx), (float)(y - (double)hy),
-                                 (float)(z - (double)hz), (float)r[1]);
-    out[4 * i + 2] = make_float4((float)r[6], (float)r[7], (float)r[8], (float)r[9]);
-    out[4 * i + 3] = make_float4((float)r[10], (float)r[11], (float)(0.5 * (r[6] + r[9] + r[11])), 0.f);
-  }
+__device__ __forceinline__ void pack_cell(const double* r, float4* o) {
+  const double x = r[3], y = r[4], z = r[5];
+  const float hx = (float)x, hy = (float)y, hz = (float)z;
+  o[0] = make_float4(hx, hy, hz, (float)r[2]);
+  o[1] = make_float4((float)(x - (double)hx), (float)(y - (double)hy), (float)(z - (double)hz),
+                     (float)r[1]);
+  o[2] = make_float4((float)r[6], (float)r[7], (float)r[8], (float)r[9]);
+  o[3] = make_float4((float)r[10], (float)r[11], (float)(0.5 * (r[6] + r[9] + r[11])), 0.f);
 }
 
-__global__ void pack_parts_kernel(const double* __restrict__ p, long long n, float4* __restrict__ out) {
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
-       i += (long long)gridDim.x * blockDim.x) {
-    const double* r = p + 5 * i;
-    const double x = r[2], y = r[3], z = r[4];
-    const float hx = (float)x, hy = (float)y, hz = (float)z;
-    out[2 * i + 0] = make_float4(hx, hy, hz, (float)r[0]);
-    out[2 * i + 1] = make_float4((float)(x - (double)hx), (float)(y - (double)hy),
-                                 (float)(z - (double)hz), (float)r[1]);
-  }
+__device__ __forceinline__ void pack_part(const double* r, float4* o) {
+  const double x = r[2], y = r[3], z = r[4];
+  const float hx = (float)x, hy = (float)y, hz = (float)z;
+  o[0] = make_float4(hx, hy, hz, (float)r[0]);
+  o[1] = make_float4((float)(x - (double)hx), (float)(y - (double)hy), (float)(z - (double)hz),
+                     (float)r[1]);
 }
 
-/* Packed hexadecapole cells (FP32-mixed form) from 27-double moments. */
-__global__ void pack_cells_hex_kernel(const double* __restrict__ m, long long n,
-                                      float4* __restrict__ out) {
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
-       i += (long long)gridDim.x * blockDim.x) {
-    const double* r = m + 27 * i;
-    const double x = r[3], y = r[4], z = r[5];
-    const float hx = (float)x, hy = (float)y, hz = (float)z;
-    float4* o = out + kCellHexPackF4 * i;
-    o[0] = make_float4(hx, hy, hz, (float)r[2]);
-    o[1] = make_float4((float)(x - (double)hx), (float)(y - (double)hy), (float)(z - (double)hz),
-                       (float)r[1]);
-    float w[24];
-    w[0] = (float)r[0];
+/* A packed hexadecapole cell (FP32-mixed form) from 27 doubles. */
+__device__ __forceinline__ void pack_cell_hex(const double* r, float4* o) {
+  const double x = r[3], y = r[4], z = r[5];
+  const float hx = (float)x, hy = (float)y, hz = (float)z;
+  o[0] = make_float4(hx, hy, hz, (float)r[2]);
+  o[1] = make_float4((float)(x - (double)hx), (float)(y - (double)hy), (float)(z - (double)hz),
+                     (float)r[1]);
+  float w[24];
+  w[0] = (float)r[0];
 #pragma unroll
-    for (int k = 0; k < 21; ++k) w[1 + k] = (float)r[6 + k];
-    w[22] = 0.f;
-    w[23] = 0.f;
+  for (int k = 0; k < 21; ++k) w[1 + k] = (float)r[6 + k];
+  w[22] = 0.f;
+  w[23] = 0.f;
 #pragma unroll
-    for (int k = 0; k < 6; ++k) o[2 + k] = make_float4(w[4 * k], w[4 * k + 1], w[4 * k + 2], w[4 * k + 3]);
+  for (int k = 0; k < 6; ++k) o[2 + k] = make_float4(w[4 * k], w[4 * k + 1], w[4 * k + 2], w[4 * k + 3]);
+}
+
+/* Packs n_cells cells and n_parts particles and zeroes the list kernels'
+ * work counters, in one launch.  Bound by memory: tiles of kPackTile rows are
+ * copied to shared memory in order (rows of 40, 96 or 216 bytes read by a
+ * thread each take as many passes over their lines as they have words) and
+ * packed from there.  2^20 particles and the cells of their tree, cold caches:
+ * 60 us in two launches of a thread per row, 38 us so. */
+constexpr int kPackTile = 128;
+template <bool HEX>
+__global__ void __launch_bounds__(kPackTile) pack_step_kernel(
+    const double* __restrict__ cells, long long n_cells, float4* __restrict__ out_cells,
+    const double* __restrict__ parts, long long n_parts, float4* __restrict__ out_parts,
+    unsigned int* __restrict__ queue) {
+  constexpr int CW = HEX ? 27 : 12, CO = HEX ? kCellHexPackF4 : kCellPackF4;
+  __shared__ double rows[kPackTile * CW];
+  const int t = threadIdx.x;
+  if (queue && blockIdx.x == 0)
+    for (int k = t; k < kQueueInts; k += kPackTile) queue[k] = 0u;
+  const long long tc = (n_cells + kPackTile - 1) / kPackTile;
+  const long long tiles = tc + (n_parts + kPackTile - 1) / kPackTile;
+  for (long long tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+    const bool cell = tile < tc;
+    const long long i0 = (cell ? tile : tile - tc) * kPackTile;
+    const int n = (int)min((long long)kPackTile, (cell ? n_cells : n_parts) - i0);
+    const int w = cell ? CW : 5;
+    const double* in = (cell ? cells : parts) + w * i0;
+    for (int k = t; k < n * w; k += kPackTile) rows[k] = __ldg(in + k);
+    __syncthreads();
+    if (t < n) {
+      if (!cell) pack_part(rows + 5 * t, out_parts + kPartPackF4 * (i0 + t));
+      else if (HEX) pack_cell_hex(rows + 27 * t, out_cells + CO * (i0 + t));
+      else pack_cell(rows + 12 * t, out_cells + CO * (i0 + t));
+    }
+    __syncthreads();
   }
 }
 
@@ -2209,6 +2233,7 @@ template <typename K>
 int blocks_per_sm(K kernel, std::atomic<int>* cache) {
   int nb = cache->load(std::memory_order_relaxed);
   if (!nb) {
+    set_carveout(kernel, kCarveoutFp32);
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kernel, kThreads, 0) != cudaSuccess ||
         nb < 1)
       nb = 1;
@@ -2223,6 +2248,8 @@ cudaError_t launch_block(K kernel, int threads, std::atomic<int>* cache, int kid
   if (a.n_buckets <= 0) return cudaSuccess;
   int nb = cache->load(std::memory_order_relaxed);
   if (!nb) {
+    set_carveout(kernel, kid == kKidListF64Cell || kid == kKidListF64Part ? kCarveoutFp64
+                                                                          : kCarveoutFp32);
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kernel, threads, 0) != cudaSuccess ||
         nb < 1)
       nb = 1;
@@ -2231,22 +2258,21 @@ cudaError_t launch_block(K kernel, int threads, std::atomic<int>* cache, int kid
   const long long cap = (long long)sm_count() * nb;
   const int grid = (int)(a.n_buckets < cap ? a.n_buckets : cap);
   TimingScope ts(kid, s);
-  kernel<<<grid, threads, 0, s>>>(a);
   count_launch();
-  return cudaGetLastError();
+  return launch_after(kernel, grid, threads, s, a.after_list && !ts.start, a);
 }
 
+/* waits: the kernel has wait_for_last, so a.after_list may overlap it */
 template <typename K>
 cudaError_t launch_kernel(K kernel, std::atomic<int>* occ_cache, int kid, const ListArgs& a,
-                          cudaStream_t s) {
+                          cudaStream_t s, bool waits = false) {
   if (a.n_buckets <= 0) return cudaSuccess;
   long long want = ((long long)a.n_buckets + kWarps - 1) / kWarps;
   long long cap = (long long)sm_count() * blocks_per_sm(kernel, occ_cache);
   int grid = (int)(want < cap ? want : cap);
   TimingScope ts(kid, s);
-  kernel<<<grid, kThreads, 0, s>>>(a);
   count_launch();
-  return cudaGetLastError();
+  return launch_after(kernel, grid, kThreads, s, waits && a.after_list && !ts.start, a);
 }
 
 /* current variant per list kernel id (FP32 forms); several host threads
@@ -2324,19 +2350,25 @@ cudaError_t launch_variant(const ListArgs& a, cudaStream_t s) {
     return launch_kernel(list_kernel_tp2<FORM, CELL, var.minb>, &occ, list_kernel_id(FORM, CELL),
                          a, s);
   } else if constexpr (var.tp == 7) {
-    /* a CTA per bucket while the buckets are fewer than the warps that
+    /* A CTA per bucket while the buckets are fewer than the warps that
      * list_kernel_far keeps resident (24 per SM).  On both sides of that
      * line, cells / particles in us, CTA against warp: 2230 buckets 30 / 37
      * against 32 / 37, 4300 buckets 83 / 169 against 85 / 173, 6030 buckets
-     * 91 / 91 against 90 / 77. */
-    return (long long)a.n_buckets <= 24ll * sm_count() ? launch_variant<FORM, CELL, kBlockVariant>(a, s)
+     * 91 / 91 against 90 / 77.  Buckets that hold fewer than 8 targets in the
+     * mean already spread a list over four or more lane groups of a warp, so
+     * there the CTA gains only where it fills idle SMs (4 per SM); us a step,
+     * CTA against warp: 530 buckets of 5.7 targets 43 / 51, 1060 of 5.7
+     * 57 / 54, 2100 of 5.7 73 / 65, 1400 of 8.5 69 / 79 (overlapped, as they
+     * run now: 25 / 28, 40 / 33, 57 / 51, 51 / 51). */
+    const bool tiny = a.n_tgt < 8ll * a.n_buckets;
+    return (long long)a.n_buckets <= (tiny ? 4ll : 24ll) * sm_count() ? launch_variant<FORM, CELL, kBlockVariant>(a, s)
                                                        : launch_variant<FORM, CELL, kFarVariant>(a, s);
   } else if constexpr (var.tp == 5)
     return launch_block(list_kernel_block<FORM, CELL, var.group, var.minb>, var.group, &occ,
                         list_kernel_id(FORM, CELL), a, s);
   else if constexpr (var.tp == 6)
     return launch_kernel(list_kernel_far<FORM, CELL, var.minb>, &occ, list_kernel_id(FORM, CELL), a,
-                         s);
+                         s, true);
   else if constexpr (var.tp == 4)
     return launch_kernel(list_kernel_rb<FORM, CELL, var.minb, var.group>, &occ,
                          list_kernel_id(FORM, CELL), a, s);
@@ -2433,12 +2465,20 @@ static int grid_for(long long n, int threads) {
   return g < 1 ? 1 : (int)g;
 }
 
-cudaError_t launch_pack_cells(const double* moments, long long n, float4* out, cudaStream_t s) {
-  if (n <= 0) return cudaSuccess;
+cudaError_t launch_pack_step(bool hex, const double* moments, long long n_moments, float4* cells,
+                             const double* parts, long long n_parts, float4* packed,
+                             unsigned int* queue, cudaStream_t s) {
+  if (n_moments <= 0 && n_parts <= 0 && !queue) return cudaSuccess;
+  const int grid = grid_for(std::max(0ll, n_moments) + std::max(0ll, n_parts) + kPackTile, kPackTile);
   TimingScope ts(kKidPack, s);
-  pack_cells_kernel<<<grid_for(n, 256), 256, 0, s>>>(moments, n, out);
+  if (hex) pack_step_kernel<true><<<grid, kPackTile, 0, s>>>(moments, n_moments, cells, parts, n_parts, packed, queue);
+  else pack_step_kernel<false><<<grid, kPackTile, 0, s>>>(moments, n_moments, cells, parts, n_parts, packed, queue);
   count_launch();
   return cudaGetLastError();
+}
+
+cudaError_t launch_pack_cells(const double* moments, long long n, float4* out, cudaStream_t s) {
+  return launch_pack_step(false, moments, n, out, nullptr, 0, nullptr, nullptr, s);
 }
 
 /* hexadecapole FP32-mixed cell kernel: 0 synchronous staging
@@ -2476,14 +2516,6 @@ int set_hex_variant(int v) {
 
 int get_hex_variant() { return g_hex_variant.load(); }
 
-cudaError_t launch_pack_cells_hex(const double* moments, long long n, float4* out, cudaStream_t s) {
-  if (n <= 0) return cudaSuccess;
-  TimingScope ts(kKidPack, s);
-  pack_cells_hex_kernel<<<grid_for(n, 256), 256, 0, s>>>(moments, n, out);
-  count_launch();
-  return cudaGetLastError();
-}
-
 cudaError_t launch_cells_as_parts(const double* moments, int stride, long long n, double* out,
                                   cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
@@ -2494,11 +2526,7 @@ cudaError_t launch_cells_as_parts(const double* moments, int stride, long long n
 }
 
 cudaError_t launch_pack_parts(const double* parts, long long n, float4* out, cudaStream_t s) {
-  if (n <= 0) return cudaSuccess;
-  TimingScope ts(kKidPack, s);
-  pack_parts_kernel<<<grid_for(n, 256), 256, 0, s>>>(parts, n, out);
-  count_launch();
-  return cudaGetLastError();
+  return launch_pack_step(false, nullptr, 0, nullptr, parts, n, out, nullptr, s);
 }
 
 }  // namespace chg

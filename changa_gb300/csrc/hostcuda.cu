@@ -954,10 +954,12 @@ static cudaError_t launch_expand_runs(const ILPart* runs, long long n_runs, cons
   return cudaGetLastError();
 }
 
-/* One list evaluation over device-resident inputs (FP64 or mixed form). */
+/* One list evaluation over device-resident inputs (FP64 or mixed form).
+ * queue_zero: the counter is zero already; after_list: see ListArgs. */
 static int run_fp(int form, bool cell, const void* src, long long n_src, const void* tgt,
                   long long n_tgt, const ChangaListRequest* req, double fperiod, double* vars,
-                  cudaStream_t s, unsigned int* queue) {
+                  cudaStream_t s, unsigned int* queue, bool queue_zero = false,
+                  bool after_list = false) {
   ListArgs a;
   a.src = src;
   a.n_src = n_src;
@@ -973,7 +975,8 @@ static int run_fp(int form, bool cell, const void* src, long long n_src, const v
   a.fperiod_f = (float)fperiod;
   a.fperiod_d = fperiod;
   a.queue = queue;
-  CHG_CUDA(cudaMemsetAsync(queue, 0, sizeof(unsigned int), s));
+  a.after_list = after_list;
+  if (!queue_zero) CHG_CUDA(cudaMemsetAsync(queue, 0, sizeof(unsigned int), s));
   CHG_CUDA(launch_list(form, cell, a, s));
   return 0;
 }
@@ -1050,23 +1053,33 @@ int changa_gravity_step(int form, const double* moments, long long n_moments, co
     pb = align256((size_t)n_parts * kPartPackF4 * sizeof(float4));
   }
   char* block = nullptr;
-  CHG_CUDA(cudaMallocAsync((void**)&block, cb + pb + 512, s));
+  CHG_CUDA(cudaMallocAsync((void**)&block, cb + pb + kQueueInts * sizeof(unsigned int), s));
   unsigned int* q = (unsigned int*)(block + cb + pb);
   const void* ksrc = moments;
   const void* kpart = parts;
   if (f == kMix) {
-    CHG_CUDA(launch_pack_cells(moments, n_moments, (float4*)block, s));
-    CHG_CUDA(launch_pack_parts(parts, n_parts, (float4*)(block + cb), s));
+    CHG_CUDA(launch_pack_step(false, moments, n_moments, (float4*)block, parts, n_parts,
+                              (float4*)(block + cb), q, s));
     ksrc = block;
     kpart = block + cb;
+  } else {
+    CHG_CUDA(cudaMemsetAsync(q, 0, kQueueInts * sizeof(unsigned int), s));
   }
+  /* The lists and the Ewald term meet only in vars, so each launch may start
+   * while the one before it drains (open_to_next); the small evaluations run
+   * side by side. */
   int rc = 0;
-  if (cells && cells->n_buckets > 0)
-    rc = run_fp(f, true, ksrc, n_moments, kpart, n_parts, cells, fperiod, vars, s, q);
-  if (!rc && plist && plist->n_buckets > 0)
-    rc = run_fp(f, false, kpart, n_parts, kpart, n_parts, plist, fperiod, vars, s, q + 64);
+  bool list = false;
+  if (cells && cells->n_buckets > 0) {
+    rc = run_fp(f, true, ksrc, n_moments, kpart, n_parts, cells, fperiod, vars, s, q, true);
+    list = true;
+  }
+  if (!rc && plist && plist->n_buckets > 0) {
+    rc = run_fp(f, false, kpart, n_parts, kpart, n_parts, plist, fperiod, vars, s, q + 64, true, list);
+    list = true;
+  }
   if (!rc && ewald) {
-    cudaError_t e = launch_ewald_fp(f, parts, n_parts, nullptr, n_parts, *ewald, vars, s);
+    cudaError_t e = launch_ewald_fp(f, parts, n_parts, nullptr, n_parts, *ewald, vars, s, false, list);
     if (e != cudaSuccess) rc = record_error((int)e, "gravity_step: ewald", __FILE__, __LINE__);
   }
   cudaError_t e = cudaFreeAsync(block, s);
@@ -1098,7 +1111,7 @@ int changa_gravity_step_hexa(int form, const double* moments, long long n_moment
     sb = align256((size_t)n_moments * kPartPackF4 * sizeof(float4));
   }
   char* block = nullptr;
-  CHG_CUDA(cudaMallocAsync((void**)&block, qb + cb + pb + sb + 1024, s));
+  CHG_CUDA(cudaMallocAsync((void**)&block, qb + cb + pb + sb + kQueueInts * sizeof(unsigned int), s));
   double* pseudo = (double*)block;
   unsigned int* q = (unsigned int*)(block + qb + cb + pb + sb);
   const void* kcell = moments;
@@ -1114,8 +1127,8 @@ int changa_gravity_step_hexa(int form, const double* moments, long long n_moment
       float4* pc = (float4*)(block + qb);
       float4* pp = (float4*)(block + qb + cb);
       float4* ps = (float4*)(block + qb + cb + pb);
-      if ((e = launch_pack_cells_hex(moments, n_moments, pc, s)) != cudaSuccess ||
-          (e = launch_pack_parts(parts, n_parts, pp, s)) != cudaSuccess)
+      if ((e = launch_pack_step(true, moments, n_moments, pc, parts, n_parts, pp, q, s)) !=
+          cudaSuccess)
         break;
       if (softcells && softcells->n_buckets > 0 &&
           (e = launch_pack_parts(pseudo, n_moments, ps, s)) != cudaSuccess)
@@ -1123,7 +1136,10 @@ int changa_gravity_step_hexa(int form, const double* moments, long long n_moment
       kcell = pc;
       kpart = pp;
       kpseudo = ps;
+    } else if ((e = cudaMemsetAsync(q, 0, kQueueInts * sizeof(unsigned int), s)) != cudaSuccess) {
+      break;
     }
+    bool list = false;
     if (cells && cells->n_buckets > 0) {
       ListArgs a;
       a.src = kcell;
@@ -1140,17 +1156,21 @@ int changa_gravity_step_hexa(int form, const double* moments, long long n_moment
       a.fperiod_f = (float)fperiod;
       a.fperiod_d = fperiod;
       a.queue = q;
-      if ((e = cudaMemsetAsync(q, 0, sizeof(unsigned int), s)) != cudaSuccess ||
-          (e = launch_list_hex(f, a, s)) != cudaSuccess)
-        break;
+      if ((e = launch_list_hex(f, a, s)) != cudaSuccess) break;
+      list = true;
     }
-    if (plist && plist->n_buckets > 0)
-      rc = run_fp(f, false, kpart, n_parts, kpart, n_parts, plist, fperiod, vars, s, q + 64);
-    if (!rc && softcells && softcells->n_buckets > 0)
+    if (plist && plist->n_buckets > 0) {
+      rc = run_fp(f, false, kpart, n_parts, kpart, n_parts, plist, fperiod, vars, s, q + 64, true,
+                  list);
+      list = true;
+    }
+    if (!rc && softcells && softcells->n_buckets > 0) {
       rc = run_fp(f, false, kpseudo, n_moments, kpart, n_parts, softcells, fperiod, vars, s,
-                  q + 128);
+                  q + 128, true, list);
+      list = true;
+    }
     if (!rc && ewald) {
-      e = launch_ewald_fp(f, parts, n_parts, nullptr, n_parts, *ewald, vars, s, true);
+      e = launch_ewald_fp(f, parts, n_parts, nullptr, n_parts, *ewald, vars, s, true, list);
       if (e != cudaSuccess)
         rc = record_error((int)e, "gravity_step_hexa: ewald", __FILE__, __LINE__);
       e = cudaSuccess;

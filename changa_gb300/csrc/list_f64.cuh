@@ -148,6 +148,7 @@ __global__ void __launch_bounds__(kF64Threads, 2) list_kernel_f64(const ListArgs
   const double* tgt = static_cast<const double*>(a.tgt);
   double* vars = static_cast<double*>(a.vars);
 
+  open_to_next();
   if (tid == 0) snext = (int)atomicAdd(a.queue, 1u);
   __syncthreads();
   for (;;) {
@@ -308,6 +309,7 @@ __global__ void __launch_bounds__(kF64Threads, 2) list_kernel_f64(const ListArgs
       red[3][tid] = CELL ? fma(-0.5, acc.quad, acc.pot) : acc.pot;
       redmax[tid] = acc.idt2;
       __syncthreads();
+      wait_for_last();
       for (int k = tid; k < 5 * nt; k += T) {
         const int q = k / nt, tt = k - q * nt;
         double* v = vars + 5 * (tbase + t0 + tt) + q;

@@ -224,6 +224,7 @@ template <int FORM, int T>
 __device__ __forceinline__ void join_groups(const ListArgs& a, const float2 (&red)[4][T],
                                             const float (&redmax)[T], int tid, int nt, int G,
                                             long long first) {
+  wait_for_last();
   for (int k = tid; k < 5 * nt; k += T) {
     const int q = k / nt, t = k - q * nt;
     const long long to = first + t;
@@ -377,6 +378,7 @@ __global__ void __launch_bounds__(T, MINB) list_kernel_block(const ListArgs a) {
   const unsigned limit = (unsigned)min(a.n_src, 0x80000000ll);
   const float fp = a.fperiod_f;
 
+  open_to_next();
   if (tid == 0) snext = (int)atomicAdd(a.queue, 1u);
   __syncthreads();
   for (;;) {
@@ -622,6 +624,7 @@ __global__ void __launch_bounds__(256, MINB) list_kernel_far(const ListArgs a) {
   const unsigned limit = (unsigned)min(a.n_src, 0x80000000ll);
   const float fp = a.fperiod_f;
 
+  open_to_next();
   for (;;) {
     int b = 0;
     if (lane == 0) b = (int)atomicAdd(a.queue, 1u);
@@ -820,6 +823,7 @@ __global__ void __launch_bounds__(256, MINB) list_kernel_far(const ListArgs a) {
       }
       if (CELL) idt2 = -idt2;
       if (G == 1) {
+        wait_for_last();
         if (lane < nt) add_target<FORM>(a, ti, sx, -cx, sy, -cy, sz, -cz, sp, -cp, idt2);
       } else {
         __syncwarp();
@@ -829,6 +833,7 @@ __global__ void __launch_bounds__(256, MINB) list_kernel_far(const ListArgs a) {
         red_[warp][3][lane] = make_float2(sp, -cp);
         redmax_[warp][lane] = idt2;
         __syncwarp();
+        wait_for_last();
         if (lane < nt) {
           float2 s[4];
 #pragma unroll
