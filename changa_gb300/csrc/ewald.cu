@@ -382,7 +382,10 @@ __global__ void __launch_bounds__(128) ewald_f64_kernel(const double* __restrict
     if (j < 0 || j >= n_parts) j = -1;
   }
   const bool live = j >= 0;
-  if (!__any_sync(0xffffffffu, live)) return;
+  if (!__any_sync(0xffffffffu, live)) {
+    wait_for_last();
+    return;
+  }
   double dd[3] = {0.0, 0.0, 0.0};
   if (live)
     for (int c = 0; c < 3; ++c) dd[c] = parts[5 * j + 2 + c] - P.mom[3 + c];
@@ -531,8 +534,8 @@ __global__ void __launch_bounds__(128) ewald_f64_kernel(const double* __restrict
       az += e[2] * t;
     }
   }
-  if (!live) return;
   wait_for_last();
+  if (!live) return;
   double* v = vars + 5 * j;
   v[0] += ax;
   v[1] += ay;
@@ -681,7 +684,10 @@ __global__ void __launch_bounds__(kMixWarps * 32) ewald_mix_kernel(
     if (pass == 0) nhole = count;
   }
   __syncwarp();
-  if (!live) return;
+  if (!live) {
+    wait_for_last();
+    return;
+  }
 
   const float a2 = P.alpha2, twoa2 = 2.f * a2, foura4 = twoa2 * twoa2, ka = P.ka;
   const float M = P.M, Q2 = P.Q2;

@@ -327,6 +327,7 @@ __global__ void __launch_bounds__(kF64Threads, 2) list_kernel_f64(const ListArgs
     }
     __syncthreads();  // snext is written (a skipped bucket has no other barrier)
   }
+  wait_for_last();
 }
 
 }  // namespace

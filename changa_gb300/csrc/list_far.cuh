@@ -599,6 +599,7 @@ __global__ void __launch_bounds__(T, MINB) list_kernel_block(const ListArgs a) {
     }
     __syncthreads();  // snext is written (a skipped bucket has no other barrier)
   }
+  wait_for_last();
 }
 
 /* One warp per bucket, from the work queue: lanes own targets, in G = 32 / nt
@@ -850,6 +851,7 @@ __global__ void __launch_bounds__(256, MINB) list_kernel_far(const ListArgs a) {
       }
     }
   }
+  wait_for_last();
 }
 
 }  // namespace
