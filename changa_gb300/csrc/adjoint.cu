@@ -614,7 +614,7 @@ extern "C" int changa_gravity_vjp_mixed(const double* moments, long long n_momen
   float* acc_part = (float*)(block + cb + pb + lb + fb + ab);
   unsigned int* q = (unsigned int*)(block + cb + pb + lb + fb + ab + qb);
   CHG_CUDA(cudaMemsetAsync(acc_cell, 0, ab + qb + 512, s));
-  CHG_CUDA(launch_pack_step(false, moments, n_moments, pc, parts, n_parts, pp, nullptr, s));
+  CHG_CUDA(launch_pack_step(kPackQuad, moments, n_moments, pc, parts, n_parts, pp, nullptr, s));
   {
     TimingScope ts(kKidPack, s);
     pack_lambda_kernel<<<grid_of(n_parts, 256), 256, 0, s>>>(lam, n_parts, pl);

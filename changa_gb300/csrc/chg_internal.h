@@ -65,16 +65,19 @@ unsigned long long tma_launches();
 cudaError_t read_device_status(unsigned* bits);
 cudaError_t launch_pack_cells(const double* moments, long long n, float4* out, cudaStream_t s);
 cudaError_t launch_pack_parts(const double* parts, long long n, float4* out, cudaStream_t s);
-/* Both (cells of 12 doubles, or of 27 for the hexadecapole form) and kQueueInts
- * zero words at queue, in one launch. */
+/* Both and kQueueInts zero words at queue, in one launch.  Cells: of 12 doubles,
+ * or of 27 for the hexadecapole form, packed as list_kernel_hex (variant 0)
+ * or as list_kernel_hex2 reads them. */
 constexpr int kQueueInts = 192;
-cudaError_t launch_pack_step(bool hex, const double* moments, long long n_moments, float4* cells,
+enum PackCells { kPackQuad = 0, kPackHex = 1, kPackHexPaired = 2 };
+cudaError_t launch_pack_step(PackCells kind, const double* moments, long long n_moments, float4* cells,
                              const double* parts, long long n_parts, float4* packed,
                              unsigned int* queue, cudaStream_t s);
 cudaError_t launch_zero_vars_f32(VariablePartData* v, long long n, cudaStream_t s);
 /* hexadecapole build: cell lists over 27-double (kF64) or packed (kMix)
  * moments; the pack; cells as point-mass particles {M, soft, cm} */
-cudaError_t launch_list_hex(int form, const ListArgs& a, cudaStream_t s);
+/* variant: get_hex_variant() as the cells were packed by launch_pack_step */
+cudaError_t launch_list_hex(int form, const ListArgs& a, int variant, cudaStream_t s);
 cudaError_t launch_cells_as_parts(const double* moments, int stride, long long n, double* out,
                                   cudaStream_t s);
 
@@ -127,7 +130,9 @@ struct TimingScope {
  * blocks has (open_to_next), the successor's blocks take the places that it
  * frees as it drains, and wait for its end (wait_for_last) before they touch
  * vars.  Without the attribute of launch_after both are no-operations.  A
- * kernel launched so has wait_for_last in every path that adds to vars.  us a
+ * kernel launched so has wait_for_last in every path that adds to vars and at
+ * its end, so that it never ends before the one it overlaps, whose end the
+ * launches after it rely on.  us a
  * step, one after another / so: 32768 Plummer particles 125 / 107, 6000 of
  * them 52 / 40, 1200 37 / 25; 12000 periodic with Ewald 87 / 51; 2^20 with
  * Ewald 2490 / 2350. */

@@ -1793,27 +1793,37 @@ __global__ void __launch_bounds__(kThreads, MINB) list_kernel_tma(const ListArgs
 
 struct RawHex {
   float4 w[kCellHexPackF4];
+  float4 h, l;
   int code;
 };
 
-/* Raw record of entry e: kMix, the packed cell (8 float4); kF32 (the
- * drop-in of the hexadecapole build), the 108-byte CudaMultipoleMoments
- * (27 floats, 4-byte aligned) rearranged into the same words with a zero
- * low part. */
+/* Records of the block's entries, e this lane's.  kF32 (the drop-in of the
+ * hexadecapole build): the lane's own 108-byte CudaMultipoleMoments (27
+ * floats, 4-byte aligned), as {cm, M} {0, soft} {radius, moments}.  kMix, the
+ * packed cells (kPackHexPaired, 128 bytes): the lane's own two first words as
+ * h and l, and the other six row by row, eight lanes to a row, so that a load
+ * touches four lines and not 32: w[i] is word lane & 7 of entry 4 i + lane / 8.
+ * Entries past the end repeat the last one (stage_hex_rows sets them far). */
 template <int FORM>
 __device__ __forceinline__ void gather_hex(const ListArgs& a, int e, int e_end, RawHex& r) {
   long long idx = 0;
   r.code = 0x49;  // replica (0, 0, 0)
-  if (e < e_end) {
-    const int2 ent = __ldg(a.list + e);
+  if (FORM == kMix || e < e_end) {
+    const int2 ent = __ldg(a.list + min(e, e_end - 1));
     idx = ent.x;
     if ((unsigned long long)idx >= (unsigned long long)a.n_src) idx = 0;  // memory safety
     r.code = (ent.y >> 22) & 0x1ff;
   }
   if constexpr (FORM == kMix) {
-    const float4* p = static_cast<const float4*>(a.src) + kCellHexPackF4 * idx;
+    const int j = threadIdx.x & 7, q = (threadIdx.x >> 3) & 3;
+    const float4* p = static_cast<const float4*>(a.src);
+    r.h = __ldg(p + kCellHexPackF4 * idx);
+    r.l = __ldg(p + kCellHexPackF4 * idx + 1);
 #pragma unroll
-    for (int k = 0; k < kCellHexPackF4; ++k) r.w[k] = __ldg(p + k);
+    for (int i = 0; i < 8; ++i) {
+      const long long row = __shfl_sync(kFull, (int)idx, 4 * i + q);
+      if (j >= 2) r.w[i] = __ldg(p + kCellHexPackF4 * row + j);
+    }
   } else {
 #ifdef HEXADECAPOLE
     /* {radius, soft, totalMass, cm.xyz, then the 21 moments} */
@@ -1836,10 +1846,9 @@ __device__ __forceinline__ void gather_hex(const ListArgs& a, int e, int e_end, 
   }
 }
 
-/* One record into half h of a staged pair (kHexFields fields): the source
- * position with the replica offset (kMix: relative to the bucket's centre,
- * as stage_entry forms it; kF32: offset + cm as the reference forms it,
- * HostCUDA.cu:1094-1099), M, then the 21 reduced moments each scaled by its
+/* One record of the drop-in (kF32) into half h of a staged pair (kHexFields
+ * fields): the source position as offset + cm, as the reference forms it
+ * (HostCUDA.cu:1094-1099), M, then the 21 reduced moments each scaled by its
  * order's gamma factor at unit distance (second order 3 R^2, third 15 R^3,
  * fourth 105 R^4, R the radius), so that the pair evaluation multiplies
  * them by 1/r^3, 1/r^4, 1/r^5 only, and four sums of scaled moments the
@@ -1847,23 +1856,47 @@ __device__ __forceinline__ void gather_hex(const ListArgs& a, int e, int e_end, 
  * (they add exact zeros). */
 constexpr int kHexFields = 30;  // 15 float4 words per staged pair
 
-template <int FORM>
-__device__ __forceinline__ void stage_hex(const ListArgs& a, const RawHex& r, bool valid,
-                                          float3 chi, float3 clo, float* pb, int h) {
+/* The block's records (gather_hex<kMix>) into its staged pairs; ne of the 32
+ * are entries.  The packed words hold the fields ready but for the position:
+ * {hi.xyz, M} {lo.xyz, Q13 + Q14} and the fields 4 .. 27.  The two lanes that
+ * hold one word of a pair's two entries exchange halves, and each stores one
+ * float4 of the pair. */
+__device__ __forceinline__ void stage_hex_rows(const ListArgs& a, const RawHex& r, int ne, float3 chi,
+                                               float3 clo, float4* st) {
+  constexpr int PW = kHexFields / 2;
   const float fp = a.fperiod_f;
-  const float4 hi = r.w[0], lo = r.w[1];
-  const float ox = (float)((r.code & 7) - 3) * fp, oy = (float)(((r.code >> 3) & 7) - 3) * fp,
-              oz = (float)(((r.code >> 6) & 7) - 3) * fp;
-  float f[kHexFields];
-  if constexpr (FORM == kMix) {
-    f[0] = ((hi.x - chi.x) + ox) + (lo.x - clo.x);
-    f[1] = ((hi.y - chi.y) + oy) + (lo.y - clo.y);
-    f[2] = ((hi.z - chi.z) + oz) + (lo.z - clo.z);
-  } else {
-    f[0] = ox + hi.x;
-    f[1] = oy + hi.y;
-    f[2] = oz + hi.z;
+  const int lane = threadIdx.x & 31, j = lane & 7;
+  const bool odd = lane & 8;
+  {
+    const float ox = (float)((r.code & 7) - 3) * fp, oy = (float)(((r.code >> 3) & 7) - 3) * fp,
+                oz = (float)(((r.code >> 6) & 7) - 3) * fp;
+    const bool valid = lane < ne;
+    float* pb = reinterpret_cast<float*>(st + (lane >> 1) * PW);
+    const int h = lane & 1;
+    pb[pair_slot(0, h)] = valid ? ((r.h.x - chi.x) + ox) + (r.l.x - clo.x) : 1e30f;
+    pb[pair_slot(1, h)] = valid ? ((r.h.y - chi.y) + oy) + (r.l.y - clo.y) : 1e30f;
+    pb[pair_slot(2, h)] = valid ? ((r.h.z - chi.z) + oz) + (r.l.z - clo.z) : 1e30f;
+    pb[pair_slot(3, h)] = valid ? r.h.w : 0.f;
+    pb[pair_slot(28, h)] = r.l.w;
   }
+  float4* out = st + (lane >> 4) * PW + 2 * j - 2 + (odd ? 1 : 0);
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const float4 v = r.w[i];
+    const float s0 = __shfl_xor_sync(kFull, odd ? v.x : v.z, 8);
+    const float s1 = __shfl_xor_sync(kFull, odd ? v.y : v.w, 8);
+    if (j >= 2) out[2 * i * PW] = odd ? make_float4(s0, v.z, s1, v.w) : make_float4(v.x, s0, v.y, s1);
+  }
+}
+
+__device__ __forceinline__ void stage_hex(const ListArgs& a, const RawHex& r, bool valid, float* pb,
+                                          int h) {
+  const float fp = a.fperiod_f;
+  const float4 hi = r.w[0];
+  float f[kHexFields];
+  f[0] = (float)((r.code & 7) - 3) * fp + hi.x;
+  f[1] = (float)(((r.code >> 3) & 7) - 3) * fp + hi.y;
+  f[2] = (float)(((r.code >> 6) & 7) - 3) * fp + hi.z;
   f[3] = hi.w;
   /* raw words 2..7: the radius, then the 21 moments (two zeros after) */
   float q[24];
@@ -2007,6 +2040,13 @@ __device__ __forceinline__ void hex_pair(const float4* __restrict__ w, f2 tx2, f
   idt2 = fmax3(idt2, e0, e1);
 }
 
+/* A warp per bucket, G = 32 / targets lane groups over the staged pairs.  Bound
+ * by the FP32 pipe and by shared memory alike (63 % of the FMA cycles; 15 loads
+ * of two wavefronts a pair step are most of the LSU's 79 %): 200000 Plummer
+ * particles in buckets of 12, 842 us with each lane gathering its own 128-byte
+ * row (32 lines a load, LSU 89 % busy), scaling its moments at every staging
+ * and 16 pairs a block whatever G; 725 us with rows gathered by eight lanes,
+ * moments scaled when packed and blocks of as many pairs as G divides. */
 template <int FORM, int MINB>
 __global__ void __launch_bounds__(kThreads, MINB) list_kernel_hex2(const ListArgs a) {
   static_assert(FORM == kMix || FORM == kF32, "FP32 arithmetic forms only");
@@ -2061,14 +2101,20 @@ __global__ void __launch_bounds__(kThreads, MINB) list_kernel_hex2(const ListArg
 
       float sx = 0.f, sy = 0.f, sz = 0.f, sp = 0.f, idt2 = 0.f;
       float cx = 0.f, cy = 0.f, cz = 0.f, cp = 0.f;
+      /* a block of as many pairs as give every group the same number (32
+       * entries where the groups outnumber the pairs) */
+      const int block = G < 16 ? 2 * G * (16 / G) : 32;
       RawHex raw;
       gather_hex<FORM>(a, e_begin + lane, e_end, raw);
-      for (int e0 = e_begin; e0 < e_end; e0 += 32) {
-        const int ne = min(32, e_end - e0);
-        stage_hex<FORM>(a, raw, lane < ne, chi, clo,
-                        reinterpret_cast<float*>(stage[warp] + (lane >> 1) * PW), lane & 1);
+      for (int e0 = e_begin; e0 < e_end; e0 += block) {
+        const int ne = min(block, e_end - e0);
+        if constexpr (FORM == kMix)
+          stage_hex_rows(a, raw, ne, chi, clo, stage[warp]);
+        else
+          stage_hex(a, raw, lane < ne, reinterpret_cast<float*>(stage[warp] + (lane >> 1) * PW),
+                    lane & 1);
         __syncwarp();
-        if (e0 + 32 < e_end) gather_hex<FORM>(a, e0 + 32 + lane, e_end, raw);
+        if (e0 + block < e_end) gather_hex<FORM>(a, e0 + block + lane, e_end, raw);
         f2 ax2 = 0ull, ay2 = 0ull, az2 = 0ull, pot2 = 0ull;  // +0.0f in both halves
         const float4* st = stage[warp];
         if (G == 1) {
@@ -2076,7 +2122,7 @@ __global__ void __launch_bounds__(kThreads, MINB) list_kernel_hex2(const ListArg
           for (int q = 0; q < 16; ++q)
             hex_pair(st + q * PW, tx2, ty2, tz2, tm2, pot2, ax2, ay2, az2, idt2);
         } else if (active) {
-          for (int q = g; q < 16; q += G)
+          for (int q = g; 2 * q < ne; q += G)
             hex_pair(st + q * PW, tx2, ty2, tz2, tm2, pot2, ax2, ay2, az2, idt2);
         }
         __syncwarp();  // the stage is rewritten by the next block
@@ -2156,7 +2202,10 @@ __device__ __forceinline__ void pack_part(const double* r, float4* o) {
                      (float)r[1]);
 }
 
-/* A packed hexadecapole cell (FP32-mixed form) from 27 doubles. */
+/* A packed hexadecapole cell (FP32-mixed form) from 27 doubles; PAIRED: the
+ * moments scaled by their order's gamma factor and the four sums, in the
+ * order of list_kernel_hex2's fields (stage_hex). */
+template <bool PAIRED>
 __device__ __forceinline__ void pack_cell_hex(const double* r, float4* o) {
   const double x = r[3], y = r[4], z = r[5];
   const float hx = (float)x, hy = (float)y, hz = (float)z;
@@ -2164,11 +2213,22 @@ __device__ __forceinline__ void pack_cell_hex(const double* r, float4* o) {
   o[1] = make_float4((float)(x - (double)hx), (float)(y - (double)hy), (float)(z - (double)hz),
                      (float)r[1]);
   float w[24];
-  w[0] = (float)r[0];
+  if (PAIRED) {
+    const float R = (float)r[0], R2 = R * R;
+    const float s2 = 3.f * R2, s3 = 5.f * s2 * R, s4 = 7.f * s3 * R;
 #pragma unroll
-  for (int k = 0; k < 21; ++k) w[1 + k] = (float)r[6 + k];
-  w[22] = 0.f;
-  w[23] = 0.f;
+    for (int k = 0; k < 21; ++k) w[k] = (float)r[6 + k] * (k < 5 ? s2 : (k < 12 ? s3 : s4));
+    w[21] = -(w[0] + w[3]);
+    w[22] = w[5] + w[6];
+    w[23] = w[7] + w[8];
+    o[1].w = w[13] + w[14];
+  } else {
+    w[0] = (float)r[0];
+#pragma unroll
+    for (int k = 0; k < 21; ++k) w[1 + k] = (float)r[6 + k];
+    w[22] = 0.f;
+    w[23] = 0.f;
+  }
 #pragma unroll
   for (int k = 0; k < 6; ++k) o[2 + k] = make_float4(w[4 * k], w[4 * k + 1], w[4 * k + 2], w[4 * k + 3]);
 }
@@ -2180,11 +2240,12 @@ __device__ __forceinline__ void pack_cell_hex(const double* r, float4* o) {
  * packed from there.  2^20 particles and the cells of their tree, cold caches:
  * 60 us in two launches of a thread per row, 38 us so. */
 constexpr int kPackTile = 128;
-template <bool HEX>
+template <int KIND>
 __global__ void __launch_bounds__(kPackTile) pack_step_kernel(
     const double* __restrict__ cells, long long n_cells, float4* __restrict__ out_cells,
     const double* __restrict__ parts, long long n_parts, float4* __restrict__ out_parts,
     unsigned int* __restrict__ queue) {
+  constexpr bool HEX = KIND != kPackQuad;
   constexpr int CW = HEX ? 27 : 12, CO = HEX ? kCellHexPackF4 : kCellPackF4;
   __shared__ double rows[kPackTile * CW];
   const int t = threadIdx.x;
@@ -2202,7 +2263,7 @@ __global__ void __launch_bounds__(kPackTile) pack_step_kernel(
     __syncthreads();
     if (t < n) {
       if (!cell) pack_part(rows + 5 * t, out_parts + kPartPackF4 * (i0 + t));
-      else if (HEX) pack_cell_hex(rows + 27 * t, out_cells + CO * (i0 + t));
+      else if (HEX) pack_cell_hex<KIND == kPackHexPaired>(rows + 27 * t, out_cells + CO * (i0 + t));
       else pack_cell(rows + 12 * t, out_cells + CO * (i0 + t));
     }
     __syncthreads();
@@ -2465,20 +2526,22 @@ static int grid_for(long long n, int threads) {
   return g < 1 ? 1 : (int)g;
 }
 
-cudaError_t launch_pack_step(bool hex, const double* moments, long long n_moments, float4* cells,
+cudaError_t launch_pack_step(PackCells kind, const double* moments, long long n_moments, float4* cells,
                              const double* parts, long long n_parts, float4* packed,
                              unsigned int* queue, cudaStream_t s) {
   if (n_moments <= 0 && n_parts <= 0 && !queue) return cudaSuccess;
   const int grid = grid_for(std::max(0ll, n_moments) + std::max(0ll, n_parts) + kPackTile, kPackTile);
   TimingScope ts(kKidPack, s);
-  if (hex) pack_step_kernel<true><<<grid, kPackTile, 0, s>>>(moments, n_moments, cells, parts, n_parts, packed, queue);
-  else pack_step_kernel<false><<<grid, kPackTile, 0, s>>>(moments, n_moments, cells, parts, n_parts, packed, queue);
+  auto* kernel = kind == kPackQuad  ? pack_step_kernel<kPackQuad>
+                 : kind == kPackHex ? pack_step_kernel<kPackHex>
+                                    : pack_step_kernel<kPackHexPaired>;
+  kernel<<<grid, kPackTile, 0, s>>>(moments, n_moments, cells, parts, n_parts, packed, queue);
   count_launch();
   return cudaGetLastError();
 }
 
 cudaError_t launch_pack_cells(const double* moments, long long n, float4* out, cudaStream_t s) {
-  return launch_pack_step(false, moments, n, out, nullptr, 0, nullptr, nullptr, s);
+  return launch_pack_step(kPackQuad, moments, n, out, nullptr, 0, nullptr, nullptr, s);
 }
 
 /* hexadecapole FP32-mixed cell kernel: 0 synchronous staging
@@ -2486,19 +2549,18 @@ cudaError_t launch_pack_cells(const double* moments, long long n, float4* out, c
  * resident blocks per SM) */
 std::atomic<int> g_hex_variant{2};
 
-cudaError_t launch_list_hex(int form, const ListArgs& a, cudaStream_t s) {
+cudaError_t launch_list_hex(int form, const ListArgs& a, int variant, cudaStream_t s) {
   if (form == kF64) {
     static std::atomic<int> occ{0};
     return launch_kernel(list_kernel_hex<kF64>, &occ, list_kernel_id(kF64, true), a, s);
   }
   if (form == kMix) {
     const int kid = list_kernel_id(kMix, true);
-    const int hv = g_hex_variant.load();
-    if (hv == 1) {
+    if (variant == 1) {
       static std::atomic<int> occ{0};
       return launch_kernel(list_kernel_hex2<kMix, 1>, &occ, kid, a, s);
     }
-    if (hv == 2) {
+    if (variant == 2) {
       static std::atomic<int> occ{0};
       return launch_kernel(list_kernel_hex2<kMix, 2>, &occ, kid, a, s);
     }
@@ -2526,7 +2588,7 @@ cudaError_t launch_cells_as_parts(const double* moments, int stride, long long n
 }
 
 cudaError_t launch_pack_parts(const double* parts, long long n, float4* out, cudaStream_t s) {
-  return launch_pack_step(false, nullptr, 0, nullptr, parts, n, out, nullptr, s);
+  return launch_pack_step(kPackQuad, nullptr, 0, nullptr, parts, n, out, nullptr, s);
 }
 
 }  // namespace chg

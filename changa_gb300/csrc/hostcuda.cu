@@ -1058,7 +1058,7 @@ int changa_gravity_step(int form, const double* moments, long long n_moments, co
   const void* ksrc = moments;
   const void* kpart = parts;
   if (f == kMix) {
-    CHG_CUDA(launch_pack_step(false, moments, n_moments, (float4*)block, parts, n_parts,
+    CHG_CUDA(launch_pack_step(kPackQuad, moments, n_moments, (float4*)block, parts, n_parts,
                               (float4*)(block + cb), q, s));
     ksrc = block;
     kpart = block + cb;
@@ -1117,6 +1117,7 @@ int changa_gravity_step_hexa(int form, const double* moments, long long n_moment
   const void* kcell = moments;
   const void* kpart = parts;
   const void* kpseudo = pseudo;
+  const int variant = get_hex_variant();
   int rc = 0;
   cudaError_t e = cudaSuccess;
   do {
@@ -1127,7 +1128,7 @@ int changa_gravity_step_hexa(int form, const double* moments, long long n_moment
       float4* pc = (float4*)(block + qb);
       float4* pp = (float4*)(block + qb + cb);
       float4* ps = (float4*)(block + qb + cb + pb);
-      if ((e = launch_pack_step(true, moments, n_moments, pc, parts, n_parts, pp, q, s)) !=
+      if ((e = launch_pack_step(variant ? kPackHexPaired : kPackHex, moments, n_moments, pc, parts, n_parts, pp, q, s)) !=
           cudaSuccess)
         break;
       if (softcells && softcells->n_buckets > 0 &&
@@ -1156,7 +1157,7 @@ int changa_gravity_step_hexa(int form, const double* moments, long long n_moment
       a.fperiod_f = (float)fperiod;
       a.fperiod_d = fperiod;
       a.queue = q;
-      if ((e = launch_list_hex(f, a, s)) != cudaSuccess) break;
+      if ((e = launch_list_hex(f, a, variant, s)) != cudaSuccess) break;
       list = true;
     }
     if (plist && plist->n_buckets > 0) {

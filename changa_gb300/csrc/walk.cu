@@ -1833,7 +1833,7 @@ extern "C" int changa_walk_forces(const ChangaTreeView* t, const ChangaWalkParam
   if (!pc || !ppk || !queue)
     return finish(record_error(cudaErrorMemoryAllocation, "walk_forces: memory", __FILE__, __LINE__));
   cudaError_t e;
-  if ((e = launch_pack_step(false, moments, t->n_nodes, pc, parts, n_parts, ppk, nullptr, s)) !=
+  if ((e = launch_pack_step(kPackQuad, moments, t->n_nodes, pc, parts, n_parts, ppk, nullptr, s)) !=
       cudaSuccess)
     return finish(record_error((int)e, "walk_forces: pack", __FILE__, __LINE__));
   const int gmax = g_group_max.load() > 0 ? g_group_max.load() : 32;

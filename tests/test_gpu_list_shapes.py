@@ -246,3 +246,63 @@ def test_dropin_list_around_two_default_chunks(cuda_ok, extra):
         inp.free()
     assert (whole[:n_tgt, :3] > 0).all() and not whole[n_tgt:].any()
     np.testing.assert_allclose(got, whole, rtol=1e-5)
+
+
+@pytest.mark.parametrize("variant", [0, 1, 2])
+@pytest.mark.parametrize("period", [0.0, 4.0])
+def test_hexadecapole_kernels_at_tile_edges(cuda_ok, variant, period):
+    """Every number of lane groups a bucket can have (1 to 32) and list lengths
+    around their blocks.  Cells of radius 0.01 at separations above 0.2: the
+    monopole dominates a pair, so its some 30 roundings are below 2e-6 of M / r^2
+    and a block's FP32 sum adds at most 32 x 2^-24 = 2e-6."""
+    import torch
+    rng = np.random.default_rng(20261206)
+    n = 6000
+    parts = np.concatenate([np.full((n, 1), 1.0 / n), np.full((n, 1), 1e-4),
+                            rng.uniform(-0.5, 0.2, (n, 3))], 1)
+    nm = 512
+    mom = np.zeros((nm, 27))
+    mom[:, 0] = 0.01
+    mom[:, 1] = 1e-4
+    mom[:, 2] = rng.uniform(0.5, 2.0, nm) / nm
+    mom[:, 3:6] = rng.uniform(0.5, 1.0, (nm, 3))
+    mom[:, 6:] = rng.normal(0, 0.3, (nm, 21)) * mom[:, 2, None]
+    sizes = np.array([s for s in range(1, 34) for _ in LENGTHS], np.int32)
+    lens = np.array([k for _ in range(1, 34) for k in LENGTHS], np.int64)
+    assert sizes.sum() <= n + 2000
+    starts = (np.concatenate([[0], np.cumsum(sizes)[:-1]]) % (n - 40)).astype(np.int32)
+    markers = np.concatenate([[0], np.cumsum(lens)]).astype(np.int32)
+    lst = np.empty((int(lens.sum()), 2), np.int32)
+    lst[:, 0] = rng.integers(0, nm, len(lst))
+    o = rng.integers(-1, 2, (len(lst), 3)) if period else np.zeros((len(lst), 3), np.int64)
+    lst[:, 1] = ((o[:, 0] + 3) | ((o[:, 1] + 3) << 3) | ((o[:, 2] + 3) << 6)) << 22
+    req = ListRequest(lst, markers, starts, sizes, np.arange(len(sizes), dtype=np.int32))
+    # buckets share particles where the starts wrap, so each is evaluated for itself
+    first = np.concatenate([[0], np.cumsum(sizes)]).astype(np.int32)
+    rows = np.concatenate([np.arange(s, s + k) for s, k in zip(starts, sizes)])
+    own = np.ascontiguousarray(parts[rows])
+    req.starts = first[:-1].copy()
+    geom = np.zeros((len(sizes), 10))
+    for b in range(len(sizes)):
+        x = own[first[b]:first[b + 1], 2:]
+        geom[b, :3], geom[b, 3] = x.mean(0), 1e-4
+        geom[b, 4:7], geom[b, 7:] = x.min(0), x.max(0)
+    ref = oracle.cell_forces_hex(mom, own, req, geom, fperiod=period)
+    lib = N.cuda_lib()
+    dp, dm = torch.from_numpy(own).cuda(), torch.from_numpy(mom).cuda()
+    v = torch.zeros((len(own), 5), dtype=torch.float64, device="cuda")
+    r, keep = device(req)
+    none = N.ChangaListRequest()
+    saved = lib.changa_gb300_get_hex_variant()
+    assert lib.changa_gb300_set_hex_variant(variant) == 0
+    try:
+        N.check(lib.changa_gravity_step_hexa(N.CHANGA_FORM_MIXED, dm.data_ptr(), nm, dp.data_ptr(), len(own),
+                                             C.byref(r), C.byref(none), C.byref(none), period, None,
+                                             v.data_ptr(), torch.cuda.current_stream().cuda_stream))
+        v = v.cpu().numpy()
+    finally:
+        lib.changa_gb300_set_hex_variant(saved)
+    acc, pot = bound(req, mom[:, 2], mom[:, 3:6], own[:, 2:], 1e-4, period)
+    assert (np.abs(v[:, :3] - ref[:, :3]).max(1) <= 5e-6 * acc).all()
+    assert (np.abs(v[:, 3] - ref[:, 3]) <= 5e-6 * pot).all()
+    np.testing.assert_allclose(v[:, 4], ref[:, 4], rtol=2e-5)
