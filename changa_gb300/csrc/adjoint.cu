@@ -176,6 +176,7 @@ __global__ void __launch_bounds__(kThreads, 4) vjp_kernel(const VjpArgs a) {
   constexpr int kStride = CELL ? kCellAcc : kPartAcc;
   float* acc = a.acc + (size_t)((blockIdx.x * kWarps + warp) % kReplicas) * a.n_src * kStride;
 
+  open_to_next();
   for (;;) {
     int b = 0;
     if (lane == 0) b = (int)atomicAdd(a.queue, 1u);
@@ -452,6 +453,7 @@ __global__ void __launch_bounds__(kThreads, 4) vjp_kernel(const VjpArgs a) {
           cur = nxt;
         }
         reduce_scatter16(v, lane);
+        wait_for_last();
         const int t = hl >> 1, q = 2 * (hl & 1);
         if (t < myn) {
           double* gt = a.grad_tgt + 4 * (tbase + tb0 + my0 + t) + q;
@@ -461,6 +463,7 @@ __global__ void __launch_bounds__(kThreads, 4) vjp_kernel(const VjpArgs a) {
       }
     }
   }
+  wait_for_last();
 }
 
 __global__ void pack_lambda_kernel(const double* __restrict__ lam, long long n,
@@ -620,6 +623,7 @@ extern "C" int changa_gravity_vjp_mixed(const double* moments, long long n_momen
     pack_lambda_kernel<<<grid_of(n_parts, 256), 256, 0, s>>>(lam, n_parts, pl);
   }
   count_launch();
+  bool after_list = false;
   for (int k = 0; k < 2; ++k) {
     const ChangaListRequest* r = reqs[k];
     if (!r || r->n_buckets == 0 || n_parts == 0 || (k == 0 ? n_moments : n_parts) == 0) continue;
@@ -642,11 +646,13 @@ extern "C" int changa_gravity_vjp_mixed(const double* moments, long long n_momen
     const int grid = grid_of(((long long)r->n_buckets + kWarps - 1) / kWarps, 1);
     {
       TimingScope ts(k == 0 ? kKidVjpCell : kKidVjpPart, s);
-      if (k == 0) vjp_kernel<true><<<grid, kThreads, 0, s>>>(va);
-      else vjp_kernel<false><<<grid, kThreads, 0, s>>>(va);
+      /* the two lists meet only in grad, so the particle lists start while
+       * the cell lists drain */
+      CHG_CUDA(launch_after(k == 0 ? vjp_kernel<true> : vjp_kernel<false>, grid, kThreads, s,
+                            after_list && !ts.start, va));
     }
+    after_list = true;
     count_launch();
-    CHG_CUDA(cudaGetLastError());
   }
   {
     TimingScope ts(kKidMoments, s);
