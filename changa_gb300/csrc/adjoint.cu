@@ -166,8 +166,13 @@ __device__ __forceinline__ void load_src(const VjpArgs& a, int e, int e_end, Src
   }
 }
 
+/* Latency-bound (a quarter of the warps, waits on the entries' records), so
+ * the particle lists' kernel takes 96 registers for a fifth resident CTA:
+ * 65536 Plummer particles 419 -> 400 us for the whole adjoint, 120000 in
+ * buckets of 32 1049 -> 973; at six CTAs it spills (424, 1082), and the cell
+ * lists' kernel spills at five (412, 982). */
 template <bool CELL>
-__global__ void __launch_bounds__(kThreads, 4) vjp_kernel(const VjpArgs a) {
+__global__ void __launch_bounds__(kThreads, CELL ? 4 : 5) vjp_kernel(const VjpArgs a) {
   __shared__ __align__(16) float4 tpos[kWarps][kTB];
   __shared__ __align__(16) float4 tlam[kWarps][kTB];
   __shared__ float tsoft[kWarps][kTB];
