@@ -151,19 +151,24 @@ static void signal(cudaStream_t s, void* cb) {
 
 static size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
-/* Bytes per upload chunk of a list of `bytes`: the caller's setting
- * (changa_gb300_set_host_chunk_bytes), else an eighth of the list, between 32
- * and 256 MiB, so that the upload of a list of a few hundred MB overlaps its
- * kernels too.  Each chunk's kernel drains for about a bucket's time, so
- * chunks below 32 MiB lose more than they overlap.  us per call with chunks
- * of 256 / 64 / 32 / 16 / 8 MiB: runs entry, 2^20 particles (208 MB of
+/* Bytes per upload chunk of a list of `bytes` for n_buckets buckets: the
+ * caller's setting (changa_gb300_set_host_chunk_bytes), else an eighth of the
+ * list, between 32 and 256 MiB, so that the upload of a list of a few hundred
+ * MB overlaps its kernels too.  Each chunk's kernel drains for about a
+ * bucket's time, so chunks below 32 MiB, and of fewer buckets than the GPU
+ * has warps for (24 per SM), lose more than they overlap.  us per call with
+ * chunks of 256 / 64 / 32 / 16 / 8 MiB: runs entry, 2^20 particles (208 MB of
  * cells) 4190 / 3540 / 3595 / 3784 / 4144; drop-in, 500009 particles (110 MB
- * and 240 MB of lists) 3470 / 3613 / 2557 / 2952 / 3391. */
+ * and 240 MB of lists) 3470 / 3613 / 2557 / 2952 / 3391; drop-in, 200000
+ * particles in 4400 buckets, 2290 whole, 2740 in chunks of 32 MiB. */
 constexpr size_t kMinHostChunkBytes = size_t(32) << 20, kMaxHostChunkBytes = size_t(256) << 20;
 static std::atomic<size_t> g_host_chunk_bytes{0};
-static size_t host_chunk_bytes(size_t bytes) {
+static size_t host_chunk_bytes(size_t bytes, long long n_buckets = 0) {
   if (const size_t set = g_host_chunk_bytes.load()) return set;
-  return std::min(kMaxHostChunkBytes, std::max(kMinHostChunkBytes, bytes / 8));
+  size_t least = kMinHostChunkBytes;
+  if (n_buckets > 0)
+    least = std::max(least, (size_t)((double)bytes * 24.0 * sm_count() / (double)n_buckets));
+  return std::min(kMaxHostChunkBytes, std::max(least, bytes / 8));
 }
 
 /* The library-owned streams of the host-array entries on each device
@@ -184,12 +189,15 @@ static cudaStream_t library_stream(int which = 0) {
 }
 
 /* Bucket ranges [b0, b1) of a request, about `per` list entries each; with
- * shrink, the last 2 per entries go in halving chunks (down to per / 16),
- * so little arithmetic is left once the final entries have landed. */
+ * shrink, the last 2 per entries go in halving chunks (down to kLastEntries,
+ * 11 to 17 MB, or per / 16 where that is more; down to per / 2 where a chunk is
+ * smaller than that), so little arithmetic is left once the final entries have
+ * landed.  Smaller ones drain longer than they take to land. */
+constexpr long long kLastEntries = (16ll << 20) / sizeof(ILPart);
 static void list_chunks(const ChangaListRequest* r, long long per, bool shrink,
                         std::vector<std::pair<int, int>>& out) {
   const long long total = r->markers[r->n_buckets];
-  const long long floor_ = std::max<long long>(1, per / 16);
+  const long long floor_ = std::max({1ll, per / 16, std::min(per / 2, kLastEntries)});
   int b0 = 0;
   while (b0 < r->n_buckets) {
     const long long left = total - r->markers[b0];
@@ -358,7 +366,7 @@ static int run_request(CudaRequest* r, bool cell, const void* sources, long long
    * not part of the capture) unless the list is past the largest chunks */
   cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
   CHG_CUDA(cudaStreamIsCapturing(r->stream, &capture));
-  size_t chunk = host_chunk_bytes((size_t)std::max(0, r->numInteractions) * sizeof(ILCell));
+  size_t chunk = host_chunk_bytes((size_t)std::max(0, r->numInteractions) * sizeof(ILCell), nb);
   if (capture != cudaStreamCaptureStatusNone) chunk = std::max(chunk, kMaxHostChunkBytes);
   const long long per = (long long)(chunk / sizeof(ILCell));
   if (r->numInteractions > 2 * per) {
@@ -1277,11 +1285,13 @@ static int step_host_impl(int form, const double* moments, long long n_moments,
       rview.markers = pruns->run_markers;
       rview.n_entries = pruns->n_runs;
       list_chunks(&rview,
-                  (long long)(host_chunk_bytes((size_t)pruns->n_runs * sizeof(ILPart)) / sizeof(ILPart)),
+                  (long long)(host_chunk_bytes((size_t)pruns->n_runs * sizeof(ILPart), r->n_buckets) /
+                              sizeof(ILPart)),
                   k == last, chunks[k]);
     } else {
       list_chunks(r,
-                  (long long)(host_chunk_bytes((size_t)r->n_entries * sizeof(ILCell)) / sizeof(ILCell)),
+                  (long long)(host_chunk_bytes((size_t)r->n_entries * sizeof(ILCell), r->n_buckets) /
+                              sizeof(ILCell)),
                   k == last, chunks[k]);
     }
   }

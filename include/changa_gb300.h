@@ -239,7 +239,8 @@ int changa_gravity_step_host_runs(int form, const double *moments, long long n_m
 
 /* List bytes per upload chunk of changa_gravity_step_host and of the
  * drop-in list transfers (at least 4 KiB; 0, the default: an eighth of the
- * list, between 32 and 256 MiB).  changa_gravity_step_host uploads the particles first, in
+ * list, but no fewer buckets than the GPU has warps for, between 32 and 256
+ * MiB).  changa_gravity_step_host uploads the particles first, in
  * slices of a quarter chunk.  A drop-in
  * request whose list exceeds two chunks uploads it chunk by chunk on the
  * library's copy stream, each chunk's buckets evaluated as it lands. */
