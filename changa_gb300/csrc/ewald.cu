@@ -353,6 +353,8 @@ __device__ __forceinline__ void ewald_term_f64(const EwaldFpArgs& P, double x, d
 }
 
 
+constexpr int kF64Warp = 32;  // threads of an FP64 block, one warp
+
 /* One thread per particle.  FP64 instructions bound it (one per SM in 16
  * cycles), so the replicas are first culled in FP32 against the box of the
  * warp's 32 particles (about 90 of 343 are left, and only they are tested in
@@ -361,20 +363,21 @@ __device__ __forceinline__ void ewald_term_f64(const EwaldFpArgs& P, double x, d
  * per h and four FP64 operations per product; the Gaussian of a replica is a
  * product over the axes.  120011 particles, cut 2.6, h-cut 2.8: 3392 us with
  * a test per replica, an exponential and an erfc per term and a sincos per h,
- * 2370 so (FP64 pipe 86% busy; erfcx is most of what is left). */
+ * 2370 so, 2193 in blocks of a warp (FP64 pipe 86% busy; erfcx is most of
+ * what is left). */
 template <bool HEX>
-__global__ void __launch_bounds__(128) ewald_f64_kernel(const double* __restrict__ parts,
-                                                        long long n_parts,
-                                                        const int* __restrict__ idx,
-                                                        long long n_idx, double* __restrict__ vars,
-                                                        const __grid_constant__ EwaldFpArgs P) {
+__global__ void __launch_bounds__(kF64Warp) ewald_f64_kernel(const double* __restrict__ parts,
+                                                             long long n_parts,
+                                                             const int* __restrict__ idx,
+                                                             long long n_idx, double* __restrict__ vars,
+                                                             const __grid_constant__ EwaldFpArgs P) {
   constexpr int kBatch = 128;  // replicas culled at a time
-  __shared__ double rx[4][kBatch], ry[4][kBatch], rz[4][kBatch];  // replica offsets
-  __shared__ int rcode[4][kBatch];                                // offsets per axis, and the hole
+  __shared__ double rx[kBatch], ry[kBatch], rz[kBatch];  // replica offsets
+  __shared__ int rcode[kBatch];                          // offsets per axis, and the hole
   /* first exp(-alpha^2 (d + i L)^2) per axis for |i| <= 3, then
    * exp(2 pi i k d / L) for k = 1 .. kWholeMax */
-  __shared__ double pw[3][kWholeMax][2][128];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  __shared__ double pw[3][kWholeMax][2][kF64Warp];
+  const int lane = threadIdx.x;
   const long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   long long j = -1;
   if (k < n_idx) {
@@ -411,7 +414,7 @@ __global__ void __launch_bounds__(128) ewald_f64_kernel(const double* __restrict
     for (int c = 0; c < 3; ++c)
       for (int i = -nE; i <= nE; ++i) {
         const double u = dd[c] + i * P.L;
-        (&pw[c][0][0][0])[(i + 3) * 128 + threadIdx.x] = exp(-P.alpha2 * (u * u));
+        (&pw[c][0][0][0])[(i + 3) * kF64Warp + threadIdx.x] = exp(-P.alpha2 * (u * u));
       }
   for (long long r0 = 0; r0 < nrep; r0 += kBatch) {
     int count = 0;
@@ -437,26 +440,26 @@ __global__ void __launch_bounds__(128) ewald_f64_kernel(const double* __restrict
       const unsigned m = __ballot_sync(0xffffffffu, keep);
       if (keep) {
         const int at = count + __popc(m & ((1u << lane) - 1u));
-        rx[warp][at] = i[0] * P.L;
-        ry[warp][at] = i[1] * P.L;
-        rz[warp][at] = i[2] * P.L;
-        rcode[warp][at] = split ? (i[0] + 3) | (i[1] + 3) << 3 | (i[2] + 3) << 6 | hole << 9 : hole << 9;
+        rx[at] = i[0] * P.L;
+        ry[at] = i[1] * P.L;
+        rz[at] = i[2] * P.L;
+        rcode[at] = split ? (i[0] + 3) | (i[1] + 3) << 3 | (i[2] + 3) << 6 | hole << 9 : hole << 9;
       }
       count += __popc(m);
     }
     __syncwarp();
     for (int q = 0; q < count; ++q) {
-      const int code = rcode[warp][q];
+      const int code = rcode[q];
       const bool hole = code >> 9;
-      const double x = dxd + rx[warp][q], y = dyd + ry[warp][q], z = dzd + rz[warp][q];
+      const double x = dxd + rx[q], y = dyd + ry[q], z = dzd + rz[q];
       const double r2 = x * x + y * y + z * z;
       if (!live || (r2 > P.fEwCut2 && !hole)) continue;
       ewald_term_f64<HEX>(P, x, y, z, r2, hole, fInner2,
                           [&](double s) {
                             if (!split) return exp(-s * P.alpha2);
                             const double* g = &pw[0][0][0][0] + threadIdx.x;
-                            return g[128 * (code & 7)] * g[128 * (8 + (code >> 3 & 7))] *
-                                   g[128 * (16 + (code >> 6 & 7))];
+                            return g[kF64Warp * (code & 7)] * g[kF64Warp * (8 + (code >> 3 & 7))] *
+                                   g[kF64Warp * (16 + (code >> 6 & 7))];
                           },
                           fPot, ax, ay, az);
     }
@@ -948,11 +951,13 @@ bool pair_h(const ChangaEwaldParams& p, double L, std::vector<HPair>& out) {
 
 }  // namespace
 
-/* Threads per block (one per particle): single warps while blocks of four
- * would leave SMs without one.  Each warp's results are the same either way
- * (a warp culls for its own 32 particles).  3000 particles, FP64: 495 us
- * with blocks of 128. */
-static int ewald_threads(long long n) { return n <= 128ll * sm_count() ? 32 : 128; }
+/* Threads per block of the mixed kernel (one per particle): single warps, which
+ * spread evenly, while there are few (us a step with blocks of 32 / 128: 40000
+ * particles 128 / 137, 60000 169 / 179, 90000 290 / 289, 200000 574 / 564).
+ * Each warp's results are the same either way (a warp culls for its own 32
+ * particles).  The FP64 kernel's blocks are always single warps (3000 particles
+ * 495 us in blocks of 128, 422 so). */
+static int ewald_threads(long long n) { return n <= 512ll * sm_count() ? 32 : 128; }
 
 cudaError_t launch_ewald_fp(int form, const double* parts, long long n_parts, const int* idx,
                             long long n_idx, const ChangaEwaldParams& p, double* vars,
@@ -992,15 +997,20 @@ cudaError_t launch_ewald_fp(int form, const double* parts, long long n_parts, co
       P.hc[i][1] = pairs[i].s;
     }
     if (hex) fill_hex_root(p.momc, P.hex);
-    const int threads = ewald_threads(n_idx);
+    const int threads = kF64Warp;
     const int blocks = (int)((n_idx + threads - 1) / threads);
     static const bool split = (set_carveout(ewald_f64_kernel<true>, kCarveoutFp64),
                                set_carveout(ewald_f64_kernel<false>, kCarveoutFp64), true);
     (void)split;
     TimingScope ts(kKidEwaldF64, s);
     count_launch();
+    /* Blocks that start early share the SMs that free up first, and an SM's
+     * FP64 pipe is the bound, so the launch overlaps the lists only when it
+     * fills every SM (24 warps): 27000 particles 2790 us a step overlapped,
+     * 1500 not. */
+    const bool fills = n_idx > 24ll * kF64Warp * sm_count();
     return launch_after(hex ? ewald_f64_kernel<true> : ewald_f64_kernel<false>, blocks, threads, s,
-                        after_list && !ts.start, parts, n_parts, idx, n_idx, vars, P);
+                        after_list && fills && !ts.start, parts, n_parts, idx, n_idx, vars, P);
   }
   if (nE > kMixMaxReps) return cudaErrorInvalidValue;
   EwaldMixArgs P;
