@@ -2530,7 +2530,8 @@ cudaError_t launch_pack_step(PackCells kind, const double* moments, long long n_
                              const double* parts, long long n_parts, float4* packed,
                              unsigned int* queue, cudaStream_t s) {
   if (n_moments <= 0 && n_parts <= 0 && !queue) return cudaSuccess;
-  const int grid = grid_for(std::max(0ll, n_moments) + std::max(0ll, n_parts) + kPackTile, kPackTile);
+  const long long want = (std::max(0ll, n_moments) + std::max(0ll, n_parts)) / kPackTile + 2;
+  const int grid = (int)std::min<long long>(want, (long long)sm_count() * 16);
   TimingScope ts(kKidPack, s);
   auto* kernel = kind == kPackQuad  ? pack_step_kernel<kPackQuad>
                  : kind == kPackHex ? pack_step_kernel<kPackHex>

@@ -430,7 +430,7 @@ void changa_walk_set_groups(int max_buckets, int min_tree_buckets);
  * bucket, then the Ewald term added when ewald is given.  The interactions
  * are the list walk's; the sums agree with changa_gravity_step on its lists
  * to FP32 summation order.  On GB300 it is slower than changa_walk plus
- * changa_gravity_step (nfw8m: 86.6 ms against 37.7 ms), which stays the
+ * changa_gravity_step (nfw8m: 84.9 ms against 31.4 ms), which stays the
  * fast route.  Returns after the stream has finished. */
 int changa_walk_forces(const ChangaTreeView *tree, const ChangaWalkParams *p,
                        const double *moments, const double *parts, long long n_parts,
