@@ -460,14 +460,15 @@ __device__ __forceinline__ int climb_chain(const int* __restrict__ parent, long 
  * down to its group node (prefix lists and frontier); 2: each bucket from
  * its group's frontier, after its group's prefix lists.
  *
- * Bound by instruction issue and by L1 wavefronts alike (66 % and 60 % of
- * their peaks for the buckets of 2^20 clustered particles), so the step is
+ * Bound by instruction issue (70 % of the slots; 42 % of the L1 wavefronts;
+ * the buckets of a million clustered particles), so the step is
  * short: a test of some 40 instructions on a 32-byte record per source node
  * and one per local node, pushes and list positions from ballots (no scans),
  * particles expanded only in steps that open a source bucket.  Shared memory
  * is kept to the stack: each KB taken from L1 costs hits on the node records
  * (with a table of chunks beside the stack and 96-byte records the L1 hit rate
- * was 38 %, and the pass took as long as one of 35 % more instructions).
+ * was 38 %, now 70 %, and the pass took as long as one of 35 % more
+ * instructions).
  * 1000003 NFW particles in buckets of 16, the bucket pass: 1982 us with FP32
  * boxes, per-axis margins and scans, 1447 us so; 2^23 in buckets of 32: the
  * whole walk 14.1 ms, 11.1 ms so. */
@@ -1544,6 +1545,9 @@ static int walk_groups(WalkGroups& gr, const ChangaTreeView* t, int gmax, Scratc
  * buckets of at most 32 (2^23 NFW particles, theta 0.7): 686 cells, 1507
  * particles, 175 in the frontier; of 5600 at theta 0.5: 1292, 2219, 365. */
 constexpr int kSlotCells = 2048, kSlotParts = 3072, kSlotFront = 1024;
+/* The slots of all groups together (87000 groups); more groups are counted
+ * and filled, which takes some 6 % of the walk of so large a tree. */
+constexpr size_t kMaxSlotBytes = size_t(4) << 30;
 
 /* Phase 1 of the two-phase walk: each group's node walked once.  Its chain
  * down to the group node is shared by all the group's buckets, so the
@@ -1576,7 +1580,8 @@ static int walk_phase1(WalkArgs& a, WalkGroups& gr, WalkTry& how, Scratch& sc, c
     a.goff[k] = nullptr;
   }
   if (how.slots && !gr.slots) {
-    gr.slots = (int2*)sc.alloc((size_t)ng * (kSlotCells + kSlotParts + kSlotFront) * sizeof(int2));
+    const size_t bytes = (size_t)ng * (kSlotCells + kSlotParts + kSlotFront) * sizeof(int2);
+    gr.slots = bytes <= kMaxSlotBytes ? (int2*)sc.alloc(bytes) : nullptr;
     if (!gr.slots) {
       cudaGetLastError();  // no room for the slots: count and fill
       how.slots = false;
