@@ -1803,7 +1803,8 @@ struct RawHex {
  * packed cells (kPackHexPaired, 128 bytes): the lane's own two first words as
  * h and l, and the other six row by row, eight lanes to a row, so that a load
  * touches four lines and not 32: w[i] is word lane & 7 of entry 4 i + lane / 8.
- * Entries past the end repeat the last one (stage_hex_rows sets them far). */
+ * Entries past the end repeat the last one (stage_hex_rows sets them far), so
+ * the list has one entry at least. */
 template <int FORM>
 __device__ __forceinline__ void gather_hex(const ListArgs& a, int e, int e_end, RawHex& r) {
   long long idx = 0;
@@ -2105,7 +2106,7 @@ __global__ void __launch_bounds__(kThreads, MINB) list_kernel_hex2(const ListArg
        * entries where the groups outnumber the pairs) */
       const int block = G < 16 ? 2 * G * (16 / G) : 32;
       RawHex raw;
-      gather_hex<FORM>(a, e_begin + lane, e_end, raw);
+      if (e_begin < e_end) gather_hex<FORM>(a, e_begin + lane, e_end, raw);
       for (int e0 = e_begin; e0 < e_end; e0 += block) {
         const int ne = min(block, e_end - e0);
         if constexpr (FORM == kMix)
