@@ -249,8 +249,9 @@ __device__ __forceinline__ void join_groups(const ListArgs& a, const float2 (&re
   }
 }
 
-/* Entry `at` of the `left` entries that start at e0; a massless entry past
- * them (offsets, not sums, are compared: e0 + at may pass the int range). */
+/* Entry `at` of the `left` entries that start at e0; past them source 0, whose
+ * record the callers leave out (offsets, not sums, are compared: e0 + at may
+ * pass the int range). */
 __device__ __forceinline__ int2 entry_at(const ListArgs& a, int e0, int at, int left) {
   return at < left ? __ldg(a.list + e0 + at) : make_int2(0, 0xdb << 22);
 }
@@ -709,6 +710,7 @@ __global__ void __launch_bounds__(256, MINB) list_kernel_far(const ListArgs a) {
         bool one_mass = false;
         if constexpr (!CELL) {
           m0 = __shfl_sync(kFull, rec[0].w, __ffs(fb) - 1);
+          if (fb == 0u) m0 = 0.f;  // no far source: lane 31's may not be in the list
           one_mass = __all_sync(kFull, !far || rec[0].w == m0);
         }
         if (fb == kFull) {

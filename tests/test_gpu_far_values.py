@@ -1,0 +1,65 @@
+"""Values that the far-first list kernels must neither spread nor lose: sources
+that are not in a bucket's list, masses that are infinite or not a number,
+sums that overflow, and the last bits of the lane groups' sums."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from changa_gb300 import _native as N
+
+pytestmark = pytest.mark.gpu
+
+HERE = (3 | 3 << 3 | 3 << 6) << 22  # the replica at the origin
+
+
+def evaluate(call, sources, targets, lists):
+    """`call` on buckets of one list each: lists holds (first target, targets,
+    source indices)."""
+    import torch
+    idx = np.concatenate([np.asarray(l[2], np.int32) for l in lists])
+    entries = np.stack([idx, np.full(len(idx), HERE, np.int32)], 1)
+    markers = np.concatenate([[0], np.cumsum([len(l[2]) for l in lists])]).astype(np.int32)
+    t = [torch.from_numpy(np.ascontiguousarray(x)).cuda() for x in
+         (entries, markers, np.array([l[0] for l in lists], np.int32),
+          np.array([l[1] for l in lists], np.int32), sources, targets)]
+    r = N.ChangaListRequest()
+    r.list, r.markers, r.starts, r.sizes = (x.data_ptr() for x in t[:4])
+    r.n_buckets, r.n_entries = len(lists), len(idx)
+    v = torch.zeros((len(targets), 5), dtype=torch.float64, device="cuda")
+    N.check(call(t[4].data_ptr(), len(sources), t[5].data_ptr(), len(targets), C.byref(r), 0.0,
+                 v.data_ptr(), torch.cuda.current_stream().cuda_stream))
+    return v.cpu().numpy()
+
+
+@pytest.fixture(params=[17, 18])
+def variant(cuda_ok, request):
+    """A warp per bucket, a CTA per bucket."""
+    lib = N.cuda_lib()
+    saved = [lib.changa_gb300_get_list_variant(k) for k in (4, 5)]
+    for k in (4, 5):
+        assert lib.changa_gb300_set_list_variant(k, request.param) == 0
+    yield request.param
+    for k, s in zip((4, 5), saved):
+        lib.changa_gb300_set_list_variant(k, s)
+
+
+@pytest.mark.parametrize("bad", [np.nan, np.inf, -np.inf])
+@pytest.mark.parametrize("n_list", [1, 5, 31])
+def test_a_mass_that_is_not_in_the_list(variant, bad, n_list):
+    """Particle 0 has no finite mass and is in no list; the buckets' sources
+    are all within the softening, so no block has a far source."""
+    rng = np.random.default_rng(n_list)
+    parts = np.concatenate([np.full((64, 1), 0.5), np.full((64, 1), 10.0),
+                            rng.uniform(-1, 1, (64, 3))], 1)
+    sizes = [1, 3, 16]
+    lists, at = [], 1
+    for s in sizes:
+        lists.append((at, s, rng.choice(np.arange(21, 64), n_list, replace=False)))
+        at += s
+    call = N.cuda_lib().changa_part_forces_mixed
+    want = evaluate(call, parts, parts, lists)
+    parts[0, 0] = bad
+    got = evaluate(call, parts, parts, lists)
+    assert np.isfinite(want).all() and (want[1:at, 3] < 0).all()
+    assert np.array_equal(got[1:at], want[1:at])
