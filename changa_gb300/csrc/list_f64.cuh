@@ -157,7 +157,8 @@ __global__ void __launch_bounds__(kF64Threads, 2) list_kernel_f64(const ListArgs
     __syncthreads();  // every thread has read snext
     if (tid == 0) snext = (int)atomicAdd(a.queue, 1u);
     const int e_begin = max(__ldg(a.markers + b), 0);
-    const int e_end = (int)min((long long)__ldg(a.markers + b + 1), a.n_entries);  // memory safety
+    /* memory safety: within the list, and no wrapped difference */
+    const int e_end = max((int)min((long long)__ldg(a.markers + b + 1), a.n_entries), e_begin);
     const long long tbase = __ldg(a.starts + b);
     const int n = __ldg(a.sizes + b);
     const bool skip = n <= 0 || tbase < 0 || tbase + n > a.n_tgt;  // memory safety

@@ -388,7 +388,8 @@ __global__ void __launch_bounds__(T, MINB) list_kernel_block(const ListArgs a) {
     __syncthreads();  // every thread has read snext
     if (tid == 0) snext = (int)atomicAdd(a.queue, 1u);
     const int e_begin = max(__ldg(a.markers + b), 0);
-    const int e_end = (int)min((long long)__ldg(a.markers + b + 1), a.n_entries);  // memory safety
+    /* memory safety: within the list, and no wrapped difference */
+    const int e_end = max((int)min((long long)__ldg(a.markers + b + 1), a.n_entries), e_begin);
     const long long tbase = __ldg(a.starts + b);
     const int n = __ldg(a.sizes + b);
     const bool skip = n <= 0 || tbase < 0 || tbase + n > a.n_tgt;  // memory safety
@@ -633,7 +634,8 @@ __global__ void __launch_bounds__(256, MINB) list_kernel_far(const ListArgs a) {
     b = __shfl_sync(kFull, b, 0);
     if (b >= a.n_buckets) break;
     const int e_begin = max(__ldg(a.markers + b), 0);
-    const int e_end = (int)min((long long)__ldg(a.markers + b + 1), a.n_entries);  // memory safety
+    /* memory safety: within the list, and no wrapped difference */
+    const int e_end = max((int)min((long long)__ldg(a.markers + b + 1), a.n_entries), e_begin);
     const long long tbase = __ldg(a.starts + b);
     const int n = __ldg(a.sizes + b);
     if (n <= 0 || tbase < 0 || tbase + n > a.n_tgt) continue;  // memory safety

@@ -63,3 +63,32 @@ def test_a_mass_that_is_not_in_the_list(variant, bad, n_list):
     got = evaluate(call, parts, parts, lists)
     assert np.isfinite(want).all() and (want[1:at, 3] < 0).all()
     assert np.array_equal(got[1:at], want[1:at])
+
+
+@pytest.mark.parametrize("name", ["part_forces_mixed", "cell_forces_mixed", "part_forces_fp64",
+                                  "cell_forces_fp64"])
+def test_a_marker_far_below_zero_is_an_empty_list(variant, name):
+    """A list that ends 2^31 before it begins holds nothing; the length of the
+    next one is that of its entries."""
+    import torch
+    rng = np.random.default_rng(4)
+    targets = np.concatenate([np.ones((40, 1)), np.full((40, 1), 0.1), rng.normal(size=(40, 3))], 1)
+    sources = targets
+    if name.startswith("cell"):
+        sources = np.zeros((40, 12))
+        sources[:, 1], sources[:, 2], sources[:, 3:6] = 0.1, 1.0, rng.normal(size=(40, 3)) + 5
+    entries = np.stack([np.arange(40), np.full(40, HERE)], 1).astype(np.int32)
+    markers = np.array([7, -2 ** 31, 40, 40], np.int32)  # lists 7.., 0..40 and an empty one
+    t = [torch.from_numpy(np.ascontiguousarray(x)).cuda() for x in
+         (entries, markers, np.array([0, 10, 30], np.int32), np.array([10, 20, 10], np.int32),
+          sources, targets)]
+    r = N.ChangaListRequest()
+    r.list, r.markers, r.starts, r.sizes = (x.data_ptr() for x in t[:4])
+    r.n_buckets, r.n_entries = 3, 40
+    v = torch.zeros((40, 5), dtype=torch.float64, device="cuda")
+    call = getattr(N.cuda_lib(), "changa_" + name)
+    N.check(call(t[4].data_ptr(), 40, t[5].data_ptr(), 40, C.byref(r), 0.0, v.data_ptr(),
+                 torch.cuda.current_stream().cuda_stream))
+    v = v.cpu().numpy()
+    want = evaluate(call, sources, targets, [(0, 10, []), (10, 20, range(40))])
+    assert (want[10:30, 3] < 0).all() and np.array_equal(v, want)
