@@ -165,6 +165,8 @@ constexpr float kU = 5.9604645e-08f;  // 2^-24, the FP32 unit roundoff
  * that the offset's part may be added to it: (a + b)^2 <= 2 a^2 + 2 b^2. */
 constexpr float kScreen = 1.3e-4f;
 constexpr double kScreenE = 2.0 * 3.0 * 8200.0;
+constexpr double kScreenH = 4.0 * kU;          // eps per unit of h
+constexpr double kScreenM = kU / 64.0;         // and of |m| + h: 2^-30
 
 /* Each node's traversal records; the opening radius squared is formed in FP64
  * exactly as open_criterion forms it.  Under the hexadecapole rules also the
@@ -203,7 +205,7 @@ __global__ void walk_prep_kernel(const double* __restrict__ geom, const double* 
       mx = fmax(mx, fabs(m[k]));
       hx = fmax(hx, fabs(h[k]));
     }
-    const double u = kU, eps = 4.0 * u * hx + 64.0 * u / 65536.0 * (mx + hx);
+    const double eps = kScreenH * hx + kScreenM * (mx + hx);
     const float px = (float)m[0], py = (float)m[1], pz = (float)m[2];
     const unsigned lxy = to_bf((float)(m[0] - px)) | to_bf((float)(m[1] - py)) << 16;
     const unsigned lze = to_bf((float)(m[2] - pz)) << 16 | to_bf_up((float)(kScreenE * eps * eps + 1e-37));
@@ -222,8 +224,9 @@ __global__ void walk_prep_kernel(const double* __restrict__ geom, const double* 
 }
 
 /* v <= r2 decided from an FP32 sum of squares v with margin e and r2 = rn32
- * of the FP64 threshold: 1 certainly, 0 certainly not, -1 too close; NaN or
- * infinity give -1 (an infinite r2 alone gives 1). */
+ * of the FP64 threshold: 1 certainly, 0 certainly not, -1 too close or not
+ * comparable (a NaN, an infinite e, or v and r2 both infinite).  An infinite r2
+ * alone gives 1, an infinite v alone 0. */
 __device__ __forceinline__ int screen_le(float v, float e, float r2) {
   if (fmaf(v, 1.0f + kScreen, e) < r2) return 1;
   if (fmaf(v, 1.0f - kScreen, -e) > r2) return 0;
