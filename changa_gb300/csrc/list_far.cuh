@@ -28,6 +28,8 @@
  */
 #pragma once
 
+#include <cfloat>
+
 #include "list_eval.cuh"
 
 namespace chg {
@@ -186,35 +188,66 @@ __device__ __forceinline__ void pp_near_one(const float* pb, int h, float soft, 
   idt = fmaxf(idt, fmaf(tmass, bv, bm));
 }
 
-/* hi + lo += x.x + x.y, hi + lo kept as an unevaluated FP32 pair (Knuth's
- * two-sum): the groups' sums join without FP64 operations, of which GB300
- * issues one for 64 in FP32. */
-__device__ __forceinline__ void two_add(float& hi, float& lo, float2 x) {
-  const float s = hi + x.x;
-  const float bb = s - hi;
-  lo += ((hi - (s - bb)) + (x.x - bb)) + x.y;
-  hi = s;
+/* a + b as its rounded value and the rounding's error (Knuth's two-sum). */
+__device__ __forceinline__ float two_sum(float a, float b, float& err) {
+  const float s = a + b;
+  const float bb = s - a;
+  err = (a - (s - bb)) + (b - bb);
+  return s;
 }
 
-/* Adds one target's sums (unevaluated FP32 pairs) and dtGrav to vars. */
+/* Sum of the groups' unevaluated FP32 pairs, kept in three FP32 parts: the
+ * errors of the high parts go exactly to lo, whose own go to rest, so that G <=
+ * 128 terms of size h carry an error below 2 G^3 2^-72 h, less than the G 2^-53 h
+ * of a sum in FP64.  FP64 additions, of which GB300 issues one for 64 in FP32,
+ * cost 15 to 35 us here in a launch of 64 buckets (a group's chain of up to 128).
+ * With the low parts in one FP32 word, some 48 bits of the sum, a step of 32768
+ * Plummer particles takes 108.0 us and of 40 clusters in buckets of 16 1611,
+ * with three words 110.2 and 1623 (1647 with a lane per target for all four
+ * sums). */
+struct JoinSum {
+  float hi, lo, rest;
+  __device__ __forceinline__ void add(float2 x) {
+    float e0, e1, e2;
+    hi = two_sum(hi, x.x, e0);
+    lo = two_sum(lo, x.y, e1);
+    lo = two_sum(lo, e0, e2);
+    rest += e1 + e2;
+  }
+};
+
+/* The sum of the pairs at x[0], x[n], .. x[(G - 1) n], in FP64.  A sum that
+ * leaves the finite FP32 range is formed in FP64 from its terms, so that an
+ * infinite one stays infinite. */
+__device__ __forceinline__ double join_sum(const float2* x, int n, int G) {
+  JoinSum s{x[0].x, x[0].y, 0.f};
+  for (int g = 1; g < G; ++g) s.add(x[g * n]);
+  double r = (double)s.hi + ((double)s.lo + (double)s.rest);
+  if (!(fabsf(s.hi) <= FLT_MAX)) {
+    r = 0.0;
+    for (int g = 0; g < G; ++g) r += (double)x[g * n].x + (double)x[g * n].y;
+  }
+  return r;
+}
+
+/* Quantity q (0 to 2 the acceleration, 3 the potential) of target `to` in vars. */
 template <int FORM>
-__device__ __forceinline__ void add_target(const ListArgs& a, long long to, float x, float xl,
-                                           float y, float yl, float z, float zl, float p, float pl,
-                                           float idt) {
+__device__ __forceinline__ void add_to_vars(const ListArgs& a, long long to, int q, double x) {
+  if constexpr (FORM == kF32)
+    reinterpret_cast<float*>(static_cast<VariablePartData*>(a.vars) + to)[q] += (float)x;
+  else
+    static_cast<double*>(a.vars)[5 * to + q] += x;
+}
+
+/* dtGrav's maximum of target `to` in vars. */
+template <int FORM>
+__device__ __forceinline__ void max_to_vars(const ListArgs& a, long long to, float idt) {
   if constexpr (FORM == kF32) {
-    VariablePartData* v = static_cast<VariablePartData*>(a.vars) + to;
-    v->a.x += x + xl;
-    v->a.y += y + yl;
-    v->a.z += z + zl;
-    v->potential += p + pl;
-    v->dtGrav = fmaxf(idt, v->dtGrav);
+    float* d = &(static_cast<VariablePartData*>(a.vars) + to)->dtGrav;
+    *d = fmaxf(idt, *d);
   } else {
-    double* v = static_cast<double*>(a.vars) + 5 * to;
-    v[0] += (double)x + (double)xl;
-    v[1] += (double)y + (double)yl;
-    v[2] += (double)z + (double)zl;
-    v[3] += (double)p + (double)pl;
-    v[4] = fmax((double)idt, v[4]);
+    double* d = static_cast<double*>(a.vars) + 5 * to + 4;
+    *d = fmax((double)idt, *d);
   }
 }
 
@@ -227,24 +260,12 @@ __device__ __forceinline__ void join_groups(const ListArgs& a, const float2 (&re
   wait_for_last();
   for (int k = tid; k < 5 * nt; k += T) {
     const int q = k / nt, t = k - q * nt;
-    const long long to = first + t;
     if (q < 4) {
-      float hi = 0.f, lo = 0.f;
-      for (int g = 0; g < G; ++g) two_add(hi, lo, red[q][g * nt + t]);
-      if constexpr (FORM == kF32)
-        reinterpret_cast<float*>(static_cast<VariablePartData*>(a.vars) + to)[q] += hi + lo;
-      else
-        static_cast<double*>(a.vars)[5 * to + q] += (double)hi + (double)lo;
+      add_to_vars<FORM>(a, first + t, q, join_sum(&red[q][t], nt, G));
     } else {
       float m = 0.f;
       for (int g = 0; g < G; ++g) m = fmaxf(m, redmax[g * nt + t]);
-      if constexpr (FORM == kF32) {
-        float* d = &(static_cast<VariablePartData*>(a.vars) + to)->dtGrav;
-        *d = fmaxf(m, *d);
-      } else {
-        double* d = static_cast<double*>(a.vars) + 5 * to + 4;
-        *d = fmax((double)m, *d);
-      }
+      max_to_vars<FORM>(a, first + t, m);
     }
   }
 }
@@ -829,7 +850,13 @@ __global__ void __launch_bounds__(256, MINB) list_kernel_far(const ListArgs a) {
       if (CELL) idt2 = -idt2;
       if (G == 1) {
         wait_for_last();
-        if (lane < nt) add_target<FORM>(a, ti, sx, -cx, sy, -cy, sz, -cz, sp, -cp, idt2);
+        if (lane < nt) {
+          add_to_vars<FORM>(a, ti, 0, (double)sx - (double)cx);
+          add_to_vars<FORM>(a, ti, 1, (double)sy - (double)cy);
+          add_to_vars<FORM>(a, ti, 2, (double)sz - (double)cz);
+          add_to_vars<FORM>(a, ti, 3, (double)sp - (double)cp);
+          max_to_vars<FORM>(a, ti, idt2);
+        }
       } else {
         __syncwarp();
         red_[warp][0][lane] = make_float2(sx, -cx);
@@ -839,17 +866,14 @@ __global__ void __launch_bounds__(256, MINB) list_kernel_far(const ListArgs a) {
         redmax_[warp][lane] = idt2;
         __syncwarp();
         wait_for_last();
+        for (int k = lane; k < 4 * nt; k += 32) {
+          const int q = (k >= nt) + (k >= 2 * nt) + (k >= 3 * nt), t1 = k - q * nt;
+          add_to_vars<FORM>(a, tbase + t0 + t1, q, join_sum(&red_[warp][q][t1], nt, G));
+        }
         if (lane < nt) {
-          float2 s[4];
-#pragma unroll
-          for (int q = 0; q < 4; ++q) s[q] = red_[warp][q][lane];
           float m = idt2;
-          for (int l = lane + nt; l < G * nt; l += nt) {
-#pragma unroll
-            for (int q = 0; q < 4; ++q) two_add(s[q].x, s[q].y, red_[warp][q][l]);
-            m = fmaxf(m, redmax_[warp][l]);
-          }
-          add_target<FORM>(a, ti, s[0].x, s[0].y, s[1].x, s[1].y, s[2].x, s[2].y, s[3].x, s[3].y, m);
+          for (int l = lane + nt; l < G * nt; l += nt) m = fmaxf(m, redmax_[warp][l]);
+          max_to_vars<FORM>(a, ti, m);
         }
         __syncwarp();
       }

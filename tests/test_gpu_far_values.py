@@ -2,11 +2,15 @@
 that are not in a bucket's list, masses that are infinite or not a number,
 sums that overflow, and the last bits of the lane groups' sums."""
 import ctypes as C
+import math
+from types import SimpleNamespace
 
 import numpy as np
 import pytest
 
 from changa_gb300 import _native as N
+from changa_gb300 import gravity
+from changa_gb300.tree import ListRequest
 
 pytestmark = pytest.mark.gpu
 
@@ -92,3 +96,59 @@ def test_a_marker_far_below_zero_is_an_empty_list(variant, name):
     v = v.cpu().numpy()
     want = evaluate(call, sources, targets, [(0, 10, []), (10, 20, range(40))])
     assert (want[10:30, 3] < 0).all() and np.array_equal(v, want)
+
+
+def test_the_groups_sums_keep_fp64_bits(variant):
+    """One target, every group one source of mass m1 and, a block later, one
+    of m2 below m1's last bit, all at distance 1: a group's compensated sum is
+    m1 + m2 exactly, of 49 bits, and the join of the G groups may lose no more
+    than G - 1 FP64 additions would."""
+    block = 32 if variant == 17 else 128
+    groups = block // 2
+    rng = np.random.default_rng(11)
+    parts, lists, want = [[1.0, 0.0, 0.0, 0.0, 0.0]], [], []
+    for _ in range(40):
+        m = [(rng.integers(1 << 23, 1 << 24, groups) | 1) * 2.0 ** -23,
+             (rng.integers(1 << 23, 1 << 24, groups) | 1) * 2.0 ** -49]
+        at = len(parts)
+        for mass in np.stack([np.concatenate(m), np.zeros(2 * groups)], 1).ravel():
+            d = np.zeros(3)
+            d[rng.integers(3)] = rng.choice([-1.0, 1.0])
+            parts.append([mass, 0.0, *d])
+        lists.append((0, 1, np.arange(at, len(parts))))
+        want.append(math.fsum(m[0]) + math.fsum(m[1]))
+    parts = np.array(parts)
+    unit = len(parts)
+    parts = np.concatenate([parts, [[1.0, 0.0, 1.0, 0.0, 0.0]]])
+    call = N.cuda_lib().changa_part_forces_mixed
+    assert evaluate(call, parts, parts, [(0, 1, [unit])])[0, 3] == -1.0  # 1 / sqrt(1) is exact
+    got = [-evaluate(call, parts, parts, [l])[0, 3] for l in lists]
+    want = np.array(want)
+    assert (np.abs(got - want) <= (groups - 1) * 2.0 ** -53 * want).all()
+
+
+@pytest.mark.parametrize("variant", [17, 18])
+def test_an_infinite_potential_of_the_fp32_form(cuda_ok, variant):
+    """A mass of 3e38 at distance 1/2, whose potential of 6e38 is past FP32,
+    among finite ones in the other groups: the potential is infinite and so is
+    the acceleration toward it, not NaN."""
+    lib = N.cuda_lib()
+    parts = np.zeros((100, 5), np.float32)
+    parts[:, 0] = 1.0
+    parts[1:, 2:] = np.random.default_rng(2).uniform(1, 2, (99, 3))
+    parts[40] = 3e38, 0.0, 0.5, 0.0, 0.0
+    one = lambda x: np.array([x], np.int32)
+    entries = np.stack([np.arange(1, 100), np.full(99, HERE)], 1).astype(np.int32)
+    empty = ListRequest(entries[:0], one(0), one(0)[:0], one(0)[:0], one(0)[:0])
+    inp = gravity.DropInInputs(SimpleNamespace(
+        n=100, order=2, period=0.0, cells=empty, abi_moments=lambda: np.zeros((4, 12), np.float32),
+        plist=ListRequest(entries, np.array([0, 99], np.int32), one(0), one(1), one(0)),
+        abi_parts=lambda: parts))
+    saved = lib.changa_gb300_get_list_variant(1)
+    assert lib.changa_gb300_set_list_variant(1, variant) == 0
+    try:
+        got = gravity.dropin_step(inp).copy()
+    finally:
+        lib.changa_gb300_set_list_variant(1, saved)
+        inp.free()
+    assert got[0, 3] == -np.inf and got[0, 0] == np.inf
