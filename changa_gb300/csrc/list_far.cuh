@@ -39,11 +39,12 @@ namespace {
 constexpr int kBlockTargets = 64;
 
 /* One lane's cell record into its half h of a staged pair: {x0 x1 y0 y1} {z0 z1 -M0 -M1} {Sxx Sxy} {Sxz Syy}
- * {Syz Szz}, S = 3 (Q - tr(Q)/3 I), the trace-free part of 3Q (tr is half
- * of Q's trace). */
-__device__ __forceinline__ void stage_cell_tf(float* pb, int h, float4 p, float4 q1, float4 q2) {
+ * {Syz Szz}.  S is 3Q for a near cell, for a far one its trace-free part
+ * 3 (Q - tr(Q)/3 I) (tr is half of Q's trace). */
+__device__ __forceinline__ void stage_cell_tf(float* pb, int h, float4 p, float4 q1, float4 q2,
+                                              bool far) {
   // p {x, y, z, M}  q1 {xx, xy, xz, yy}  q2 {yz, zz, tr, soft}
-  const float t2 = 2.f * q2.z;
+  const float t2 = far ? 2.f * q2.z : 0.f;
   pb[pair_slot(0, h)] = p.x;
   pb[pair_slot(1, h)] = p.y;
   pb[pair_slot(2, h)] = p.z;
@@ -124,12 +125,10 @@ __device__ __forceinline__ void pc_near_one(const float* pb, int h, float tr, fl
     c3 = b * s;
     u = c3 * s;
   }
-  /* 3Q r from the trace-free part */
-  const float t2 = 2.f * tr;
   const float sxy = pb[pair_slot(5, h)], sxz = pb[pair_slot(6, h)], syz = pb[pair_slot(8, h)];
-  const float qx = fmaf(pb[pair_slot(4, h)] + t2, rx, fmaf(sxy, ry, sxz * rz));
-  const float qy = fmaf(sxy, rx, fmaf(pb[pair_slot(7, h)] + t2, ry, syz * rz));
-  const float qz = fmaf(sxz, rx, fmaf(syz, ry, (pb[pair_slot(9, h)] + t2) * rz));
+  const float qx = fmaf(pb[pair_slot(4, h)], rx, fmaf(sxy, ry, sxz * rz));  // 3 Q r
+  const float qy = fmaf(sxy, rx, fmaf(pb[pair_slot(7, h)], ry, syz * rz));
+  const float qz = fmaf(sxz, rx, fmaf(syz, ry, pb[pair_slot(9, h)] * rz));
   const float w = fmaf(qx, rx, fmaf(qy, ry, qz * rz));
   const float bM = b * M;
   const float q3 = fmaf(2.5f * u, w, fmaf(-3.f * c3, tr, bM));
@@ -351,12 +350,13 @@ __device__ __forceinline__ float finish_entry(float fp, const RawRec<FORM, CELL>
 }
 
 template <bool CELL>
-__device__ __forceinline__ void stage_source(float4* stage, int slot, const float4* rec) {
+__device__ __forceinline__ void stage_source(float4* stage, int slot, const float4* rec,
+                                             bool far) {
   constexpr int PW = CELL ? 5 : 2;
   float* pb = reinterpret_cast<float*>(stage + (slot >> 1) * PW);
   const int h = slot & 1;
   if constexpr (CELL) {
-    stage_cell_tf(pb, h, rec[0], rec[1], rec[2]);
+    stage_cell_tf(pb, h, rec[0], rec[1], rec[2], far);
   } else {
     pb[pair_slot(0, h)] = rec[0].x;
     pb[pair_slot(1, h)] = rec[0].y;
@@ -533,7 +533,7 @@ __global__ void __launch_bounds__(T, MINB) list_kernel_block(const ListArgs a) {
         const int nf2 = (nf + 1) & ~1;
         if (valid) {
           const int slot = far ? fbefore : nf2 + (tid - fbefore);
-          stage_source<CELL>(stage, slot, rec);
+          stage_source<CELL>(stage, slot, rec, far);
           if constexpr (CELL) strace[slot] = rec[2].z;
           ssoft[slot] = ls;
         }
@@ -737,7 +737,7 @@ __global__ void __launch_bounds__(256, MINB) list_kernel_far(const ListArgs a) {
           one_mass = __all_sync(kFull, !far || rec[0].w == m0);
         }
         if (fb == kFull) {
-          stage_source<CELL>(st, lane, rec);
+          stage_source<CELL>(st, lane, rec, true);
         } else {
           const int nf = __popc(fb), before = __popc(fb & below);
           nf2 = (nf + 1) & ~1;
@@ -745,7 +745,7 @@ __global__ void __launch_bounds__(256, MINB) list_kernel_far(const ListArgs a) {
           trips = (nf2 >> 1) / G;
           if (lane < ne) {
             const int slot = far ? before : nf2 + (lane - before);
-            stage_source<CELL>(st, slot, rec);
+            stage_source<CELL>(st, slot, rec, far);
             ss[slot] = ls;
             if constexpr (CELL) str[slot] = rec[2].z;
           }

@@ -152,3 +152,17 @@ def test_an_infinite_potential_of_the_fp32_form(cuda_ok, variant):
         lib.changa_gb300_set_list_variant(1, saved)
         inp.free()
     assert got[0, 3] == -np.inf and got[0, 0] == np.inf
+
+
+@pytest.mark.parametrize("xx", [1e-3, 3.3e-5, 7e-7])
+def test_a_near_cells_small_moment(variant, xx):
+    """A cell at distance 1 along x, near because another target's softening
+    is large but softening none of its own pair: there 1/r is exact, the trace
+    terms are M = 3 tr and cancel, and the acceleration is 3 xx (1 - 5/2).
+    Five FP32 roundings of that: its moment is not read off the trace."""
+    tgt = np.array([[1.0, 0.0, 0.0, 0.0, 0.0], [1.0, 10.0, 0.1, 0.1, 0.1]])
+    cell = np.zeros((1, 12))
+    cell[0, 2:6] = 3.0, -1.0, 0.0, 0.0
+    cell[0, 6], cell[0, 9], cell[0, 11] = xx, 1.0, 1.0 - xx  # half the trace is 1
+    got = evaluate(N.cuda_lib().changa_cell_forces_mixed, cell, tgt, [(0, 2, [0])])
+    assert abs(got[0, 0] / (-4.5 * xx) - 1.0) < 5 * 2.0 ** -24
