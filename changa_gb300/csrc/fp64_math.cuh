@@ -15,7 +15,13 @@ __device__ __forceinline__ double rsqrt_normal(double x) {
   return fma(fma(e, 0.375, 0.5), e * y, y);
 }
 
-/* The larger of two doubles that are not negative, on the integer pipe. */
+/* Whether x is not a number, on the integer pipe. */
+__device__ __forceinline__ bool is_nan(double x) {
+  return (__double_as_longlong(x) & 0x7fffffffffffffffLL) > 0x7ff0000000000000LL;
+}
+
+/* The larger of a, not negative, and b, on the integer pipe; a NaN b of
+ * positive sign is taken for the larger, so callers keep NaNs out. */
 __device__ __forceinline__ double max_nonneg(double a, double b) {
   return __longlong_as_double(max(__double_as_longlong(a), __double_as_longlong(b)));
 }

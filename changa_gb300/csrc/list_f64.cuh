@@ -211,8 +211,9 @@ __global__ void __launch_bounds__(kF64Threads, 2) list_kernel_f64(const ListArgs
           rec[3] = __ldg(s + (CELL ? 2 : 0));
           rec[4] = __ldg(s + 1);
           /* far: beyond its own softening plus the targets' largest from
-           * their box, with room for the rounding of these coordinates, and
-           * at a distance whose square is a normal number */
+           * their box, with room for the rounding of these coordinates, at a
+           * distance whose square is a normal number, and of a mass that
+           * max_nonneg can take */
           const float x = (float)(rec[0] - cx), y = (float)(rec[1] - cy), z = (float)(rec[2] - cz);
           const float bx = fmax3(box[0] - x, x - box[3], 0.f);
           const float by = fmax3(box[1] - y, y - box[4], 0.f);
@@ -221,7 +222,7 @@ __global__ void __launch_bounds__(kF64Threads, 2) list_kernel_f64(const ListArgs
           const float own = fmaf(__double2float_ru(rec[4]) + box[6], 1.0001f,
                                  1e-6f * (fabsf(x) + fabsf(y) + fabsf(z) + box[3] - box[0] + box[4] -
                                           box[1] + box[5] - box[2]));
-          far = d2 > fmaxf(own * own, 1e-30f) && d2 < 1e37f;
+          far = d2 > fmaxf(own * own, 1e-30f) && d2 < 1e37f && !is_nan(rec[3]);
         }
         if (warp < SW) {
           const unsigned fb = __ballot_sync(kFull, far);
