@@ -6,8 +6,9 @@ namespace {
 
 /* 1/sqrt(x) for positive normal x, from the hardware's approximation (some
  * 20 bits): with e = 1 - x y^2, 1/sqrt(x) = y (1 - e)^(-1/2), whose series
- * y (1 + e/2 + 3 e^2 / 8) is cut at e^3 / 3, below FP64 rounding.  Five FP64
- * operations; 0 at infinity as rsqrt gives, NaN for a zero or subnormal. */
+ * y (1 + e/2 + 3 e^2 / 8) is cut at 5 e^3 / 16, below 2^-58; the roundings of
+ * x y, of e and of the last sum make at most 2^-52 of the root.  Five FP64
+ * operations; NaN at infinity, for a zero and for a subnormal. */
 __device__ __forceinline__ double rsqrt_normal(double x) {
   double y;
   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
