@@ -246,6 +246,7 @@ CUDA_SIGNATURES = {
     "changa_walk_lists_free": (None, [C.POINTER(ChangaWalkLists)]),
     "changa_walk_set_pool_factor": (None, [_D]),
     "changa_walk_set_test_small_stack": (None, [C.c_int]),
+    "changa_walk_set_test_memory": (None, [C.c_size_t]),
     "changa_walk_set_groups": (None, [C.c_int, C.c_int]),
     "changa_walk_forces": (_I, [C.POINTER(ChangaTreeView), C.POINTER(ChangaWalkParams), _VP, _VP,
                                 _LL, C.POINTER(ChangaEwaldParams), _VP, _VP]),

@@ -1486,19 +1486,56 @@ extern "C" void changa_walk_lists_free(ChangaWalkLists* out) {
   std::memset(out, 0, sizeof(*out));
 }
 
-/* Stream-ordered scratch blocks of one call, freed together. */
+/* Testing only: the bytes that a walk may hold at once, scratch and lists (0:
+ * no limit but the device's), so that its ways out of a shortage are taken. */
+static std::atomic<size_t> g_test_memory{0};
+
+extern "C" void changa_walk_set_test_memory(size_t bytes) { g_test_memory.store(bytes); }
+
+/* Stream-ordered blocks of one call, freed together. */
 struct Scratch {
   cudaStream_t s;
   std::vector<void*> blocks;
-  void* alloc(size_t bytes) {
+  std::vector<size_t> sizes;
+  size_t held = 0;
+  Scratch(cudaStream_t st, void* first) : s(st), blocks{first}, sizes{0} {}
+  /* A block that outlives the call (not freed here). */
+  void* lend(size_t bytes) {
     void* q = nullptr;
-    if (cudaMallocAsync(&q, bytes < 256 ? 256 : bytes, s) != cudaSuccess) return nullptr;
-    blocks.push_back(q);
+    if (bytes < 256) bytes = 256;
+    const size_t most = g_test_memory.load();
+    if ((most && held + bytes > most) || cudaMallocAsync(&q, bytes, s) != cudaSuccess) {
+      cudaGetLastError();
+      return nullptr;
+    }
+    held += bytes;
     return q;
+  }
+  void* alloc(size_t bytes) {
+    void* q = lend(bytes);
+    if (!q) return nullptr;
+    blocks.push_back(q);
+    sizes.push_back(bytes < 256 ? 256 : bytes);
+    return q;
+  }
+  /* Frees a block before the others. */
+  template <typename T>
+  void drop(T*& p) {
+    for (size_t i = 0; p && i < blocks.size(); ++i)
+      if (blocks[i] == p) {
+        cudaFreeAsync(p, s);
+        held -= sizes[i];
+        blocks.erase(blocks.begin() + i);
+        sizes.erase(sizes.begin() + i);
+        break;
+      }
+    p = nullptr;
   }
   void release() {
     for (void* q : blocks) cudaFreeAsync(q, s);
     blocks.clear();
+    sizes.clear();
+    held = 0;
   }
 };
 
@@ -1585,11 +1622,9 @@ static int walk_phase1(WalkArgs& a, WalkGroups& gr, WalkTry& how, Scratch& sc, c
   if (how.slots && !gr.slots) {
     const size_t bytes = (size_t)ng * (kSlotCells + kSlotParts + kSlotFront) * sizeof(int2);
     gr.slots = bytes <= kMaxSlotBytes ? (int2*)sc.alloc(bytes) : nullptr;
-    if (!gr.slots) {
-      cudaGetLastError();  // no room for the slots: count and fill
-      how.slots = false;
-    }
+    if (!gr.slots) how.slots = false;  // no room for the slots: count and fill
   }
+  if (!how.slots) sc.drop(gr.slots);
   if (how.slots) {
     a.cells = gr.slots;
     a.parts = a.cells + (size_t)ng * kSlotCells;
@@ -1650,7 +1685,7 @@ extern "C" int changa_walk(const ChangaTreeView* t, const ChangaWalkParams* p,
   WalkArgs a;
   char* block = nullptr;
   if (int rc = walk_setup(t, p, a, &block, s)) return rc;
-  Scratch sc{s, {block}};
+  Scratch sc(s, block);
   auto finish = [&](int rc) {
     sc.release();
     if (rc) {
@@ -1698,6 +1733,12 @@ extern "C" int changa_walk(const ChangaTreeView* t, const ChangaWalkParams* p,
   unsigned int hc[16];
   int h_err[2];
   WalkTry how;
+  auto drop_pools = [&] {
+    for (int k = 0; k < nl; ++k) {
+      sc.drop(a.pool[k]);
+      sc.drop(a.chunk_bucket[k]);
+    }
+  };
   for (;;) {
     if (phase == 2) {
       if (int rc = walk_phase1(a, gr, how, sc, s)) return finish(rc);
@@ -1738,7 +1779,7 @@ extern "C" int changa_walk(const ChangaTreeView* t, const ChangaWalkParams* p,
         a.pool_chunks[k] = chunks[k];
         pools = a.pool[k] && a.chunk_bucket[k];
       }
-      if (!pools) cudaGetLastError();  // pools that did not fit: count and fill instead
+      if (!pools) drop_pools();  // pools that did not fit: count and fill instead
       a.pool_next = ctr;
       a.overflow = reinterpret_cast<int*>(ctr + 8);
     }
@@ -1765,12 +1806,31 @@ extern "C" int changa_walk(const ChangaTreeView* t, const ChangaWalkParams* p,
       return finish(record_error(CHANGA_E_TOO_LARGE, "walk: list exceeds int32 markers", __FILE__,
                                  __LINE__));
     out->n_entries[k] = tot[k];
-    if (cudaMallocAsync((void**)&out->list[k], (size_t)(tot[k] > 0 ? tot[k] : 1) * sizeof(ILCell),
-                        s) != cudaSuccess)
-      return no_memory("walk: lists");
   }
-  const bool overflow = pools && hc[8] != 0;
-  if (pools && !overflow) {
+  /* The lists.  Where there is no room for them beside the pools, the pools go
+   * and the entries come from a second traversal; then the groups' slots go
+   * too, and the groups are counted and filled. */
+  auto take_lists = [&] {
+    for (int k = 0; k < nl; ++k)
+      if (!out->list[k] &&
+          !(out->list[k] = (ILCell*)sc.lend((size_t)(tot[k] > 0 ? tot[k] : 1) * sizeof(ILCell))))
+        return false;
+    return true;
+  };
+  bool gather = pools && hc[8] == 0;
+  bool room = take_lists();
+  if (!room && pools) {
+    drop_pools();
+    gather = false;
+    room = take_lists();
+  }
+  if (!room && gr.slots) {
+    how.slots = false;
+    if (int rc = walk_phase1(a, gr, how, sc, s)) return finish(rc);
+    room = take_lists();
+  }
+  if (!room) return no_memory("walk: lists");
+  if (gather) {
     for (int k = 0; k < nl; ++k) {
       const long long used = (long long)hc[k] < chunks[k] ? (long long)hc[k] : chunks[k];
       if (used == 0) continue;
@@ -1782,7 +1842,8 @@ extern "C" int changa_walk(const ChangaTreeView* t, const ChangaWalkParams* p,
       count_launch();
     }
   } else {
-    /* entries by a second traversal (pools that ran short or did not fit) */
+    /* entries by a second traversal (pools that ran short, did not fit or had
+     * to go) */
     a.off_cells = off;
     a.off_parts = off + (nb + 1);
     a.off_soft = nl == 3 ? off + 2 * (size_t)(nb + 1) : nullptr;
@@ -1792,7 +1853,7 @@ extern "C" int changa_walk(const ChangaTreeView* t, const ChangaWalkParams* p,
     walk_run(a, kFill, s, phase, how.large);
     cudaMemcpyAsync(h_err, a.error, sizeof(h_err), cudaMemcpyDeviceToHost, s);
   }
-  out->passes = !pools ? 2 : overflow ? 3 : 1;
+  out->passes = !pools ? 2 : gather ? 1 : 3;
   if (cudaStreamSynchronize(s) != cudaSuccess)
     return finish(record_error((int)cudaGetLastError(), "walk: entries", __FILE__, __LINE__));
   if (h_err[0]) return finish(walk_error(h_err[0]));
@@ -1827,7 +1888,7 @@ extern "C" int changa_walk_forces(const ChangaTreeView* t, const ChangaWalkParam
   WalkArgs a;
   char* block = nullptr;
   if (int rc = walk_setup(t, p, a, &block, s)) return rc;
-  Scratch sc{s, {block}};
+  Scratch sc(s, block);
   auto finish = [&](int rc) {
     sc.release();
     if (rc) cudaStreamSynchronize(s);

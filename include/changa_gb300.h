@@ -388,7 +388,13 @@ int changa_walk_fill(const ChangaTreeView *tree, const ChangaWalkParams *p,
  * when order is 4) holds n_entries[k] ILCells, bucket b's entries at
  * markers[k][b] .. markers[k][b + 1], in the same order as count + fill
  * write them.  passes: 1 (append + gather), 2 (count + fill, when the
- * pools cannot be had), 3 (append, then fill).  Returns after the stream has finished. */
+ * pools cannot be had), 3 (append, then fill: a pool ran short, or went to
+ * make room for the lists).  Returns after the stream has finished.
+ * Scratch, freed to the device's default memory pool before it returns: the
+ * pools (1.2 times the estimated entries and a chunk per bucket; small trees
+ * 12 KB per bucket and list, 190 MB a list at 16383 buckets) and 48 KB per
+ * group of a two-phase walk (4 GiB at most); with less memory it counts and
+ * fills. */
 typedef struct ChangaWalkLists {
   int n_buckets;
   int order;
@@ -408,6 +414,10 @@ void changa_walk_set_pool_factor(double factor);
  * stack per warp, so that the re-run with the large stack (taken when a
  * warp exhausts its stack) is exercised. */
 void changa_walk_set_test_small_stack(int on);
+/* Testing only: the bytes that a walk may hold at once, scratch and lists
+ * (0: no limit but the device's), so that its ways out of a shortage are
+ * exercised. */
+void changa_walk_set_test_memory(size_t bytes);
 /* Traversal launches re-run with the large stack so far (in this process). */
 long long changa_walk_stack_reruns(void);
 /* changa_walk of a tree with at least min_tree_buckets buckets walks in
