@@ -282,7 +282,8 @@ struct EwaldFpArgs {
   /* the table as whole h, one of each pair h, -h with its coefficients
    * doubled; n_whole is 0 for a table of other vectors */
   int n_whole;
-  float cut2;  // fEwCut2 rounded up
+  double per_L;  // 1 / L
+  float cut;     // the real-space cut in units of L
   signed char h[CHANGA_MAX_EWH][4];
   double hc[CHANGA_MAX_EWH][2];  // cosine and sine coefficients
 };
@@ -393,20 +394,25 @@ __global__ void __launch_bounds__(kF64Warp) ewald_f64_kernel(const double* __res
   if (live)
     for (int c = 0; c < 3; ++c) dd[c] = parts[5 * j + 2 + c] - P.mom[3 + c];
   const double dxd = dd[0], dyd = dd[1], dzd = dd[2];
-  float lo[3], hi[3];
+  const int nE = P.nEwReps, nR = P.nReps;
+  const long long side = 2 * nE + 1, nrep = side * side * side;
+  /* The warp's box in units of L.  A distance from it to a replica's offset,
+   * whose parts d and i are below far, is within sqrt(3) 2^-23 far of the
+   * FP64 one. */
+  float lo[3], hi[3], far = (float)nE;
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
-    lo[c] = live ? (float)dd[c] : 3e38f;
-    hi[c] = live ? (float)dd[c] : -3e38f;
+    const float d = (float)(dd[c] * P.per_L);
+    lo[c] = live ? d : 3e38f;
+    hi[c] = live ? d : -3e38f;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
       lo[c] = fminf(lo[c], __shfl_xor_sync(0xffffffffu, lo[c], o));
       hi[c] = fmaxf(hi[c], __shfl_xor_sync(0xffffffffu, hi[c], o));
     }
+    far = fmaxf(far, fmaxf(fabsf(lo[c]), fabsf(hi[c])));
   }
-  const int nE = P.nEwReps, nR = P.nReps;
-  const long long side = 2 * nE + 1, nrep = side * side * side;
-  const float L = (float)P.L;
+  const float within = fmaf(P.cut, 1.00001f, 1e-6f * far);
   double fPot = P.mom[2] * P.k1, ax = 0, ay = 0, az = 0;
   const double fInner2 = 1.2e-3 * P.L * P.L;
   const bool split = nE <= 3;  // the Gaussian as a product over the axes
@@ -431,11 +437,11 @@ __global__ void __launch_bounds__(kF64Warp) ewald_f64_kernel(const double* __res
         float d2 = 0.f;
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-          const float a = lo[c] + i[c] * L, z = hi[c] + i[c] * L;
+          const float a = lo[c] + (float)i[c], z = hi[c] + (float)i[c];
           const float m = a > 0.f ? a : (z < 0.f ? -z : 0.f);
           d2 = fmaf(m, m, d2);
         }
-        keep = hole || !(d2 > P.cut2 * 1.0001f);  // room for the rounding of FP32 offsets
+        keep = hole || !(d2 > within * within);
       }
       const unsigned m = __ballot_sync(0xffffffffu, keep);
       if (keep) {
@@ -984,7 +990,8 @@ cudaError_t launch_ewald_fp(int form, const double* parts, long long n_parts, co
     P.nEwhLoop = p.nEwhLoop;
     for (int i = 0; i < p.nEwhLoop; ++i)
       for (int k = 0; k < 5; ++k) P.ewt[i][k] = p.ewt[5 * i + k];
-    P.cut2 = (float)P.fEwCut2;
+    P.per_L = 1.0 / L;
+    P.cut = (float)fabs(p.fEwCut);
     /* the powers serve tables whose rows are 2 pi h / L to rounding */
     std::vector<HPair> pairs;
     P.n_whole = pair_h(p, L, pairs) ? (int)pairs.size() : 0;
