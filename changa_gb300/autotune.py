@@ -7,7 +7,7 @@ workload: bucket occupancy, list lengths and the share of softened pairs
 shift the balance between occupancy and spills.  ``tune`` times every shape
 on the actual device-resident lists with the library's per-kernel CUDA-event
 timing, selects the fastest for the cell and the particle kernel separately,
-and caches the choice per (GPU, form, workload signature) in
+and caches the choice per (GPU, form, set of shapes, workload) in
 ``_build/tuning.json``.
 """
 from __future__ import annotations
@@ -23,12 +23,15 @@ KERNELS = {"mixed": ("list_mixed_cell", "list_mixed_part")}
 
 
 def signature(ds, form):
+    """Key of a choice: the GPU, the library's set of shapes (a choice among
+    fewer shapes does not stand for a library that has more) and the
+    workload."""
     import torch
     name = torch.cuda.get_device_name()
     L = ds.lists
     nb = max(1, L.cells.n_buckets)
-    return "%s|%s|n=%d|cells=%d|parts=%d|nb=%d" % (
-        name, form, L.n, L.cells.n_entries // nb, L.plist.n_entries // max(1, L.plist.n_buckets),
+    return "%s|%s|shapes=%d|n=%d|cells=%d|parts=%d|nb=%d" % (
+        name, form, N.cuda_lib().changa_gb300_list_variant_count(), L.n, L.cells.n_entries // nb, L.plist.n_entries // max(1, L.plist.n_buckets),
         round(L.n / max(1, len(L.bucket_starts))))
 
 
