@@ -402,6 +402,16 @@ def traffic_from_profiles():
     return {}
 
 
+def captured(traffic, kernel, variant):
+    """The ncu figures of `traffic` for `kernel` (list_mixed_cell or _part):
+    DRAM bytes per launch, FMA pipe share and note, when they were taken on
+    the shape variant that ran; empty otherwise."""
+    if variant not in traffic.get("capture", {}).get("variants", {}).get(kernel, []):
+        return {}
+    return {"bytes": traffic[kernel + "_bytes_per_launch"],
+            "fma_pipe_pct": traffic[kernel + "_fma_pipe_pct"], "note": traffic["note"]}
+
+
 def main_reference(args):
     world = int(os.environ.get("WORLD_SIZE", "1"))
     rank = int(os.environ.get("RANK", "0"))
@@ -983,6 +993,7 @@ def main_ours(args):
     ms_pc, n_pc = ktimes["list_mixed_cell"]
     ms_pp, n_pp = ktimes["list_mixed_part"]
     if n_pc:
+        cap = captured(tr, "list_mixed_cell", lib_v[0])
         t_pc = ms_pc / n_pc / 1e3
         ach = I_c * FLOP_PC / t_pc / 1e12
         roof = {"bound": "fp32", "kernel": "FP32-mixed cell-list kernel, shape variant %d" % lib_v[0],
@@ -991,11 +1002,12 @@ def main_ours(args):
                 "algorithmic_flop_per_launch": I_c * FLOP_PC,
                 "flop_per_interaction": FLOP_PC, "interactions_per_launch": I_c,
                 "avg_launch_ms": 1e3 * t_pc,
-                "traffic": tr.get("list_mixed_cell_bytes_per_launch"),
-                "fma_pipe_active_ncu_pct": tr.get("list_mixed_cell_fma_pipe_pct"),
-                "traffic_note": tr.get("note")}
+                "traffic": cap.get("bytes"),
+                "fma_pipe_active_ncu_pct": cap.get("fma_pipe_pct"),
+                "traffic_note": cap.get("note")}
     roof_pp = None
     if n_pp:
+        cap = captured(tr, "list_mixed_part", lib_v[1])
         t_pp = ms_pp / n_pp / 1e3
         ach = I_p * FLOP_PP / t_pp / 1e12
         roof_pp = {"bound": "fp32",
@@ -1003,8 +1015,8 @@ def main_ours(args):
                    "achieved": ach, "peak": peak, "unit": "TFLOP/s", "frac": ach / peak,
                    "algorithmic_flop_per_launch": I_p * FLOP_PP, "flop_per_interaction": FLOP_PP,
                    "interactions_per_launch": I_p, "avg_launch_ms": 1e3 * t_pp,
-                   "traffic": tr.get("list_mixed_part_bytes_per_launch"),
-                   "fma_pipe_active_ncu_pct": tr.get("list_mixed_part_fma_pipe_pct")}
+                   "traffic": cap.get("bytes"),
+                   "fma_pipe_active_ncu_pct": cap.get("fma_pipe_pct")}
     kshare = {k: {"ms_per_step": v[0] / max(1, args.steps), "launches": v[1]}
               for k, v in ktimes.items() if v[1]}
     # Ewald on its own: particle evaluations/s and the reference's per-particle
