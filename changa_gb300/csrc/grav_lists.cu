@@ -1783,12 +1783,12 @@ __global__ void __launch_bounds__(kThreads, MINB) list_kernel_tma(const ListArgs
 /* ------------------------------------------------------------------ */
 /* Paired target-parallel kernel for hexadecapole cells (FP32-mixed):  */
 /* list_kernel_tp2's structure with momEvalFmomrcm (hex_eval) on two    */
-/* staged cells per .f32x2 instruction.  Staged pair: 26 fields {x y z */
-/* M radius, 21 moments} of both cells, 13 float4 words; hexadecapole  */
-/* cells carry no softening (softened cells have their own list), so   */
-/* there is no near-field branch.  One staging buffer per warp (the    */
-/* record is 2.2x the quadrupole's); the next block's packed records   */
-/* are loaded into registers while the current block computes.        */
+/* staged cells per .f32x2 instruction.  Staged pair: 30 fields of both */
+/* cells (stage_hex), 15 float4 words; hexadecapole cells carry no      */
+/* softening (softened cells have their own list), so there is no       */
+/* near-field branch.  One staging buffer per warp (the record is 2.5x  */
+/* the quadrupole's); the next block's packed records are loaded into   */
+/* registers while the current block computes.                         */
 /* ------------------------------------------------------------------ */
 
 struct RawHex {
@@ -2235,11 +2235,12 @@ __device__ __forceinline__ void pack_cell_hex(const double* r, float4* o) {
 }
 
 /* Packs n_cells cells and n_parts particles and zeroes the list kernels'
- * work counters, in one launch.  Bound by memory: tiles of kPackTile rows are
+ * work counters, in one launch.  Tiles of kPackTile rows are
  * copied to shared memory in order (rows of 40, 96 or 216 bytes read by a
  * thread each take as many passes over their lines as they have words) and
  * packed from there.  2^20 particles and the cells of their tree, cold caches:
- * 60 us in two launches of a thread per row, 38 us so. */
+ * 60 us in two launches of a thread per row, 38 us so.  2^23: 267 us, 40 % of
+ * the copy bandwidth, as two launches took; what bounds it there is not known. */
 constexpr int kPackTile = 128;
 template <int KIND>
 __global__ void __launch_bounds__(kPackTile) pack_step_kernel(
@@ -2287,7 +2288,7 @@ __global__ void cells_as_parts_kernel(const double* __restrict__ m, int stride, 
   }
 }
 
-/* The FP64 form runs list_kernel (its cost is the FP64 pipe); the FP32
+/* The FP64 form runs list_kernel_f64 (its cost is the FP64 pipe); the FP32
  * forms run one of the variants below: the far-first kernels by default
  * (the fastest on the measured workloads), the others on request or by the
  * autotuner. */
@@ -2421,7 +2422,16 @@ cudaError_t launch_variant(const ListArgs& a, cudaStream_t s) {
      * there the CTA gains only where it fills idle SMs (4 per SM); us a step,
      * CTA against warp: 530 buckets of 5.7 targets 43 / 51, 1060 of 5.7
      * 57 / 54, 2100 of 5.7 73 / 65, 1400 of 8.5 69 / 79 (overlapped, as they
-     * run now: 25 / 28, 40 / 33, 57 / 51, 51 / 51). */
+     * run now: 25 / 28, 40 / 33, 57 / 51, 51 / 51).
+     *
+     * n_tgt counts the particle array, not the request's targets, so the mean
+     * is right only where every bucket is in the request.  A request of a part
+     * of the buckets takes the line of 24 per SM whatever they hold, and there
+     * the warp is often the better: a request of 300 / 1200 / 3600 of the
+     * buckets of 100000 particles, a captured step in us, CTA against warp:
+     * buckets of 5.5 targets 29 / 37, 53 / 41, 93 / 75, of 10.9 targets
+     * 29 / 45, 61 / 52, 116 / 106 (the paired kernels: 60, 62, 107 and 77, 80,
+     * 139). */
     const bool tiny = a.n_tgt < 8ll * a.n_buckets;
     return (long long)a.n_buckets <= (tiny ? 4ll : 24ll) * sm_count() ? launch_variant<FORM, CELL, kBlockVariant>(a, s)
                                                        : launch_variant<FORM, CELL, kFarVariant>(a, s);

@@ -22,9 +22,11 @@
  * walk's, in this traversal's order, and each list's entries of one step
  * are written contiguously.
  *
- * Two launches: a count pass (per-bucket list lengths) and, after the
- * counts have become offsets, a fill pass; changa_walk runs both and the
- * prefix sums in between.
+ * changa_walk makes one traversal, which counts every bucket's lists and
+ * appends their entries to pools of chunks, and a gather that puts the chunks
+ * in list order.  changa_walk_count and changa_walk_fill are the two passes
+ * for callers that own the lists: the lengths and, after these have become
+ * offsets, the entries; changa_walk fills so where its pools fall short.
  *
  * Decisions equal the host walk's FP64 decisions.  GB300 issues FP64 at a
  * small fraction of its FP32 rate, so each opening test is first made in
@@ -437,8 +439,8 @@ __device__ __noinline__ int take_chunks(const WalkArgs& a, int k, int b, int ran
   return (int)c;
 }
 
-/* Local nodes of a walk: chain[0] the unit's node, upward to `top` (the root
- * when top is negative).  Returns top's level, or -1 when the chain is longer
+/* Local nodes of a walk: chain[0] the unit's node, upward to `top` (0, the
+ * root, or a group's node).  Returns top's level, or -1 when the chain is longer
  * than 64 or does not meet top.  Lane 0 climbs; the result is the warp's. */
 __device__ __forceinline__ int climb_chain(const int* __restrict__ parent, long long n_nodes, int bn,
                                            int top, int* chain) {
