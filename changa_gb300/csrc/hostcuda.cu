@@ -160,7 +160,12 @@ static size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
  * chunks of 256 / 64 / 32 / 16 / 8 MiB: runs entry, 2^20 particles (208 MB of
  * cells) 4190 / 3540 / 3595 / 3784 / 4144; drop-in, 500009 particles (110 MB
  * and 240 MB of lists) 3470 / 3613 / 2557 / 2952 / 3391; drop-in, 200000
- * particles in 4400 buckets, 2290 whole, 2740 in chunks of 32 MiB. */
+ * particles in 4400 buckets, 2290 whole, 2740 in chunks of 32 MiB.  Drop-in
+ * requests on several streams in turn overlap without chunks: a cell and a
+ * particle list of 80 and 97 MB on each of 1 / 2 / 4 / 8 streams, whole 1344 /
+ * 1938 / 3666 / 7132, in chunks 1022 / 1994 / 3902 / 7759; of 86 and 192 MB 2366
+ * / 3306 / 5932 / 11314 and 1633 / 3105 / 6014 / 11802 (a caller of many streams
+ * sets 256 MiB). */
 constexpr size_t kMinHostChunkBytes = size_t(32) << 20, kMaxHostChunkBytes = size_t(256) << 20;
 static std::atomic<size_t> g_host_chunk_bytes{0};
 static size_t host_chunk_bytes(size_t bytes, long long n_buckets = 0) {
