@@ -520,16 +520,23 @@ __global__ void __launch_bounds__(kWalkWarps * 32, 8)
   int n[3] = {0, 0, 0}, nf = 0;     // entries so far
   /* append pass, per list: entries that the chunks taken hold, and where entry
    * q goes in the last chunk taken before this step (less that chunk's first
-   * entry) and in those taken in it; a negative pool position drops entries */
+   * entry) and in those taken in it */
   int room[3] = {0, 0, 0}, last[3] = {-1, -1, -1};
   int split = 0, fresh = -1;
+  /* a pool has run short, here or in another warp: a fill pass writes the
+   * entries, so from here on they are only counted (200000 particles in
+   * buckets of 2000, whose lists outgrow the guessed pools: the walk 1103 us
+   * with the entries still placed, 561 so, 632 as count and fill) */
+  bool count_only = MODE == kCount;
+  if (POOL) count_only = __shfl_sync(full, *static_cast<volatile int*>(a.overflow), 0) != 0;
   auto reserve = [&](int k, int total) {
-    if (POOL) {
+    if (POOL && !count_only) {
       split = room[k];
       if (n[k] + total > room[k]) {  // uniform over the warp
         const int m = (n[k] + total - room[k] + kChunk - 1) / kChunk;
         fresh = take_chunks(a, k, b, room[k] / kChunk, m);
         room[k] += m * kChunk;
+        count_only = fresh < 0;
       }
     }
   };
@@ -537,12 +544,12 @@ __global__ void __launch_bounds__(kWalkWarps * 32, 8)
     if (FILL) base[k][q] = e;
     if (SLOT && q < a.slot[k]) base[k][q] = e;
     if (POOL) {
-      const int c = q < split ? last[k] : fresh < 0 ? -1 : fresh + (q - split) / kChunk;
-      if (c >= 0) a.pool[k][(size_t)c * kChunk + q % kChunk] = e;
+      const int c = q < split ? last[k] : fresh + (q - split) / kChunk;
+      a.pool[k][(size_t)c * kChunk + q % kChunk] = e;
     }
   };
   auto done = [&](int k) {  // the step's entries are put
-    if (POOL && room[k] > split) last[k] = fresh < 0 ? -1 : fresh + (room[k] - split) / kChunk - 1;
+    if (POOL && !count_only && room[k] > split) last[k] = fresh + (room[k] - split) / kChunk - 1;
   };
   int2* st = stk + warp * stack;
   int sp = 0;
@@ -573,19 +580,19 @@ __global__ void __launch_bounds__(kWalkWarps * 32, 8)
           const unsigned mc = __ballot_sync(full, lane < tot && !soft);
           const unsigned ms = __ballot_sync(full, lane < tot && soft);
           reserve(0, __popc(mc));
-          if (MODE != kCount && lane < tot && !soft) put(0, n[0] + __popc(mc & below), e);
+          if (!count_only && lane < tot && !soft) put(0, n[0] + __popc(mc & below), e);
           done(0);
           n[0] += __popc(mc);
           reserve(2, __popc(ms));
-          if (MODE != kCount && lane < tot && soft) put(2, n[2] + __popc(ms & below), e);
+          if (!count_only && lane < tot && soft) put(2, n[2] + __popc(ms & below), e);
           done(2);
           n[2] += __popc(ms);
         }
         continue;
       }
-      if (MODE != kCount) {
+      if (!count_only) {
         reserve(k, cnt);
-        for (int j = lane; j < cnt; j += 32) put(k, j, pre[j]);
+        for (int j = lane; j < cnt && !count_only; j += 32) put(k, j, pre[j]);
         done(k);
       }
       n[k] = cnt;
@@ -664,7 +671,7 @@ __global__ void __launch_bounds__(kWalkWarps * 32, 8)
     const unsigned mc = __ballot_sync(full, kind == 0);
     if (mc) {
       reserve(0, __popc(mc));
-      if (MODE != kCount && kind == 0)
+      if (!count_only && kind == 0)
         put(0, n[0] + __popc(mc & below), make_int2(g, code << 22));
       done(0);
       n[0] += __popc(mc);
@@ -673,7 +680,7 @@ __global__ void __launch_bounds__(kWalkWarps * 32, 8)
       const unsigned ms = __ballot_sync(full, kind == 1);
       if (ms) {
         reserve(2, __popc(ms));
-        if (MODE != kCount && kind == 1)
+        if (!count_only && kind == 1)
           put(2, n[2] + __popc(ms & below), make_int2(g, code << 22));
         done(2);
         n[2] += __popc(ms);
@@ -682,7 +689,7 @@ __global__ void __launch_bounds__(kWalkWarps * 32, 8)
     const int pcount = kind == 2 && nb > 0 ? nb : 0;
     const unsigned mp = __ballot_sync(full, pcount > 0);
     if (mp) {
-      if (MODE == kCount) {
+      if (count_only) {
         n[1] += __reduce_add_sync(full, pcount);
       } else {
         /* the step's particle entries, 32 at a time: the runs compacted in
@@ -695,7 +702,7 @@ __global__ void __launch_bounds__(kWalkWarps * 32, 8)
         reserve(1, tpart);
         __syncwarp();
         int rank0 = -1;  // runs starting before this window, less one
-        for (int j0 = 0; j0 < tpart; j0 += 32) {
+        for (int j0 = 0; j0 < tpart && !count_only; j0 += 32) {
           const unsigned at = (unsigned)(ppos - j0);
           const unsigned mw = __reduce_or_sync(full, pcount > 0 && at < 32u ? 1u << at : 0u);
           const int j = j0 + lane;

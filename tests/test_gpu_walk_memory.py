@@ -47,3 +47,28 @@ def test_walk_with_less_memory(cuda_ok, order, groups):
     assert passes[0] == 1 and passes[-1] == 2 and 3 in passes
     assert limit > lists / 2
     assert same_entries(L.cells, gpu_walk(L)[0], nb)
+
+
+@pytest.mark.parametrize("groups", [0, 8])
+@pytest.mark.parametrize("order", [2, 4])
+@pytest.mark.parametrize("n_bucket", [8, 300])
+def test_walk_whose_pools_run_short(cuda_ok, n_bucket, order, groups):
+    """Pools of a chunk per bucket and list: warps that find them short, and
+    those that start after, only count; the counts and the filled lists are the
+    host walk's."""
+    p = ics.plummer(12000, ics.rng_for(10), soft=0.3)
+    L = tree.build_lists(p["pos"], p["mass"], p["soft"], n_bucket=n_bucket, theta=0.6, order=order)
+    nb = len(L.bucket_starts)
+    lib = N.cuda_lib()
+    lib.changa_walk_set_groups(groups, 1)
+    lib.changa_walk_set_pool_factor(0.0)
+    try:
+        tm = {}
+        got = gpu_walk(L, timings=tm)
+    finally:
+        lib.changa_walk_set_pool_factor(1.2)
+        lib.changa_walk_set_groups(32, 10240)
+    assert tm["passes"] == 3
+    assert same_entries(L.cells, got[0], nb) and same_entries(L.plist, got[1], nb)
+    if order == 4:
+        assert same_entries(L.softcells, got[2], nb)
