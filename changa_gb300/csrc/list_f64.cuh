@@ -11,7 +11,8 @@
  * run on the integer pipe: 17 FP64 instructions per particle pair and 39 per
  * cell pair, about 27 and 60 before.  The far test itself is made in FP32 on
  * bucket-relative coordinates, with a margin for their rounding; a source it
- * calls near gets the full evaluation, which is always right.
+ * calls near gets the full evaluation, which is always right.  Buckets of one
+ * or two targets are not staged (few_targets_f64).
  * nfw 120011, bucket 32, us: particles 11209 -> 6000, cells 5660 -> 3210, the FP64
  * pipe busy 88-89% of cycles (its practical limit).
  */
@@ -129,6 +130,114 @@ __device__ __noinline__ void near_f64(const double* rec, double tx, double ty, d
   acc->idt2 = fmax(acc->idt2, (tmass + M) * b);
 }
 
+/* A bucket of N targets, one or two: the threads take a list entry each and
+ * evaluate it on all of them.  Nothing is staged, whose FP64 operations (some 15
+ * per entry) only pay where more targets share them, and no thread waits for
+ * another before the sums are joined.  us a step, 40000 Plummer particles in
+ * buckets of at most 1 / 2 / 3 (1.0, 1.6 and 2.2 in the mean): staged as the
+ * larger ones 7237 / 4624 / 3636, so 3146 / 2861 / 2968 (a warp per bucket,
+ * which the CTA replaced, 3501 / 2938 / 3159).  Three and four targets gain by
+ * staging: buckets of at most 4, 2803, with those taken one target after
+ * another too 3427. */
+constexpr int kF64Few = 2;
+
+template <bool CELL, int N>
+__device__ __noinline__ void few_targets_f64(const double* src, unsigned limit, double fp,
+                                             const int2* list, int n_list, const double* tgt,
+                                             double* vars, double (&red)[4][kF64Threads],
+                                             double (&redmax)[kF64Threads]) {
+  constexpr int T = kF64Threads;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  Acc64 acc[N];
+#pragma unroll
+  for (int t = 0; t < N; ++t) acc[t] = Acc64{0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+  for (long long k = tid; k < n_list; k += T) {
+    const int2 ent = __ldg(list + k);
+    const size_t idx = (unsigned)ent.x < limit ? (unsigned)ent.x : 0u;  // memory safety
+    const int code = (ent.y >> 22) & 0x1ff;
+    const double* s = src + (CELL ? 12 : 5) * idx;
+    /* {x y z M soft}, and for cells {tr xx xy xz yy yz zz}; their trace-free form */
+    double rec[CELL ? 12 : 5], tf[CELL ? 10 : 5];
+#pragma unroll
+    for (int q = 0; q < 3; ++q) rec[q] = __ldg(s + (CELL ? 3 : 2) + q);
+    if (code != 0xdb) {  // replica (0, 0, 0) adds nothing
+      rec[0] += (double)((code & 7) - 3) * fp;
+      rec[1] += (double)(((code >> 3) & 7) - 3) * fp;
+      rec[2] += (double)(((code >> 6) & 7) - 3) * fp;
+    }
+    rec[3] = __ldg(s + (CELL ? 2 : 0));
+    rec[4] = __ldg(s + 1);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) tf[q] = rec[q];
+    if constexpr (CELL) {
+#pragma unroll
+      for (int q = 6; q < 12; ++q) rec[q] = __ldg(s + q);
+      const double tr = rec[6] + rec[9] + rec[11];
+      rec[5] = 0.5 * tr;
+      tf[4] = fma(3.0, rec[6], -tr);
+      tf[5] = 3.0 * rec[7];
+      tf[6] = 3.0 * rec[8];
+      tf[7] = fma(3.0, rec[9], -tr);
+      tf[8] = 3.0 * rec[10];
+      tf[9] = fma(3.0, rec[11], -tr);
+    }
+#pragma unroll
+    for (int t = 0; t < N; ++t) {
+      const double* p = tgt + 5 * t;
+      const double tmass = __ldg(p), tsoft = __ldg(p + 1), tx = __ldg(p + 2), ty = __ldg(p + 3),
+                   tz = __ldg(p + 4);
+      const double rx = CELL ? tx - rec[0] : rec[0] - tx, ry = CELL ? ty - rec[1] : rec[1] - ty,
+                   rz = CELL ? tz - rec[2] : rec[2] - tz;
+      const long long r2 = __double_as_longlong(fma(rx, rx, fma(ry, ry, rz * rz)));
+      const double twoh = rec[4] + tsoft;
+      /* unsoftened, the square a normal number (a NaN is past the last bound),
+       * and a mass that max_nonneg can take */
+      const bool far = r2 >= __double_as_longlong(twoh * twoh) &&
+                       r2 >= __double_as_longlong(1e-290) && r2 < __double_as_longlong(1e300) &&
+                       !is_nan(rec[3]);
+      if (!far) {
+        /* copies, so that only these have addresses */
+        double r[CELL ? 12 : 5];
+#pragma unroll
+        for (int q = 0; q < (CELL ? 12 : 5); ++q) r[q] = rec[q];
+        Acc64 c = acc[t];
+        near_f64<CELL>(r, tx, ty, tz, tsoft, tmass, &c);
+        acc[t] = c;
+      } else if constexpr (CELL) {
+        pc_far_f64(tf, tx, ty, tz, tmass, acc[t]);
+      } else {
+        pp_far_f64<false>(tf, tx, ty, tz, tmass, acc[t]);
+      }
+    }
+  }
+#pragma unroll
+  for (int t = 0; t < N; ++t) {
+    red[0][tid] = acc[t].ax;
+    red[1][tid] = acc[t].ay;
+    red[2][tid] = acc[t].az;
+    red[3][tid] = CELL ? fma(-0.5, acc[t].quad, acc[t].pot) : acc[t].pot;
+    redmax[tid] = acc[t].idt2;
+    __syncthreads();
+    wait_for_last();
+    if (warp < 5) {  // a warp per quantity
+      const double* r = warp < 4 ? red[warp] : redmax;
+      double v = r[lane];
+#pragma unroll
+      for (int j = 32; j < T; j += 32) v = warp < 4 ? v + r[lane + j] : max_nonneg(v, r[lane + j]);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        const double w = __shfl_xor_sync(kFull, v, o);
+        v = warp < 4 ? v + w : max_nonneg(v, w);
+      }
+      if (lane == 0) {
+        double* to = vars + 5 * t + warp;
+        *to = warp < 4 ? *to + v : fmax(v, *to);
+      }
+    }
+    __syncthreads();  // red is free again
+  }
+}
+
 template <bool CELL>
 __global__ void __launch_bounds__(kF64Threads, 2) list_kernel_f64(const ListArgs a) {
   constexpr int T = kF64Threads, W = T / 32, SB = kF64Block, SW = SB / 32;
@@ -163,6 +272,13 @@ __global__ void __launch_bounds__(kF64Threads, 2) list_kernel_f64(const ListArgs
     const int n = __ldg(a.sizes + b);
     const bool skip = n <= 0 || tbase < 0 || tbase + n > a.n_tgt;  // memory safety
 
+    if (!skip && n <= kF64Few) {
+      (n == 1 ? few_targets_f64<CELL, 1> : few_targets_f64<CELL, 2>)(
+          src, limit, fp, a.list + e_begin, e_end - e_begin, tgt + 5 * tbase, vars + 5 * tbase, red,
+          redmax);
+      __syncthreads();  // snext is written
+      continue;
+    }
     for (int t0 = 0; !skip && t0 < n; t0 += T) {
       const int nt = min(T, n - t0);
       const int G = T / nt;
