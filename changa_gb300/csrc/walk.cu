@@ -277,8 +277,12 @@ __device__ __forceinline__ int screen_le_t(float v, float ev, float t, float et)
  * 1 certainly true, 0 certainly false, -1 too close to call.  Per
  * axis the FP32 inputs and their sums carry at most delta = 6u (|cm| + |o| + |node's cm or box face|) against the FP64
  * values; the softening sums 2 s_g + 2 s_node carry at most 3u of their
- * value, so their square at most 7u (bounded here by 8u). */
-__device__ __noinline__ int open_softening_screened(const WalkArgs& a, float sg, const float* c,
+ * value, so their square at most 7u (bounded here by 8u).  Inlined: a call
+ * passes the arrays through local memory in every step of an order-4 walk (us a
+ * walk, called / inlined / the walk before with its tests in FP32 boxes: 2806
+ * buckets of 21 Plummer particles 638 / 525 / 558, 21791 of 11 1710 / 1322 /
+ * 1690; 12374 of 19 NFW particles 1274 / 1037 / 1288). */
+__device__ __forceinline__ int open_softening_screened(const WalkArgs& a, float sg, const float* c,
                                        const float* cm, const float* o, int node) {
   const float4 nc = a.nodes[node].geo;
   const float sn = a.hexf[node].x;
